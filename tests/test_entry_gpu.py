@@ -206,3 +206,39 @@ def test_model_drawn_on_the_device_is_the_folder_written_from_the_same_seed(tmp_
     m3 = tl.load(d, dtype="float32", max_tokens=256, random_weights=True, seed=21)
     (s,) = m3.start_sequences(1)
     assert np.array_equal(m3.step([s], [toks], "all").cpu().numpy(), got)
+
+
+@pytest.mark.parametrize("rows,V", [(1, 1), (3, 257), (2, 4096), (2, 4097), (2, 8193), (5, 32000), (2, 65537), (3, 131072),
+                                    (2, 151936), (1, 262144), (1, 262145),
+                                    (40, 32000), (80, 32768), (150, 5000)])
+def test_a_cluster_of_blocks_samples_what_one_block_samples(rows, V):
+    """Both kernels add whole numbers, so they must agree on every token: at the vocabularies where the blocks per
+    row and the entries per thread change, with rows that do and do not start on 16 bytes, ties across blocks, entries
+    that are no numbers, infinities and rows of the lowest value."""
+    from torchless_rs_b200.csrc import ops
+    s = ops.sampling_ops()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    for pad in (0, 1, 4):
+        x = (torch.randn((rows, V + pad), generator=g, device="cuda") * 3)[:, :V]
+        forms = [x, torch.round(x), torch.zeros_like(x), torch.full_like(x, -3.0e38)]
+        y = x.clone()
+        y[:, ::3] = -float("inf")
+        forms.append(y)
+        y = torch.round(x)
+        y[:, V // 2:] = float("nan")
+        forms.append(y)
+        y = x.clone()
+        y[:, V - 1] = float("inf")
+        forms.append(y)
+        y = torch.full_like(x, -float("inf"))
+        forms.append(y)
+        for y in forms:
+            wide = torch.empty((rows, V + pad), device="cuda")
+            wide[:, :V] = y
+            y = wide[:, :V]
+            for t, k, p in ((1.0, 0, 0.0), (0.7, 0, 0.9), (1.3, 1, 0.0), (0.9, 50, 0.95), (1.0, max(V - 1, 1), 0.5), (2.0, 0, 0.01)):
+                u = torch.rand((rows,), generator=g, device="cuda")
+                a, b = (torch.full((rows,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+                s.sample(y, t, k, p, u, a)
+                s.sample(y, t, k, p, u, b, walk=True)
+                assert a.tolist() == b.tolist(), (V, pad, t, k, p)

@@ -1267,6 +1267,7 @@ class SamplingOps:
         self.lib = build.load_library("sampling")
         self.lib.tl_argmax.restype = c_int
         self.lib.tl_sample.restype = c_int
+        self.lib.tl_sample_walk.restype = c_int
 
     def argmax(self, logits: torch.Tensor, out: torch.Tensor) -> None:
         _need(logits, torch.float32, "argmax logits", contiguous=False)
@@ -1278,16 +1279,19 @@ class SamplingOps:
                                   _ptr(out), _stream()), "argmax")
 
     def sample(self, logits: torch.Tensor, temperature: float, top_k: int, top_p: float,
-               uniform: torch.Tensor, out: torch.Tensor) -> None:
+               uniform: torch.Tensor, out: torch.Tensor, walk: bool = False) -> None:
+        """`walk`: by one block per row through memory whatever the vocabulary (else only beyond what a
+        cluster of blocks holds in registers); the same tokens."""
         _need(logits, torch.float32, "sample logits", contiguous=False)
         _need(uniform, torch.float32, "sample uniform")
         _need(out, torch.int32, "sample out")
         rows, V = logits.shape
         if logits.stride(1) != 1 or uniform.numel() < rows or out.numel() < rows:
             raise KernelError("sample: bad arguments")
-        _check(self.lib.tl_sample(_ptr(logits), c_int(logits.stride(0)), c_int(rows), c_int(V),
-                                  c_float(temperature), c_int(top_k), c_float(top_p),
-                                  _ptr(uniform), _ptr(out), _stream()), "sample")
+        call = self.lib.tl_sample_walk if walk else self.lib.tl_sample
+        _check(call(_ptr(logits), c_int(logits.stride(0)), c_int(rows), c_int(V),
+                    c_float(temperature), c_int(top_k), c_float(top_p),
+                    _ptr(uniform), _ptr(out), _stream()), "sample")
 
 
 _core: dict = {}

@@ -2,10 +2,11 @@
 // top-p in the order of the reference (src/sampler/mod.rs:194-222): logits / T, top-k
 // on the scaled logits, softmax, top-p on the probabilities, inverse-CDF draw.
 //
-// One block per row of logits.  Probabilities are kept as 40-bit fixed-point
-// integers of exp(z - max): integer sums do not depend on the order of addition, so
-// every threshold and the draw are the same from run to run and equal to a
-// sequential pass in index order.  The uniform number of each row comes from the
+// A cluster of blocks per row of logits holds the row in registers (vocabularies of up to
+// 262,144 entries; one block per row walks longer ones through memory).  Probabilities are kept
+// as 40-bit fixed-point integers of exp(z - max): integer sums do not depend on the order of
+// addition, so every threshold and the draw are the same from run to run, the same from both
+// kernels and equal to a sequential pass in index order.  The uniform number of each row comes from the
 // host, which derives it from (seed, sequence, step).
 //
 // Ties: arg-max keeps the highest index among equal maxima, as the reference's max_by does
@@ -309,15 +310,12 @@ __device__ int nth_in_order(const float* row, int V, int need, SampleShared& sm,
                          [&](int i, float x) { return pred(i, x) ? 1ull : 0ull; });
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature, int top_k,
-              float top_p, const float* __restrict__ uniform, int* __restrict__ out) {
-  __shared__ SampleShared sm;
-  pdl_wait();
-  pdl_launch_dependents();
+// One row by one block, walking it through memory.
+__device__ __noinline__ void sample_row(const float* row, int V, float temperature, int top_k, float top_p, float r,
+                                        int* out, SampleShared& sm) {
   const int tid = threadIdx.x;
   RowView rv;
-  rv.row = logits + (size_t)blockIdx.x * ld;
+  rv.row = row;
   rv.V = V;
   rv.T = temperature;
   rv.use_k = top_k > 0 && top_k < V;
@@ -430,7 +428,6 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
   }
 
   // ---- draw: first kept index whose running weight exceeds floor(r * S)
-  float r = uniform[blockIdx.x];
   r = r < 0.0f ? 0.0f : (r >= 1.0f ? 0.99999994f : r);
   u64 target = (u64)((double)r * (double)S);
   if (target >= S) target = S ? S - 1ull : 0ull;
@@ -442,17 +439,359 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
     if (rvd.use_p && !(w > rvd.p_thr || (w == rvd.p_thr && i <= rvd.p_cut))) return 0ull;
     return w;
   });
-  if (tid == 0) out[blockIdx.x] = chosen >= 0 ? chosen : V - 1;  // the reference's fallback, :237
+  if (tid == 0) *out = chosen >= 0 ? chosen : V - 1;  // the reference's fallback, :237
+}
+
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature, int top_k,
+              float top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+  __shared__ SampleShared sm;
+  pdl_wait();
+  pdl_launch_dependents();
+  sample_row(logits + (size_t)blockIdx.x * ld, V, temperature, top_k, top_p, uniform[blockIdx.x], out + blockIdx.x, sm);
+}
+
+// --------------------------------------------------------------------------
+// The same by a cluster of blocks per row, each thread with EPT consecutive entries of the row
+// in registers.  The kernel above is bound by its passes over the row: ten to fifteen, 128 entries
+// per thread of its one block at 131,072 entries, with the division, the exponential and the
+// fixed-point weight again in each.  Here an entry is read, divided and turned into its weight
+// once, a pass touches EPT registers, and what the blocks have to add up (histograms, sums,
+// counts of ties) goes through distributed shared memory.  Measured, temperature / top-k 50 / top-p 0.95 / both,
+// with the launch from Python: 8 rows of 131,072 entries 74 / 178 / 916 / 378 us by one block, 10 / 29 / 60 / 48 us
+// here; 8 x 32,000: 21 / 63 / 306 / 145 and 9 / 18 / 28 / 32 us; 64 x 131,072: 80 / 202 / 968 / 407 and 32 / 112 / 211 /
+// 169 us; 64 x 1000: 7 / 33 / 81 / 93 and 7 / 14 / 21 / 25 us.  What is left at top-p is the atomics of its four
+// passes on shared memory and eight cluster barriers.
+// --------------------------------------------------------------------------
+// A block holds at most 32 x 1024 entries, so the sums of 16-bit pieces of its weights fit 32 bits, whose atomics
+// on shared memory are single instructions (64-bit ones are loops: with them a top-k pass took twice as long).
+// The first digit of a selection is little more than the exponent: a warp's lanes share a few bins, and one of them
+// adds for all that share its bin.  Later digits are spread, and every lane adds for itself (with the first form
+// there too, top-p over 8 x 131,072 took 82 us).
+template <bool SHARED_BINS>
+__device__ __forceinline__ void part_add(uint32_t (*part)[256], int bin, u64 w) {
+  if (SHARED_BINS) {
+    if (!__any_sync(0xffffffffu, bin >= 0)) return;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    const uint32_t a = __reduce_add_sync(peers, (uint32_t)(w & 0xffffull));
+    const uint32_t b = __reduce_add_sync(peers, (uint32_t)((w >> 16) & 0xffffull));
+    const uint32_t c = __reduce_add_sync(peers, (uint32_t)(w >> 32));
+    if (bin >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+      atomicAdd(&part[0][bin], a);
+      atomicAdd(&part[1][bin], b);
+      atomicAdd(&part[2][bin], c);
+    }
+  } else if (bin >= 0) {
+    atomicAdd(&part[0][bin], (uint32_t)(w & 0xffffull));
+    atomicAdd(&part[1][bin], (uint32_t)((w >> 16) & 0xffffull));
+    atomicAdd(&part[2][bin], (uint32_t)(w >> 32));
+  }
+}
+template <bool SHARED_BINS>
+__device__ __forceinline__ void part_count(uint32_t (*part)[256], int bin) {
+  if (SHARED_BINS) {
+    if (!__any_sync(0xffffffffu, bin >= 0)) return;
+    const unsigned peers = __match_any_sync(0xffffffffu, bin);
+    if (bin >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&part[0][bin], (uint32_t)__popc(peers));
+  } else if (bin >= 0) {
+    atomicAdd(&part[0][bin], 1u);
+  }
+}
+
+struct ClusterShared {
+  uint32_t part[3][256];// the block's histogram as it grows: counts, or weights in pieces of 16, 16 and 9 bits
+  u64 hist[2][256];     // of this block; two in turn, so that one cluster barrier per exchange is enough
+  u64 word[2][2];       // two numbers of this block, in turn likewise
+  u64 pick[2];
+  SampleShared blk;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ u64 ld_peer_u64(const u64* local, uint32_t rank) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
+  uint32_t r;
+  u64 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(r) : "memory");
+  return v;
+}
+
+// What the blocks of a row exchange.  `turn` counts the exchanges of either kind: a buffer is written
+// again two exchanges later, when the barrier between has seen every block past its reads.
+struct RowCluster {
+  ClusterShared& sm;
+  uint32_t rank, size;
+  int turn;
+
+  // The sums over the row's blocks of two numbers, and of the first one over the blocks before this one.
+  // Every thread of a block passes the same numbers.
+  __device__ void sums(u64 a, u64 b, u64* before_a, u64* total_a, u64* total_b) {
+    u64* w = sm.word[turn & 1];
+    ++turn;
+    if (threadIdx.x == 0) { w[0] = a; w[1] = b; }
+    cluster_barrier();
+    u64 before = 0, ta = 0, tb = 0;
+    for (uint32_t r = 0; r < size; ++r) {
+      const u64 x = ld_peer_u64(w, r), y = ld_peer_u64(w + 1, r);
+      if (r < rank) before += x;
+      ta += x;
+      tb += y;
+    }
+    *before_a = before; *total_a = ta; *total_b = tb;
+  }
+  __device__ float max(float m) {
+    u64* w = sm.word[turn & 1];
+    ++turn;
+    if (threadIdx.x == 0) w[0] = (u64)__float_as_uint(m);
+    cluster_barrier();
+    for (uint32_t r = 0; r < size; ++r) m = fmaxf(m, __uint_as_float((uint32_t)ld_peer_u64(w, r)));
+    return m;
+  }
+  __device__ void clear() {
+    if (threadIdx.x < 256) sm.part[0][threadIdx.x] = sm.part[1][threadIdx.x] = sm.part[2][threadIdx.x] = 0u;
+    __syncthreads();
+  }
+  // The highest bin at which the sum from the top bin down, on top of `above`, reaches `target` (bin 0 if none
+  // does); `above` then holds what lies above that bin.  With `share` the target is that share of the whole.
+  __device__ int choose(u64& above, u64& target, float share, bool share_given) {
+    u64* h = sm.hist[turn & 1];
+    ++turn;
+    __syncthreads();
+    if (threadIdx.x < 256)
+      h[threadIdx.x] = (u64)sm.part[0][threadIdx.x] + ((u64)sm.part[1][threadIdx.x] << 16) +
+                       ((u64)sm.part[2][threadIdx.x] << 32);
+    cluster_barrier();
+    u64 v = 0;
+    if (threadIdx.x < 256)
+      for (uint32_t r = 0; r < size; ++r) v += ld_peer_u64(h + (255 - threadIdx.x), r);
+    u64 total;
+    const u64 inc = blk_scan(v, sm.blk, &total);
+    if (share_given) {
+      target = (u64)ceil((double)share * (double)total);
+      if (target > total) target = total;
+      if (target < 1ull) target = 1ull;
+    }
+    if (threadIdx.x == 255) { sm.pick[0] = 0ull; sm.pick[1] = above + inc - v; }   // bin 0 unless another one takes it
+    __syncthreads();
+    if (threadIdx.x < 255 && above + inc - v < target && above + inc >= target) {
+      sm.pick[0] = (u64)(255 - threadIdx.x);
+      sm.pick[1] = above + inc - v;
+    }
+    __syncthreads();
+    above = sm.pick[1];
+    const int bin = (int)sm.pick[0];
+    __syncthreads();
+    return bin;
+  }
+};
+
+template <int EPT>
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float temperature, int top_k,
+                      float top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+  __shared__ ClusterShared sm;
+  uint32_t rank, size;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+  RowCluster rc{sm, rank, size, 0};
+  const int tid = threadIdx.x;
+  const int r = blockIdx.x / size;
+  const float* row = logits + (size_t)r * ld;
+  const int i0 = ((int)rank * SAMPLE_THREADS + tid) * EPT;
+  pdl_wait();
+
+  // ---- the scaled logits, and their maximum
+  float z[EPT];
+  if (((uintptr_t)row & 15) == 0 && i0 + EPT <= V) {
+#pragma unroll
+    for (int e = 0; e < EPT; e += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(row + i0 + e);
+      z[e] = x.x; z[e + 1] = x.y; z[e + 2] = x.z; z[e + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) z[e] = i0 + e < V ? row[i0 + e] : 0.0f;
+  }
+  pdl_launch_dependents();
+  const int valid = min(max(V - i0, 0), EPT);     // this thread's entries
+  float m = -INFINITY;
+#pragma unroll
+  for (int e = 0; e < EPT; ++e) {
+    z[e] = z[e] / temperature;
+    if (e < valid && z[e] == z[e]) m = fmaxf(m, z[e]);
+  }
+  m = rc.max(blk_max(m, sm.blk));
+  if (!(m - m == 0.0f)) {
+    // no finite maximum (an infinite logit, or none that is a number): the weights are no numbers; one block
+    // walks the row, so that what comes out does not depend on the kernel
+    if (rank == 0) sample_row(row, V, temperature, top_k, top_p, uniform[r], out + r, sm.blk);
+    cluster_barrier();   // no block leaves while another reads its shared memory
+    return;
+  }
+
+  // ---- top-k: key of the k-th largest scaled logit by radix selection
+  const bool use_k = top_k > 0 && top_k < V;
+  uint32_t dropped = 0;                           // bit e: not among the k largest
+  if (use_k) {
+    uint32_t prefix = 0u, mask = 0u;
+    u64 above = 0, target = (u64)top_k;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      rc.clear();
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) {
+        const uint32_t k = float_key(z[e]);
+        const int bin = (e < valid && (k & mask) == prefix) ? (int)((k >> shift) & 255u) : -1;
+        if (shift == 24) part_count<true>(sm.part, bin);
+        else part_count<false>(sm.part, bin);
+      }
+      prefix |= (uint32_t)rc.choose(above, target, 0.0f, false) << shift;
+      mask |= 255u << shift;
+    }
+    // target - above entries equal to the threshold are kept, lowest indices first
+    u64 equal = 0, total, before, all, unused;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) equal += (e < valid && float_key(z[e]) == prefix) ? 1ull : 0ull;
+    u64 inc = blk_scan(equal, sm.blk, &total);
+    rc.sums(total, 0ull, &before, &all, &unused);
+    u64 at = before + inc - equal;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const uint32_t k = float_key(z[e]);
+      if (k < prefix || (k == prefix && e < valid && at >= target - above)) dropped |= 1u << e;
+      if (k == prefix && e < valid) ++at;
+    }
+  }
+
+  // ---- weights of the kept entries; from here z[e] is exp(z - max), 0 where nothing is kept
+#pragma unroll
+  for (int e = 0; e < EPT; ++e) z[e] = (e < valid && z[e] == z[e] && !(dropped >> e & 1)) ? expf(z[e] - m) : 0.0f;
+  auto weight = [](float e) { return (u64)(e * FIX_ONE); };
+
+  // ---- top-p: the largest weight w such that the weights of w and above reach the share, by radix selection on
+  // the bits of exp(z - max), which are in the order of the weights
+  u64 S = 0;
+  const bool use_p = top_p > 0.0f && top_p < 1.0f;
+  if (use_p) {
+    uint32_t prefix = 0u, mask = 0u;
+    u64 above = 0, target = 0;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      rc.clear();
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) {
+        const uint32_t k = __float_as_uint(z[e]);
+        const u64 w = weight(z[e]);
+        const int bin = (w != 0ull && (k & mask) == prefix) ? (int)((k >> shift) & 255u) : -1;
+        if (shift == 24) part_add<true>(sm.part, bin, w);
+        else part_add<false>(sm.part, bin, w);
+      }
+      prefix |= (uint32_t)rc.choose(above, target, top_p, shift == 24) << shift;
+      mask |= 255u << shift;
+    }
+    // small exponentials share a weight: ties are ties of the weight
+    const u64 thr = weight(__uint_as_float(prefix));
+    u64 over = 0, equal = 0, total, before, all, over_all;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const u64 w = weight(z[e]);
+      over += w > thr ? w : 0ull;
+      equal += (w == thr && thr != 0ull) ? 1ull : 0ull;
+    }
+    blk_scan(over, sm.blk, &over_all);
+    const u64 inc = blk_scan(equal, sm.blk, &total);
+    rc.sums(total, over_all, &before, &all, &above);
+    u64 need = 0;
+    if (thr > 0ull) {
+      need = target > above ? (target - above + thr - 1ull) / thr : 1ull;
+      if (need < 1ull) need = 1ull;
+    }
+    u64 at = before + inc - equal;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const u64 w = weight(z[e]);
+      if (w < thr || (w == thr && at >= need)) z[e] = 0.0f;
+      if (w == thr && thr != 0ull) ++at;
+    }
+    S = above + need * thr;
+  }
+
+  // ---- draw: first kept index whose running weight exceeds floor(u * S)
+  u64 mine = 0, total, before, all, unused;
+#pragma unroll
+  for (int e = 0; e < EPT; ++e) mine += weight(z[e]);
+  const u64 inc = blk_scan(mine, sm.blk, &total);
+  rc.sums(total, 0ull, &before, &all, &unused);
+  if (!use_p) S = all;
+  float u = uniform[r];
+  u = u < 0.0f ? 0.0f : (u >= 1.0f ? 0.99999994f : u);
+  u64 target = (u64)((double)u * (double)S);
+  if (target >= S) target = S ? S - 1ull : 0ull;
+  u64 run = before + inc - mine;
+  if (mine && run + mine > target && run <= target) {   // the crossing lies in this thread's entries
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const bool ahead = run <= target;
+      run += weight(z[e]);
+      if (ahead && run > target) out[r] = i0 + e;
+    }
+  }
+  cluster_barrier();   // no block leaves while another reads its shared memory
+}
+
+template <int EPT>
+static int launch_sample_cluster(int blocks_per_row, const float* logits, int ld, int rows, int V, float temperature,
+                                 int top_k, float top_p, const float* uniform, int* out, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(rows * blocks_per_row);
+  cfg.blockDim = dim3(SAMPLE_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks_per_row;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<EPT>, logits, ld, V, temperature, top_k, top_p,
+                                     uniform, out);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// One block per row, any vocabulary.  temperature must be > 0.
+extern "C" int tl_sample_walk(const float* logits, int ld, int rows, int V, float temperature, int top_k,
+                              float top_p, const float* uniform, int* out, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (V <= 0 || !(temperature > 0.0f)) return -1;
+  return tl_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V,
+                   temperature, top_k, top_p, uniform, out);
 }
 
 // temperature must be > 0; rows with temperature <= 0 go through tl_argmax.
+#define SAMPLE_MAX_CLUSTER 8   // portable cluster size
 extern "C" int tl_sample(const float* logits, int ld, int rows, int V, float temperature,
                          int top_k, float top_p, const float* uniform, int* out,
                          cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (V <= 0 || !(temperature > 0.0f)) return -1;
-  return tl_launch(sample_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V,
-                   temperature, top_k, top_p, uniform, out);
+  // As many blocks per row as give a thread four entries, at most 8 and no more than run at once (a block fills an
+  // SM), but enough that 32 entries per thread cover the row: a pass costs what a thread holds, a barrier of eight
+  // blocks little more than one of two, and a second round of blocks as much as the first.
+  int blocks = 1;
+  while (blocks < SAMPLE_MAX_CLUSTER && blocks * SAMPLE_THREADS * 4 < V &&
+         (blocks * SAMPLE_THREADS * 32 < V || (long long)rows * blocks * 2 <= 148))
+    blocks *= 2;
+  const int per = (V + blocks * SAMPLE_THREADS - 1) / (blocks * SAMPLE_THREADS);
+#define SAMPLE_CLUSTER(EPT_) \
+  return launch_sample_cluster<EPT_>(blocks, logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream)
+  if (per <= 4) SAMPLE_CLUSTER(4);
+  if (per <= 8) SAMPLE_CLUSTER(8);
+  if (per <= 16) SAMPLE_CLUSTER(16);
+  if (per <= 32) SAMPLE_CLUSTER(32);
+#undef SAMPLE_CLUSTER
+  return tl_sample_walk(logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream);
 }
 
 TL_TRACE_EXPORT(sampling)
