@@ -18,7 +18,7 @@
 // cycles of arithmetic (bound by the 16 exponentials a cycle of an SM when two blocks share
 // it), 450 for the P stores and the proxy fence that the tensor core's reads of shared memory
 // need (what moving P to tensor memory saves), 200 for the barrier; issuing one tcgen05.mma
-// costs its thread about 80 cycles.
+// cost its thread about 80 cycles before it was chosen by elect_one (umma.cuh).
 // Arithmetic as in attention_prefill_bf16.cu (reference: src/model/modules/attention.rs:88-121,
 // src/model/modules/flash_attention.rs:101-136, window of src/model/models/gpt_oss.rs:168-176).
 // Head sizes 64 and 128.
@@ -29,6 +29,7 @@
 #include <stdlib.h>
 
 #include "attention_bf16_common.cuh"
+#include "umma.cuh"
 
 #include <map>
 #include <mutex>
@@ -117,8 +118,6 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -268,7 +267,7 @@ FN(attn_prefill_tc_kernel)(const __grid_constant__ CUtensorMap tm_q, const __gri
   const int ps = blk_lo / PAGE;
   const int n_pg = blk_last / PAGE - ps + 1;
 
-  if (warp == 4 && lane == 0) {
+  if (warp == 4 && elect_one()) {
     // ---- TMA producer: the block's queries once, then the pages
     tc_mbar_expect_tx(q_full, TC_Q_BYTES);
 #pragma unroll
@@ -292,8 +291,8 @@ FN(attn_prefill_tc_kernel)(const __grid_constant__ CUtensorMap tm_q, const __gri
         tc_tma_load_2d(v_s + (size_t)s * TC_V_BYTES, &tm_v, &v_full[s], 0, slab * HEAD_DIM);
       }
     }
-  } else if ((warp == 5 || warp == 6) && lane == 0) {
-    // ---- two MMA issuers.  Issuing costs some 80 cycles an instruction, twelve instructions a
+  } else if ((warp == 5 || warp == 6) && elect_one()) {
+    // ---- two MMA issuers.  Issuing cost some 80 cycles an instruction (see above), twelve instructions a
     // page, so one thread (warp 5) issues Q . K^T and another (warp 6) P . V.  A descriptor is a
     // constant high word and a low word = (address >> 4) | 1 << 16.
     const uint32_t idesc_s = tc_idesc(PAGE), idesc_o = tc_idesc(HEAD_DIM);

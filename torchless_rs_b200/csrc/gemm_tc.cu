@@ -13,8 +13,9 @@
 // costs nothing that matters) and more tokens (up to BN = 256; from 129 tokens on the
 // kernel on pairs of SMs further down takes over).  Operands come by TMA into
 // 128-byte-swizzled shared memory tiles of 64 K-elements, one or two of them per operand
-// and stage; one thread issues the instructions (each costs it some 70 cycles, a stage's
-// barrier wait, commit and loop some 400, which is why a stage holds eight instructions);
+// and stage; one thread issues the instructions (a stage's barrier
+// wait, commit and loop cost it some 400 cycles, which is why a stage holds eight instructions;
+// elect_one says what an instruction costs);
 // four warps read the accumulator back with tcgen05.ld and write C, each warp-store
 // covering 32 consecutive columns of one row of C.
 //
@@ -36,6 +37,7 @@
 #include <stdint.h>
 #include "bounded_wait.cuh"
 #include "pdl.cuh"
+#include "umma.cuh"
 
 #include <map>
 #include <mutex>
@@ -54,104 +56,10 @@
 
 __device__ int tl_gemm_tc_error = 0;
 
-// ---------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return tl_smem_u32(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) { tl_mbar_init(bar, count); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
 // Bounded wait (bounded_wait.cuh).  Returns false when the bound is hit or another role has given up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int code) {
   return tl_mbar_wait(bar, parity, abort_flag, code, &tl_gemm_tc_error);
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
-      "{%3, %4}], [%2];"
-      :
-      : "r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(slot)),
-               "r"(cols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols)
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The mbarrier gets one arrival when all tcgen05.mma issued so far by this thread are done.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-      "%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared memory matrix descriptor of a K-major tile whose rows are 128 bytes with the
-// 128-byte swizzle: 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_k128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);   // start address, 16-byte units
-  d |= (uint64_t)1 << 16;                     // leading byte offset (unused with a swizzle)
-  d |= (uint64_t)(1024 >> 4) << 32;           // stride byte offset between 8-row groups
-  d |= (uint64_t)1 << 46;                     // descriptor version of sm_100
-  d |= (uint64_t)2 << 61;                     // SWIZZLE_128B
-  return d;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ float ld_remote_f32(uint32_t local_saddr, uint32_t rank) {
-  uint32_t raddr;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"(local_saddr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(raddr) : "memory");
-  return v;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
@@ -285,7 +193,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) pdl_launch_dependents();
 
-  if (warp == 4 && lane == 0) {
+  if (warp == 4 && elect_one()) {
     // ---- TMA producer.  The weights do not depend on earlier kernels, so the tiles of the
     // first stages are requested before the wait for those kernels; the activations after it.
     const int pre = n_kb < stages ? n_kb : stages;
@@ -325,7 +233,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       load_x(st, &full_bar[s], kof(i));
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5 && elect_one()) {
     // ---- MMA issuer
     bool ok = true;
     int s = 0;
@@ -778,7 +686,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w,
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) pdl_launch_dependents();
 
-  if (warp == 4 && lane == 0) {
+  if (warp == 4 && elect_one()) {
     // ---- TMA producer: one ring of stages across all tiles of this block
     bool waited = false;
     uint32_t it = 0;
@@ -797,7 +705,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_w,
         tma_load_2d(st + A_BYTES * (SWIGLU ? 2 : 1), &tm_x, &full_bar[s], k, m0);
       }
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5 && elect_one()) {
     // ---- MMA issuer
     uint32_t it = 0, local = 0;
     bool ok = true;
@@ -1030,7 +938,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w,
   const uint32_t tmem_base = *tmem_slot;
   if (threadIdx.x == 0) pdl_launch_dependents();
 
-  if (warp == 4 && lane == 0) {
+  if (warp == 4 && elect_one()) {
     // ---- TMA producer of this block's halves; the bytes count at the first block's barrier
     bool waited = false;
     int s = 0;
@@ -1065,7 +973,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_w,
         if (++s == stages) { s = 0; ph ^= 1u; }
       }
     }
-  } else if (warp == 5 && lane == 0 && rank == 0) {
+  } else if (warp == 5 && rank == 0 && elect_one()) {
     // ---- MMA issuer of the pair
     uint32_t local = 0, ph = 0;
     int s = 0;
