@@ -73,7 +73,7 @@ def test_silu_mul(dtype):
 # ---------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("M,N,K", [(1, 50, 33), (3, 129, 72), (8, 64, 4096), (9, 65, 100),
-                                   (70, 200, 177), (130, 31, 64)])
+                                   (70, 200, 177), (130, 31, 64), (3, 4097, 72), (4, 4096, 520), (5, 2051, 64), (8, 4099, 1024)])
 def test_gemm_generic(dtype, M, N, K):
     from torchless_rs_b200.csrc import ops
     o = _ops(dtype)
@@ -96,6 +96,75 @@ def test_gemm_generic(dtype, M, N, K):
     o.gemm_generic(a, w, c4, ops.MODE_SWIGLU)
     up = ad @ wd[N:].T
     assert torch.allclose(c4.double(), ref / (1 + torch.exp(-ref)) * up, **tol)
+
+
+@pytest.mark.parametrize("M,N,K", [(4, 1024, 1024), (8, 200, 5120), (16, 1100, 1024), (96, 1027, 1056), (97, 1027, 1056), (17, 1027, 1500), (64, 640, 2052), (65, 640, 2048),
+                                   (192, 1028, 1024), (193, 700, 1600), (531, 320, 4096), (300, 96, 14336)])
+def test_gemm_split_is_no_further_off_than_the_cuda_core_kernel(M, N, K):
+    """32-bit products on tensor cores, at the edges of tiles (64 and 128 rows of weights, 16 to 192 tokens), of K
+    (stages of 32, several splits) and with strided rows.  Bound, per output: a sum of 16 leading products is cut 16 times,
+    K / 64 such sums are rounded, and the small products (2^-8) are cut 5 K / 16 times, each by 2^-23 at most."""
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    g, o, ws = GemmF32.get(), _ops(torch.float32), Workspace(torch.device(DEV))
+    assert GemmF32.takes(M, N, K) or N * K < 1 << 20
+    g_takes, GemmF32.takes = GemmF32.takes, staticmethod(lambda *a: True)
+    try:
+        for pad in (0, 3):       # rows of X and C that do not start on 16 bytes
+            a = _rand((M, K + pad), torch.float32, 5)[:, :K]
+            w = _rand((2 * N, K), torch.float32, 6, 1.0 / math.sqrt(K))
+            ad, wd = a.double(), w.double()
+            ref, up = ad @ wd[:N].T, ad @ wd[N:].T
+            size = ad.abs() @ wd[:N].abs().T
+            bound = (16 + 8 + K / 64 + 5 * K / 16 / 256) * 2.0 ** -23 * size
+            base = _rand((M, N + pad), torch.float32, 7)[:, :N]
+            for mode in (ops.MODE_STORE_F32, ops.MODE_ACCUM_F32, ops.MODE_STORE_ACT, ops.MODE_SWIGLU):
+                c, plain = base.clone(), base.clone()
+                if pad:
+                    c = torch.zeros((M, N + pad), device=DEV)[:, :N].copy_(base)
+                x = w if mode == ops.MODE_SWIGLU else w[:N]
+                assert g.run(a, x, c, mode, ws)
+                o.gemm_generic(a, x, plain, mode)
+                if mode == ops.MODE_SWIGLU:
+                    want = ref / (1 + torch.exp(-ref)) * up
+                    assert torch.allclose(c.double(), want, rtol=1e-5, atol=1e-4)
+                else:
+                    want = ref + base.double() if mode == ops.MODE_ACCUM_F32 else ref
+                    assert ((c.double() - want).abs() <= bound + 2.0 ** -23 * want.abs()).all()
+                # (the sum of squares of a few hundred outputs and more; a fifth for chance)
+                err = [float((y.double() - want).norm()) for y in (c, plain)]
+                assert err[0] <= 1.2 * err[1], (mode, err)
+        assert g.take_error() == 0
+    finally:
+        GemmF32.takes = staticmethod(g_takes)
+
+
+def test_gemm_split_gives_what_the_cuda_core_kernel_gives_where_results_are_not_finite():
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    g, o, ws = GemmF32.get(), _ops(torch.float32), Workspace(torch.device(DEV))
+    M, N, K = 40, 2048, 1024
+    inf, nan, big = float("inf"), float("nan"), 3.4e38
+    for where, value in (("x", inf), ("x", -inf), ("x", nan), ("x", big), ("w", inf), ("w", nan), ("w", -big), ("both", 2e38)):
+        a = _rand((M, K), torch.float32, 8)
+        w = _rand((2 * N, K), torch.float32, 9, 1.0 / math.sqrt(K))
+        if where in ("x", "both"):
+            a[3, 700] = value
+        if where in ("w", "both"):
+            w[900, 700] = value
+            w[N + 5, 1] = value
+        for mode in (ops.MODE_STORE_F32, ops.MODE_ACCUM_F32, ops.MODE_SWIGLU):
+            c, plain = torch.ones((M, N), device=DEV), torch.ones((M, N), device=DEV)
+            x = w if mode == ops.MODE_SWIGLU else w[:N]
+            assert g.run(a, x, c, mode, ws)
+            o.gemm_generic(a, x, plain, mode)
+            assert torch.equal(c.isnan(), plain.isnan()) and torch.equal(c.isinf(), plain.isinf()), (where, value, mode)
+            ok = plain.isfinite()
+            assert torch.equal(torch.where(plain.isinf(), plain, 0.0), torch.where(c.isinf(), c, 0.0))
+            # an operand near the largest number meets others of size 1: relative to what the row holds
+            assert torch.allclose(c[ok], plain[ok], rtol=1e-4, atol=1e-3), (where, value, mode)
 
 
 # ---------------------------------------------------------------------------

@@ -41,3 +41,26 @@ __device__ __forceinline__ bool tl_mbar_wait(uint64_t* bar, uint32_t parity, vol
   atomicCAS(error_word, 0, code);
   return false;
 }
+
+// The same for roles with many waiting threads beside threads that compute: the hardware parks a waiting warp
+// (try_wait) for some microseconds at most instead of letting it poll, so it takes no issue slots.  One look in 64
+// at the flag; the limit is as many fewer looks as a look is longer.
+__device__ __forceinline__ bool tl_mbar_park(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
+                                             int* error_word) {
+  const uint32_t a = tl_smem_u32(bar);
+  for (uint32_t i = 0; i < TL_WAIT_LIMIT / 16; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((i & 63u) == 63u && *abort_flag) return false;
+  }
+  *abort_flag = code;
+  atomicCAS(error_word, 0, code);
+  return false;
+}

@@ -1,0 +1,74 @@
+"""Products of the true 32-bit path on tensor cores (kernels in gemm_split.cu).  `run` returns False for a shape it
+does not take; the caller then uses the CUDA-core kernel."""
+from __future__ import annotations
+
+from ctypes import c_int, c_longlong, c_void_p
+
+import torch
+
+from . import build
+from .ops import MODE_SWIGLU, KernelError, _check, _stream, register_error_word
+
+build.register_library("gemm_split", ("gemm_split.cu",), ())
+
+
+class GemmF32:
+    _inst = None
+
+    @classmethod
+    def get(cls) -> "GemmF32":
+        if cls._inst is None:
+            cls._inst = cls()
+        return cls._inst
+
+    def __init__(self):
+        self.lib = build.load_library("gemm_split")
+        P, I = c_void_p, c_int
+        self.lib.tl_gemm_split.restype = c_int
+        self.lib.tl_gemm_split.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P, P]
+        self.lib.tl_gemm_split_scratch.restype = c_longlong
+        self.lib.tl_gemm_split_scratch.argtypes = [I, I]
+        self.lib.tl_gemm_split_take_error.restype = c_int
+        register_error_word("gemm_split", self.take_error)
+        self._sms = {}
+
+    @staticmethod
+    def takes(M: int, N: int, K: int) -> bool:
+        """Up to three rows the CUDA-core kernel reads the weights at the copy rate or near it (three rows of 6144 x
+        4096: 30 us here and there; four rows of 4096 x 4096 19 us there, 21 here, of 6144 x 4096 38 and 32; eight rows of
+        4096 x 1024 16 and 17, of 4096 x 2048 26 and 18).  From nine rows on it is several times slower, until the
+        launch more that is made here costs what the product does.  Below 1024 elements its sums are so short that
+        they are nearer to the exact result."""
+        least = 1 << 20 if M > 8 else (6 << 20 if M > 4 else 20 << 20)
+        return M >= 4 and K >= 1024 and N * K >= least
+
+    def run(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, workspace) -> bool:
+        """out (op)= a @ w.T, all 32-bit.  `workspace` gives the buffer for a's pieces."""
+        M, K = a.shape
+        N = out.shape[1]
+        if not self.takes(M, N, K) or a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32:
+            return False
+        if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
+            return False
+        if w.shape != ((2 * N if mode == MODE_SWIGLU else N), K) or out.shape[0] != M:
+            raise KernelError(f"gemm: shapes do not fit: a {tuple(a.shape)} w {tuple(w.shape)} out {tuple(out.shape)} "
+                              f"mode {mode}")
+        for t in (a, w, out):
+            if not t.is_cuda:
+                raise KernelError("kernel argument is not on a CUDA device; this package has no CPU path")
+        key = a.device.index if a.device.index is not None else torch.cuda.current_device()
+        if key not in self._sms:
+            self._sms[key] = torch.cuda.get_device_properties(a.device).multi_processor_count
+        n = int(self.lib.tl_gemm_split_scratch(M, K))
+        scratch = workspace.get("gemm_split_pieces", ((n + 3) // 4,), torch.int32)
+        st = self.lib.tl_gemm_split(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
+                                    M, N, K, mode, self._sms[key], scratch.data_ptr(), _stream())
+        if st == -2:
+            return False
+        _check(st, "gemm_split")
+        _check(0, "split_rows")      # the kernel before it counts too
+        return True
+
+    def take_error(self) -> int:
+        """Nonzero if a kernel gave up on a bounded wait since the last call (synchronises)."""
+        return int(self.lib.tl_gemm_split_take_error())

@@ -3,5 +3,6 @@ lists all of them (used by the build check; at run time a library is built when 
 model first needs it)."""
 from . import build  # noqa: F401
 from . import gemm_bf16  # noqa: F401
+from . import gemm_f32  # noqa: F401
 from . import attention_bf16  # noqa: F401
 from . import sink_attention_bf16  # noqa: F401

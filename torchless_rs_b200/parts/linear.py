@@ -1,7 +1,8 @@
 """Matrix products of the parts: picks the kernel for a shape.
 
-`out (op)= a @ w.T` with 32-bit accumulation.  In 32-bit everything runs on the
-CUDA-core kernels.  In bfloat16 the tensor-core kernels take the shapes they are
+`out (op)= a @ w.T` with 32-bit accumulation.  In 32-bit a few rows, small matrices and odd shapes run on
+the CUDA-core kernels, the rest on tensor cores with three bfloat16 numbers for each 32-bit one (nearer to the exact
+result than the CUDA-core kernels are).  In bfloat16 the tensor-core kernels take the shapes they are
 built for and the CUDA-core kernels take the rest; which kernel ran never changes
 what is computed, only its rounding order.
 """
@@ -35,8 +36,11 @@ def new_carry(rt: Runtime, name: str, n_tokens: int, size: int, eps: float) -> N
 class Matmul:
     def __init__(self, rt: Runtime):
         self.rt = rt
-        self.fast = None
-        if not rt.is_f32:
+        self.fast = self.split = None
+        if rt.is_f32:
+            from ..csrc import gemm_f32
+            self.split = gemm_f32.GemmF32.get()
+        else:
             from ..csrc import gemm_bf16
             self.fast = gemm_bf16.GemmBf16.get()
 
@@ -54,7 +58,8 @@ class Matmul:
             emit[1].valid = False
         if self.fast is not None and self.fast.run(a, w, out, mode, emit=emit, rope=rope):
             return self.fast.rope_applied
-        self.rt.ops.gemm_generic(a, w, out, mode)
+        if self.split is None or not self.split.run(a, w, out, mode, self.rt.workspace):
+            self.rt.ops.gemm_generic(a, w, out, mode)
         return False
 
     def activated(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, act) -> bool:
