@@ -515,6 +515,72 @@ def test_attention_prefill_tc_many_blocks_repeated(nh, nkv, hd, window, lens, ne
         assert torch.allclose(out.double().view(T, nh, hd), ref, **_attn_tol(dtype)), f"repetition {rep}"
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window", [(4, 2, 16, 16), (3, 1, 32, None), (8, 8, 64, 100), (16, 2, 64, None), (12, 1, 128, 64),
+                                               (6, 2, 128, None), (8, 2, 128, 65), (64, 1, 32, 7)])
+def test_attention_f32_prompts_and_decode(nh, nkv, hd, window):
+    """The 32-bit kernels of the common head sizes: sequences from their start, going on, and of one token, with groups that
+    do and do not divide the tile, page borders, and values of other tokens of the page that must not reach a
+    query; decode steps with every number of pages per block."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc import attention_f32 as f32
+    from torchless_rs_b200.parts.runtime import Workspace
+    o, ws, att = _ops(torch.float32), Workspace(torch.device(DEV)), f32.AttentionF32.get(hd)
+    scale = 1 / math.sqrt(hd)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def check(lens, new, decode, plan=None):
+        pc = Paged(lens, nkv, hd, torch.float32, 20 + hd)
+        T = sum(new)
+        q = _rand((T, nh * hd), torch.float32, 21)
+        starts = [sum(new[:b]) for b in range(len(new) + 1)]
+        batch = SimpleNamespace(is_decode=decode, n_seqs=len(lens), len_bucket=max(256, 1 << (max(lens) - 1).bit_length()),
+                                total_bucket=sum(lens), max_new=max(new), seq_start=i32(starts), seq_len=i32(lens),
+                                seq_slot=pc.seq_slot)
+        view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
+        out = torch.full((T, nh * hd), float("nan"), device=DEV)
+        keep = f32.decode_split
+        if plan is not None:
+            f32.decode_split = plan
+        try:
+            ran = att.run(q, view, out, batch, nh, nkv, window, scale, ws)
+        finally:
+            f32.decode_split = keep
+        assert ran == (not decode or nh // nkv <= f32.MAX_GROUP_DECODE)
+        if not ran:
+            return
+        qc, got = q.cpu().view(T, nh, hd), out.cpu().double().view(T, nh, hd)
+        for b, n in enumerate(new):
+            for t in range(n):
+                at = starts[b] + t
+                ref = attention_reference(qc[at], pc.k[b], pc.v[b], lens[b] - n + t, window, scale)
+                assert torch.allclose(got[at], ref, **_attn_tol(torch.float32)), (b, t)
+    check([70, 200, 131, 64, 1], [70, 5, 1, 64, 1], False)
+    check([130], [129], False)
+    check([1, 64, 65, 300, 128], [1] * 5, True)
+    for per in (1, 2, 3, 16):
+        check([257, 40, 300], [1] * 3, True, lambda *a, per=per: (per, -(-512 // 64 // per) + 1))
+
+
+@pytest.mark.parametrize("poison", [float("inf"), float("nan")])
+def test_attention_f32_keeps_unseen_values_out(poison):
+    """A later token's value that is no number reaches the queries that see it and no other."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc.attention_f32 import AttentionF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    nh, nkv, hd, n, bad = 4, 2, 64, 100, 80
+    pc = Paged([n], nkv, hd, torch.float32, 5)
+    page = int(pc.table[pc.slots[0], bad // PAGE])
+    pc.v_pages[page, :, :, bad % PAGE] = poison
+    q = _rand((n, nh * hd), torch.float32, 6)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(is_decode=False, n_seqs=1, len_bucket=256, total_bucket=256, max_new=n, seq_start=i32([0, n]),
+                            seq_len=i32([n]), seq_slot=pc.seq_slot)
+    out = torch.empty((n, nh * hd), device=DEV)
+    view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
+    assert AttentionF32.get(hd).run(q, view, out, batch, nh, nkv, None, 0.125, Workspace(torch.device(DEV)))
+    assert out[:bad].isfinite().all() and not out[bad:].isfinite().any()
+
+
 @pytest.mark.parametrize("kernel", ["prefill_bf16_tc", "prefill_bf16_tma", "prefill_bf16_plain", "generic_bf16",
                                     "generic_f32"])
 def test_attention_far_key_stands_out_in_every_kernel(kernel):

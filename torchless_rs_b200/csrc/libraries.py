@@ -4,5 +4,6 @@ model first needs it)."""
 from . import build  # noqa: F401
 from . import gemm_bf16  # noqa: F401
 from . import gemm_f32  # noqa: F401
+from . import attention_f32  # noqa: F401
 from . import attention_bf16  # noqa: F401
 from . import sink_attention_bf16  # noqa: F401

@@ -55,8 +55,10 @@ class Attention:
         self.w_qkv: Optional[torch.Tensor] = None
         self.w_o: Optional[torch.Tensor] = None
         self.cache = None
-        self.fast = None
-        if not rt.is_f32:
+        if rt.is_f32:
+            from ..csrc import attention_f32
+            self.fast = attention_f32.AttentionF32.get(self.hd)
+        else:
             from ..csrc import attention_bf16
             self.fast = attention_bf16.AttentionBf16.get(self.hd)
 
@@ -97,7 +99,7 @@ class Attention:
         q = ws.get("attn_q", (T, self.nh * self.hd), rt.act_dtype)
         pos = self.position
         rope = None
-        if self.fast is not None and self.own_cache:
+        if not rt.is_f32 and self.fast is not None and self.own_cache:
             # the product may rotate and write q, k and v itself (it does when K is split)
             from ..csrc.gemm_bf16 import RopeArgs
             rope = RopeArgs(q.data_ptr(), c.k_pages.data_ptr(), c.v_pages.data_ptr(),
