@@ -22,6 +22,11 @@ from .registry import register_feed_forward
 from .runtime import Runtime
 
 
+def _grouped_rows(rt: Runtime, rows: int, hidden: int) -> Optional[torch.Tensor]:
+    """Room for the experts' input rows in the grouped order; the 32-bit kernel reads them where they lie."""
+    return None if rt.is_f32 else rt.workspace.get("moe_rows", (rows, hidden), rt.act_dtype)
+
+
 @register_feed_forward("moe_clamped")
 class ClampedMoE:
     """Parameters: `hidden_size`, `ff` (an expert's inner size), `experts`, `identity`, `top`, `limit`,
@@ -80,8 +85,8 @@ class ClampedMoE:
         if E:
             act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
             rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, limit=self.limit,
-                            alpha=self.gate_alpha)
-            rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False)
+                            alpha=self.gate_alpha, grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+            rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         rt.ops.moe_combine(yk, row_of, wt, xn, residual, accumulate=not overwrite)
 
 
@@ -162,8 +167,9 @@ class GroupedSigmoidMoE:
         rt.ops.moe_plan(idx, E, offsets, row_token, row_of)
         yk = ws.get("moe_expert_out", (T * top, self.hidden), torch.float32)
         act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
-        rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, limit=self.limit, alpha=self.gate_alpha)
-        rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False)
+        rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, limit=self.limit, alpha=self.gate_alpha,
+                        grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+        rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         rt.ops.moe_combine(yk, row_of, wt, xn, residual, accumulate=not overwrite)
         if self.shared_ff:
             sact = ws.get("moe_shared_act", (T, self.shared_ff), rt.act_dtype)
@@ -252,8 +258,9 @@ class SoftmaxChosenMoE:
         rt.ops.moe_plan(idx, E, offsets, row_token, row_of)
         yk = ws.get("moe_expert_out", (T * top, self.hidden), torch.float32)
         act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
-        rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, act=ops.ACT_PLAIN)
-        rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False)
+        rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, act=ops.ACT_PLAIN,
+                        grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+        rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         if not self.shared_ff:
             return (yk, row_of, wt), None
         sact = ws.get("moe_shared_act", (T, self.shared_ff), rt.act_dtype)
