@@ -451,3 +451,47 @@ def test_headwise_products(dtype, M, heads, N, K):
     refg = ref.reshape(M, heads * N) / (1 + np.exp(-g64))
     tol = 1e-4 if dtype == torch.float32 else 2e-2 * np.abs(refg).max()
     assert np.abs(cg.float().cpu().numpy() - refg).max() <= tol
+
+
+@pytest.mark.parametrize("lens,new,heads,rot,dims,window,sink", [
+    ([64], [64], 16, 64, 64, None, False), ([300, 70, 129], [300, 5, 64], 16, 64, 32, None, True),
+    ([300, 70, 129], [129, 70, 1], 32, 32, 32, 100, False), ([300, 70], [200, 70], 5, 0, 0, 70, True),
+    ([500], [333], 128, 16, 16, None, False), ([400], [333], 1, 64, 64, 64, False), ([700], [130], 24, 48, 30, 300, True)])
+def test_latent_attention_of_prompts_on_tensor_memory(lens, new, heads, rot, dims, window, sink):
+    """The kernel for prompts against the one for every step: numbers of heads that do and do not divide the tile,
+    rotated parts of every width, windows, sinks, several sequences, some going on.  Both round the weights to
+    bfloat16 (2^-9 each), so an output differs by at most 2^-8 of the largest value, and a little for the scores' 32-bit
+    sums in another order."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.latent_bf16 import LatentBf16
+    from torchless_rs_b200.parts.runtime import Workspace
+    o, ws, rank, T, B = ops.core_ops(torch.bfloat16), Workspace(torch.device("cuda:0")), 512, sum(new), len(lens)
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    need = [-(-n // 64) for n in lens]
+    pages = torch.randn((sum(need) + 2, 64, rank + rot), device="cuda", generator=g).to(torch.bfloat16)
+    order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(3)).tolist()
+    slots = list(range(B, 0, -1))
+    table = torch.full((B + 1, max(need)), -1, dtype=torch.int32)
+    for b in range(B):
+        table[slots[b], :need[b]] = torch.tensor([order.pop() for _ in range(need[b])], dtype=torch.int32)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    q = torch.randn((T, heads * (rank + rot)), device="cuda", generator=g) * 0.3
+    batch = SimpleNamespace(is_decode=False, n_seqs=B, max_new=max(new), seq_start=i32([sum(new[:b]) for b in range(B + 1)]))
+    inv = 1e4 ** (-torch.arange(max(dims // 2, 1), device="cuda").float() * 2 / max(dims, 1))
+    sinks = torch.randn(heads, device="cuda", generator=g) if sink else None
+    args = (q, rank + rot, q, rank + rot, rank, pages)
+    rest = (i32(sum([list(range(n - m, n)) for n, m in zip(lens, new)], [])), i32(sum([[b] * m for b, m in enumerate(new)], [])),
+            i32(slots), table.cuda(), inv, heads, rank, rot, dims, window, 0.07)
+    a, c = torch.full((T, heads, rank), float("nan"), device="cuda"), torch.empty((T, heads, rank), device="cuda")
+    keep, LatentBf16.FROM_ROWS = LatentBf16.FROM_ROWS, 0
+    try:
+        before = ops.launch_counts().get("latent_attn_tc", 0)
+        o.latent_attn(*args, a, *rest, max_keys=max(lens), workspace=ws, sink=sinks, amplitude=1.1, batch=batch)
+        assert ops.launch_counts().get("latent_attn_tc", 0) == before + 1
+    finally:
+        LatentBf16.FROM_ROWS = keep
+    o.latent_attn(*args, c, *rest, max_keys=max(lens), workspace=ws, sink=sinks, amplitude=1.1)
+    assert LatentBf16.get().take_error() == 0
+    assert (a - c).abs().max() <= 2.0 ** -8 * pages.float().abs().max() * 1.05
+    assert (a - c).norm() <= 4e-3 * c.norm()

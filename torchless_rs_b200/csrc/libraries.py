@@ -6,5 +6,6 @@ from . import gemm_bf16  # noqa: F401
 from . import gemm_f32  # noqa: F401
 from . import attention_f32  # noqa: F401
 from . import moe_bf16  # noqa: F401
+from . import latent_bf16  # noqa: F401
 from . import attention_bf16  # noqa: F401
 from . import sink_attention_bf16  # noqa: F401

@@ -446,7 +446,7 @@ class CoreOps:
                     seq_slot: torch.Tensor, page_table: torch.Tensor, inv_freq: Optional[torch.Tensor], heads: int,
                     rank: int, rot: int, dims: int, window: Optional[int], scale: float,
                     max_keys: Optional[int] = None, workspace=None, sink: Optional[torch.Tensor] = None,
-                    amplitude: float = 1.0) -> None:
+                    amplitude: float = 1.0, batch=None) -> None:
         """out[t, h, :] = softmax over the visible positions of ((qa[t, h] . c + rotate(q_rot[t, h]) . r) *
         scale) times the positions' c; page rows are [c | r].  Head h's latent-space query starts at column
         h * qa_head of `qa`, its part to rotate at column h * q_head + q_off of `q` (one buffer may be both).
@@ -455,7 +455,8 @@ class CoreOps:
         rank <= 512); `max_keys` (an upper bound of the keys a token of the step sees) lets it cut the keys
         of a step of few tokens into parts, whose partial sums lie in a buffer of `workspace`.  `sink` (one
         32-bit number per head) adds exp(sink[h]) to the softmax's denominator, once.  The rotation's sine and cosine
-        are multiplied by `amplitude`."""
+        are multiplied by `amplitude`.  With `batch` (the step; its tokens are those of `qa`) prompts run on the
+        tensor-memory kernel, where that takes the sizes."""
         if sink is not None:
             _need(sink, torch.float32, "sink")
             if sink.numel() != heads:
@@ -471,6 +472,15 @@ class CoreOps:
                 qa.shape[1] < (heads - 1) * qa_head + rank:
             raise KernelError("latent_attn: sizes do not match")
         if self.act_dtype == torch.bfloat16:
+            if batch is not None and not getattr(batch, "is_decode", True):
+                from .latent_bf16 import LatentBf16
+                for t in (qa, q, pages, out):
+                    if not t.is_cuda:
+                        raise KernelError("kernel argument is not on a CUDA device; this package has no CPU path")
+                if LatentBf16.get().run(qa, qa_head, q, q_head, q_off, pages, out, token_pos, batch.seq_start, seq_slot,
+                                        page_table, inv_freq, batch.n_seqs, batch.max_new, heads, rank, rot, dims, window,
+                                        scale, amplitude, sink):
+                    return
             from ctypes import byref, c_longlong
             n = c_longlong(0)
             bound = min(int(max_keys), int(window)) if (max_keys and window) else int(max_keys or window or (1 << 30))

@@ -198,7 +198,8 @@ class LatentAttention:
             qa, qa_head, q_head, q_off = q, rank + rot, rank + rot, rank
         o.latent_attn(qa, qa_head, q, q_head, q_off, c.pages, mix, batch.token_pos, batch.token_seq, batch.seq_slot,
                       c.page_table, inv_freq, H, rank, rot, self.rot_dims, self.window, self.scale,
-                      max_keys=batch.len_bucket, workspace=ws, sink=self.sink, amplitude=self.amplitude)
+                      max_keys=batch.len_bucket, workspace=ws, sink=self.sink, amplitude=self.amplitude,
+                      batch=batch)
         gated = ws.get("latent_gated", (T, H * vdim), rt.act_dtype)
         o.headwise_gemm(mix.view(T, H * rank), rank, self.w_uv, gated, vdim,
                         gate=s[:, g_off:g_off + self.gate_rows] if self.gate_rows else None, act_out=True)
