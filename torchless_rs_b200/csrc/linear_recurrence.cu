@@ -148,6 +148,125 @@ gated_scan_kernel(const float* __restrict__ zq, const float* __restrict__ zf, co
   }
 }
 
+// The walk of many tokens for states of 64 and 128 rows (the gates are there already).  In the kernel above a token costs a
+// warp some hundred instructions for 128 entries of the state: the loads of its gates, six shuffles for four sums and
+// the store.  Here a lane owns one column and RPT rows, so a token's gates come from shared memory 16 bytes at a time, the
+// same address for all lanes of a column group, and no lane sums across others: a block holds all rows of 16 columns, its
+// sixteen row groups leave their sums of WALK_T tokens in shared memory, and those are added once per WALK_T tokens.
+// Gates and values of the next tokens arrive meanwhile.  The state goes through the same operations; a token's sum is
+// added row group by row group.  With the gates, 16 heads of 128 x 128, before / now: one
+// sequence of 2048 tokens 716 / 310 us, of 300 107 / 50, four of 400 365 / 129, eight of 30 85 / 27; 32 heads, 2048 tokens 958 / 332
+// (an entry's four operations at the full rate: 60).  What bounds it is the chain of a token in a block of eight warps.
+#define WALK_T 8
+#define WALK_COLS 16
+#define WALK_THREADS 256
+#define WALK_GROUPS 16       // row groups: a half warp each
+#define WALK_STAGES 8        // rounds of inputs in flight: a round's arithmetic takes less than half a microsecond (with two,
+                             // 2048 tokens took 607 us)
+
+__device__ __forceinline__ void walk_cp16(void* smem, const void* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void walk_cp4(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+
+template <int RPT>
+__global__ void __launch_bounds__(WALK_THREADS)
+gated_walk_kernel(const float* __restrict__ zq, const float* __restrict__ zf, const float* __restrict__ zv, int ld,
+                  float* __restrict__ state, float* __restrict__ o, int ldo, const int* __restrict__ seq_start,
+                  const int* __restrict__ seq_slot, int heads, int vdim) {
+  constexpr int DIM = WALK_GROUPS * RPT;
+  extern __shared__ __align__(16) float walk_smem[];
+  float (*fs)[WALK_T][DIM] = reinterpret_cast<float (*)[WALK_T][DIM]>(walk_smem);
+  float (*qs)[WALK_T][DIM] = fs + WALK_STAGES;
+  float (*vs)[WALK_T][WALK_COLS] = reinterpret_cast<float (*)[WALK_T][WALK_COLS]>(qs + WALK_STAGES);
+  float (*part)[WALK_GROUPS * WALK_COLS + WALK_COLS] =
+      reinterpret_cast<float (*)[WALK_GROUPS * WALK_COLS + WALK_COLS]>(vs + WALK_STAGES);
+  pdl_wait();
+  const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * WALK_COLS;
+  const int tid = threadIdx.x, col = tid & 15, g = tid >> 4, c = c0 + col;
+  const int t0 = seq_start[b], t1 = seq_start[b + 1];
+  float* S = state + (((size_t)seq_slot[b] * heads + h) * DIM + g * RPT) * vdim + c;
+  const bool vec = (ld & 3) == 0 && (((uintptr_t)zq | (uintptr_t)zf) & 15) == 0;
+  auto fetch = [&](int tb, int buf) {       // tokens past the end repeat the last one; their results are not used
+    if (tb < t1) {
+      if (vec) {
+        for (int i = tid; i < WALK_T * (DIM / 4); i += WALK_THREADS) {
+          const int p = i / (DIM / 4), e = (i % (DIM / 4)) * 4;
+          const size_t at = (size_t)min(tb + p, t1 - 1) * ld + h * DIM + e;
+          walk_cp16(&qs[buf][p][e], zq + at);
+          walk_cp16(&fs[buf][p][e], zf + at);
+        }
+      } else {
+        for (int i = tid; i < WALK_T * DIM; i += WALK_THREADS) {
+          const int p = i / DIM, e = i % DIM;
+          const size_t at = (size_t)min(tb + p, t1 - 1) * ld + h * DIM + e;
+          walk_cp4(&qs[buf][p][e], zq + at);
+          walk_cp4(&fs[buf][p][e], zf + at);
+        }
+      }
+      if (tid < WALK_T * WALK_COLS) {
+        const int p = tid / WALK_COLS, e = tid % WALK_COLS;
+        if (c0 + e < vdim) walk_cp4(&vs[buf][p][e], zv + (size_t)min(tb + p, t1 - 1) * ld + (size_t)h * vdim + c0 + e);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < WALK_STAGES - 1; ++i) fetch(t0 + i * WALK_T, i);
+  float s[RPT];
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) s[r] = c < vdim ? S[(size_t)r * vdim] : 0.0f;
+  int buf = 0;
+  for (int tb = t0; tb < t1; tb += WALK_T, buf = (buf + 1) % WALK_STAGES) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(WALK_STAGES - 2) : "memory");
+    __syncthreads();                 // this round's inputs are there; the round before's sums are written
+    fetch(tb + (WALK_STAGES - 1) * WALK_T, (buf + WALK_STAGES - 1) % WALK_STAGES);
+    const int n = min(WALK_T, t1 - tb);
+    auto token = [&](int p) {
+      const float v = vs[buf][p][col];
+      float sum[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int r0 = 0; r0 < RPT; r0 += 4) {
+        const float4 f4 = *reinterpret_cast<const float4*>(&fs[buf][p][g * RPT + r0]);
+        const float4 q4 = *reinterpret_cast<const float4*>(&qs[buf][p][g * RPT + r0]);
+        const float f[4] = {f4.x, f4.y, f4.z, f4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          s[r0 + r] = fmaf(f[r], s[r0 + r], (1.0f - f[r]) * v);
+          sum[r & 1] = fmaf(s[r0 + r], q[r], sum[r & 1]);
+        }
+      }
+      part[p][g * WALK_COLS + col] = sum[0] + sum[1];
+    };
+    if (n == WALK_T) {      // without a branch per token, so that a token's loads are issued during the ones before
+#pragma unroll
+      for (int p = 0; p < WALK_T; ++p) token(p);
+    } else {
+      for (int p = 0; p < n; ++p) token(p);
+    }
+    __syncthreads();
+    if (tid < WALK_T * WALK_COLS) {
+      const int p = tid / WALK_COLS, e = tid % WALK_COLS;
+      if (p < n && c0 + e < vdim) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < WALK_GROUPS; ++k) sum += part[p][k * WALK_COLS + e];
+        o[(size_t)(tb + p) * ldo + (size_t)h * vdim + c0 + e] = sum;
+      }
+    }
+  }
+  pdl_launch_dependents();
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int r = 0; r < RPT; ++r)
+    if (c < vdim) S[(size_t)r * vdim] = s[r];
+}
+
+// Steps of more than four tokens per sequence, whose gates are computed ahead.
+static bool walks(int T, int B, int dim) { return T > 4 * B && (dim == 64 || dim == 128); }
+
 // o[t, c] = the sum of the row groups' slices, in their order.
 __global__ void scan_sum_slices_kernel(const float* __restrict__ slices, float* __restrict__ o, size_t n, int groups) {
   pdl_wait();
@@ -170,6 +289,7 @@ __global__ void scan_sum_slices_kernel(const float* __restrict__ slices, float* 
 extern "C" int TL_NAME(tl_gated_scan_groups)(int T, int B, int dim) {
   const int r = (dim + 31) / 32;
   const int need = (r + SCAN_MAX_R - 1) / SCAN_MAX_R;      // a lane holds at most SCAN_MAX_R rows
+  if (walks(T, B, dim)) return 1;
   if (T <= 4 * B || T < 256) return need;
   const int fast = r >= 4 ? 4 : r >= 2 ? 2 : 1;
   return fast > need ? fast : need;
@@ -196,6 +316,21 @@ extern "C" int TL_NAME(tl_gated_scan)(float* zq, float* zf, const float* zv, int
     const int rc = tl_launch(scan_gates_kernel, dim3(blocks), dim3(256), 0, stream, zq, zf, ld, bias, low, T,
                              heads * dim);
     if (rc != 0) return rc;
+  }
+  if (walks(T, B, dim)) {
+    const dim3 walk(B, heads, (vdim + WALK_COLS - 1) / WALK_COLS);
+    const size_t smem = sizeof(float) * (WALK_STAGES * WALK_T * (2 * dim + WALK_COLS) + WALK_T * (WALK_GROUPS + 1) * WALK_COLS);
+#define WALK(RPT)                                                                                                       \
+  do {                                                                                                                  \
+    static const cudaError_t set =                                                                                      \
+        cudaFuncSetAttribute(gated_walk_kernel<RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);           \
+    if (set != cudaSuccess) return (int)set;                                                                            \
+    return tl_launch(gated_walk_kernel<RPT>, walk, dim3(WALK_THREADS), smem, stream, (const float*)zq, (const float*)zf, zv, \
+                     ld, state, o, ldo, seq_start, seq_slot, heads, vdim);                                              \
+  } while (0)
+    if (dim == 128) WALK(8);
+    WALK(4);
+#undef WALK
   }
   int rc;
 #define SCAN(RR)                                                                                               \
