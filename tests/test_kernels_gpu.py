@@ -108,7 +108,7 @@ def test_gemm_split_is_no_further_off_than_the_cuda_core_kernel(M, N, K):
     from torchless_rs_b200.csrc.gemm_f32 import GemmF32
     from torchless_rs_b200.parts.runtime import Workspace
     g, o, ws = GemmF32.get(), _ops(torch.float32), Workspace(torch.device(DEV))
-    assert GemmF32.takes(M, N, K) or N * K < 1 << 20
+    assert GemmF32.takes(M, N, K) or N * K < 20 << 20
     g_takes, GemmF32.takes = GemmF32.takes, staticmethod(lambda *a: True)
     try:
         for pad in (0, 3):       # rows of X and C that do not start on 16 bytes
@@ -535,16 +535,16 @@ def test_attention_f32_prompts_and_decode(nh, nkv, hd, window):
         starts = [sum(new[:b]) for b in range(len(new) + 1)]
         batch = SimpleNamespace(is_decode=decode, n_seqs=len(lens), len_bucket=max(256, 1 << (max(lens) - 1).bit_length()),
                                 total_bucket=sum(lens), max_new=max(new), seq_start=i32(starts), seq_len=i32(lens),
-                                seq_slot=pc.seq_slot)
+                                seq_slot=pc.seq_slot, max_len=max(lens))
         view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
         out = torch.full((T, nh * hd), float("nan"), device=DEV)
-        keep = f32.decode_split
+        keep, least, f32.PROMPT_FROM = f32.decode_split, f32.PROMPT_FROM, 0
         if plan is not None:
             f32.decode_split = plan
         try:
             ran = att.run(q, view, out, batch, nh, nkv, window, scale, ws)
         finally:
-            f32.decode_split = keep
+            f32.decode_split, f32.PROMPT_FROM = keep, least
         assert ran == (not decode or nh // nkv <= f32.MAX_GROUP_DECODE)
         if not ran:
             return
@@ -574,7 +574,7 @@ def test_attention_f32_keeps_unseen_values_out(poison):
     q = _rand((n, nh * hd), torch.float32, 6)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     batch = SimpleNamespace(is_decode=False, n_seqs=1, len_bucket=256, total_bucket=256, max_new=n, seq_start=i32([0, n]),
-                            seq_len=i32([n]), seq_slot=pc.seq_slot)
+                            seq_len=i32([n]), seq_slot=pc.seq_slot, max_len=n)
     out = torch.empty((n, nh * hd), device=DEV)
     view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
     assert AttentionF32.get(hd).run(q, view, out, batch, nh, nkv, None, 0.125, Workspace(torch.device(DEV)))

@@ -14,6 +14,7 @@ build.register_library("gemm_split", ("gemm_split.cu",), ())
 
 class GemmF32:
     _inst = None
+    LEAST = 1 << 20       # no product with a smaller matrix is taken
 
     @classmethod
     def get(cls) -> "GemmF32":
@@ -22,6 +23,10 @@ class GemmF32:
         return cls._inst
 
     def __init__(self):
+        self.lib = None       # loaded with the first product that it takes (a model can be put together without a device)
+        self._sms = {}
+
+    def _load(self) -> None:
         self.lib = build.load_library("gemm_split")
         P, I = c_void_p, c_int
         self.lib.tl_gemm_split.restype = c_int
@@ -30,7 +35,6 @@ class GemmF32:
         self.lib.tl_gemm_split_scratch.argtypes = [I, I]
         self.lib.tl_gemm_split_take_error.restype = c_int
         register_error_word("gemm_split", self.take_error)
-        self._sms = {}
 
     @staticmethod
     def takes(M: int, N: int, K: int) -> bool:
@@ -39,7 +43,7 @@ class GemmF32:
         4096 x 1024 16 and 17, of 4096 x 2048 26 and 18).  From nine rows on it is several times slower, until the
         launch more that is made here costs what the product does.  Below 1024 elements its sums are so short that
         they are nearer to the exact result."""
-        least = 1 << 20 if M > 8 else (6 << 20 if M > 4 else 20 << 20)
+        least = GemmF32.LEAST if M > 8 else (6 << 20 if M > 4 else 20 << 20)
         return M >= 4 and K >= 1024 and N * K >= least
 
     def run(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, workspace) -> bool:
@@ -56,6 +60,8 @@ class GemmF32:
         for t in (a, w, out):
             if not t.is_cuda:
                 raise KernelError("kernel argument is not on a CUDA device; this package has no CPU path")
+        if self.lib is None:
+            self._load()
         key = a.device.index if a.device.index is not None else torch.cuda.current_device()
         if key not in self._sms:
             self._sms[key] = torch.cuda.get_device_properties(a.device).multi_processor_count
@@ -71,4 +77,4 @@ class GemmF32:
 
     def take_error(self) -> int:
         """Nonzero if a kernel gave up on a bounded wait since the last call (synchronises)."""
-        return int(self.lib.tl_gemm_split_take_error())
+        return int(self.lib.tl_gemm_split_take_error()) if self.lib is not None else 0

@@ -13,8 +13,9 @@
 //   warp 4     TMA of the pages, four in flight
 //   warp 5     issues Q . K^T (the queries' half of c from tensor memory), up to two pages ahead (two S buffers)
 //   warp 6     issues P . V, P from tensor memory
-// Bound by the chain of a page in the softmax threads, 2.5 us: the scores' way out of tensor memory and to the other block,
-// the exponentials, the weights' way back (the tensor core's part of a page is some 1100 cycles and overlaps it).
+// Bound by the chain of a page, 2 us where the GPU is otherwise idle: the scores' way out of tensor memory and to the other
+// block, the exponentials, the weights' way back (the tensor core's part of a page is some 1100 cycles and overlaps it).
+// It is the exchange and not the exponentials: with two threads per row, each half of a page's keys, it took as long.
 // Measured, 16 heads, on mma.sync with a token's heads per tile / here: one prompt of 2048 tokens 582 / 235 us, of 4096
 // 1941 / 664 us; 32 heads, 2048 tokens 1025 / 439 us.
 //
@@ -329,7 +330,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       lt_ld32(t_s + u * PAGE + 32, sb);
       tmem_ld_wait();
       // the half sums go to the other block, 16 bytes of a row beside the next row's; their bytes count at its barrier (plain
-      // stores and an arrival that waits for them took 1.3 us more a page)
+      // stores and an arrival that waits for them took 0.6 us more a page)
 #pragma unroll
       for (int g = 0; g < 16; ++g) {
         const uint32_t* v = g < 8 ? sa + 4 * g : sb + 4 * (g - 8);

@@ -58,7 +58,7 @@ class Matmul:
             emit[1].valid = False
         if self.fast is not None and self.fast.run(a, w, out, mode, emit=emit, rope=rope):
             return self.fast.rope_applied
-        if self.split is None or not self.split.run(a, w, out, mode, self.rt.workspace):
+        if self.split is None or w.numel() < self.split.LEAST or not self.split.run(a, w, out, mode, self.rt.workspace):
             self.rt.ops.gemm_generic(a, w, out, mode)
         return False
 
