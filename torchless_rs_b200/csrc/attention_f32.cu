@@ -13,7 +13,7 @@
 //   decode   a run of pages of one sequence and key/value head per block, two pages in flight, all query heads of the
 //            group; blocks of one sequence merge through a second kernel.  Bound by the pages' bytes.
 // Measured, 32 heads over 8 of 128, by the kernel for every head size / here: prompts of 400 and 131 tokens 1770 / 99 us, one
-// of 2000 tokens 38,086 / 1152 us (14.7 of some 70 TFLOP/s); one token each of four sequences of 500 to 2000 tokens 244 / 26 us
+// of 2000 tokens 38,086 / 1152 us (28 of some 70 TFLOP/s); one token each of four sequences of 500 to 2000 tokens 244 / 26 us
 // with the merge (5.5 at the copy rate), of eight of 4000 tokens 760 / 100 us (40); 20 tokens after 980 440 / 161 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -248,6 +248,7 @@ attn_f32_decode_kernel(const AttnArgs a) {
   float* m_s = alpha_s + GM;
   float* l_s = m_s + GM;
   pdl_wait();
+  pdl_launch_dependents();   // (at once: in a small model's step the next kernel's launch is what this one hides)
   const int b = blockIdx.z, kvh = blockIdx.y, split = blockIdx.x, group = a.nh / a.nkv;
   const int pos = a.seq_len[b] - 1;
   const int lo = a.window > 0 ? max(pos - a.window + 1, 0) : 0;
@@ -350,7 +351,6 @@ attn_f32_decode_kernel(const AttnArgs a) {
     __syncthreads();       // the page and its weights are used up
     fetch(i + 2, at);
   }
-  pdl_launch_dependents();
   cp_wait<0>();
 #pragma unroll
   for (int g = 0; g < GM; ++g) Os[g * D_THREADS + tid] = acc[g];

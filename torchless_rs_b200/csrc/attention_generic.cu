@@ -1,7 +1,7 @@
 // Attention over the paged cache on CUDA cores, for prefill and decode alike, with
 // every head size that is a multiple of 16 up to 256 and any number of heads and
-// groups.  It is the attention of the true 32-bit path and the fallback of the
-// bfloat16 path.
+// groups.  It is the fallback of the 32-bit path (attention_f32.cu takes the common head
+// sizes) and of the bfloat16 path.
 //
 // One block per (token, query head).  The token's position p and its sequence's page
 // table give the keys: i in [max(0, p - W + 1), p] with a window W, else [0, p]

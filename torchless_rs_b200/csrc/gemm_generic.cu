@@ -2,9 +2,10 @@
 //
 //   C[M, N] (op)= A[M, K] * W[N, K]^T        A, W of act_t, K contiguous in both
 //
-// These kernels are the whole of the true 32-bit path (no tensor-core mode of
-// reduced precision is ever used there) and the fallback of the bfloat16 path for
-// shapes that the tensor-core kernels refuse.  The reference computes each output as
+// These kernels take the products of the true 32-bit path that gemm_split.cu does not
+// (few rows, small matrices, odd strides; no mode of reduced precision is used there
+// either) and are the fallback of the bfloat16 path for shapes that the tensor-core
+// kernels refuse.  The reference computes each output as
 // one sequential 32-bit dot product (src/loader/parameters.rs:551-594).
 //
 // Output modes:

@@ -26,7 +26,7 @@
 //   warp 13     issues the instructions
 //   warp 14     TMA of the pieces of X, which a kernel before has made
 // W's pieces are operands from tensor memory because an instruction that reads both operands from shared memory is
-// bound by that: with W's pieces there a stage of 192 tokens took 2900 cycles where its arithmetic takes 576.  While
+// bound by that: with W's pieces there a stage of 192 tokens took 2900 cycles where its arithmetic takes 1152.  While
 // the sum of the leading products is read, the instructions of the other five run.
 //
 // Products with few tiles split K over a cluster of blocks, which add their partial tiles in the order of the splits
