@@ -496,3 +496,40 @@ def test_latent_attention_of_prompts_on_tensor_memory(lens, new, heads, rot, dim
     assert LatentBf16.get().take_error() == 0
     assert (a - c).abs().max() <= 2.0 ** -8 * pages.float().abs().max() * 1.05
     assert (a - c).norm() <= 4e-3 * c.norm()
+
+
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("size", [0.3, 1.0, 3.0, 10.0])
+def test_latent_attention_of_prompts_is_as_near_to_64_bits_as_the_kernel_for_every_step(size, sink):
+    """Flat and peaked softmaxes.  Both kernels round queries, weights and nothing else to bfloat16, at the same points, so
+    their errors against 64 bits are alike but for the order of 32-bit sums: their difference (some 2^-16 of the result, rounding
+    flips of single weights included) cannot move an error of 2^-10 and more by a hundredth."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.latent_bf16 import LatentBf16
+    from torchless_rs_b200.parts.runtime import Workspace
+    o, ws, T, heads, rank, rot = ops.core_ops(torch.bfloat16), Workspace(torch.device("cuda:0")), 500, 16, 512, 64
+    w, scale = rank + rot, (rank + rot) ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(int(10 * size))
+    pages = torch.randn((8, 64, w), device="cuda", generator=g).to(torch.bfloat16)
+    q = torch.randn((T, heads * w), device="cuda", generator=g) * size
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    sinks = torch.randn(heads, device="cuda", generator=g) * 3 if sink else None
+    batch = SimpleNamespace(is_decode=False, n_seqs=1, max_new=T, seq_start=i32([0, T]))
+    outs = []
+    for b in (batch, None):
+        out = torch.empty((T, heads, rank), device="cuda")
+        before = ops.launch_counts().get("latent_attn_tc", 0)
+        o.latent_attn(q, w, q, w, rank, pages, out, i32(list(range(T))), i32([0] * T), i32([0]), i32([list(range(8))]), None, heads,
+                      rank, rot, 0, None, scale, max_keys=T, workspace=ws, sink=sinks, batch=b)
+        assert ops.launch_counts().get("latent_attn_tc", 0) == before + (b is not None)
+        outs.append(out.double())
+    keys = pages.reshape(-1, w)[:T].double()
+    s = torch.einsum("thw,kw->htk", q.view(T, heads, w).double(), keys) * scale
+    s.masked_fill_(torch.ones((T, T), dtype=torch.bool, device="cuda").triu(1), -float("inf"))
+    if sink:
+        s = torch.cat([s, sinks.double()[:, None, None].expand(heads, T, 1)], -1)
+    want = (torch.softmax(s, -1)[..., :T] @ keys[:, :rank]).transpose(0, 1)
+    tc, every = (float((x - want).norm() / want.norm()) for x in outs)
+    assert LatentBf16.get().take_error() == 0
+    assert tc <= 1.01 * every, (tc, every)

@@ -8,16 +8,16 @@
 // of the shared memory.  So two blocks of a cluster share a tile: each holds the queries' and the pages' half of c (the
 // first also r), multiplies its half for scores that are half sums, hands them to the other through distributed shared
 // memory, and after the softmax, which both compute from the same sums, sums its own half of c.
-//   warps 0-3  softmax, a row per thread (as in attention_prefill_tc.cu: the reference of the exponentials moves only
-//              when a score exceeds it by 2^8); exchange of the half scores; output
+//   warps 0-3  softmax, a row per thread; exchange of the half scores; output
 //   warp 4     TMA of the pages, four in flight
 //   warp 5     issues Q . K^T (the queries' half of c from tensor memory), up to two pages ahead (two S buffers)
 //   warp 6     issues P . V, P from tensor memory
 // Bound by the chain of a page, 2 us where the GPU is otherwise idle: the scores' way out of tensor memory and to the other
 // block, the exponentials, the weights' way back (the tensor core's part of a page is some 1100 cycles and overlaps it).
-// It is the exchange and not the exponentials: with two threads per row, each half of a page's keys, it took as long.
-// Measured, 16 heads, on mma.sync with a token's heads per tile / here: one prompt of 2048 tokens 582 / 235 us, of 4096
-// 1941 / 664 us; 32 heads, 2048 tokens 1025 / 439 us.
+// It is the exchange and not the exponentials: with two threads per row, each half of a page's keys, it took as long (before
+// the maximum below moved with every page).
+// Measured, 16 heads, on mma.sync with a token's heads per tile / here: one prompt of 2048 tokens 582 / 251 us, of 4096
+// 1941 / 711 us; 32 heads, 2048 tokens 1025 / 471 us.
 //
 // Every wait on an mbarrier is bounded; when a bound is hit the block records a code in tl_latent_tc_error, stops, frees
 // its tensor memory and returns.
@@ -314,9 +314,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
     const int pos = valid ? p0 + r / a.heads : p_last;
     const int lo = a.window > 0 ? max(pos - a.window + 1, 0) : 0;
     const uint32_t lanes = (uint32_t)(warp * 32) << 16, t_s = tmem + lanes, t_o = tmem + LT_COL_O + lanes;
-    const float* sink = a.sink;
-    float m = sink != nullptr && valid ? sink[r % a.heads] * 1.4426950408889634f : -INFINITY;
-    float l = sink != nullptr && valid ? 1.0f : 0.0f;
+    float m = -INFINITY, l = 0.0f;
     const uint32_t mine = smem_u32(x_s) + (uint32_t)r * 16u, theirs = lt_mapa(mine, half ^ 1u);
     const uint32_t bar_theirs = lt_mapa(smem_u32(x_full), half ^ 1u);
     bool ok = true;
@@ -365,9 +363,14 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       }
 #pragma unroll
       for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fmaxf(__uint_as_float(sa[j]), __uint_as_float(sb[j])));
-      const float m_new = (mx > m + 8.0f || m == -INFINITY) ? fmaxf(m, mx) : m;
+      // The reference is the running maximum itself: the weight of the key that stands out is then 1, which bfloat16 holds
+      // exactly.  (A reference that moves only when a score exceeds it by 2^8 spares most of the rescaling of O, but rounds
+      // that weight too while l sums weights as they are: 235 us instead of 251 for 2048 tokens, and up to 7 % further from 64
+      // bits where few keys count.)
+      const float m_new = fmaxf(m, mx);
       const float ref = m_new == -INFINITY ? 0.0f : m_new;
-      const float alpha = valid ? exp2f(m - ref) : 1.0f;   // (a row without a token must not ask for rescaling)
+      // (a row without a token, or that sees no key so far, must not ask for rescaling)
+      const float alpha = valid && m_new != -INFINITY ? exp2f(m - ref) : 1.0f;
       m = m_new;
       uint32_t pk[32];   // the row of P as bfloat16 pairs
       float sum = 0.0f, sum_hi = 0.0f;
@@ -381,7 +384,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
         pk[16 + j] = lt_pack(w2, w3);
       }
       l = l * alpha + (sum + sum_hi);
-      // O is touched only when some row's reference moved; every warp waits for P(i - 1) . V(i - 1) on every page all the
+      // O is touched only when some row's maximum moved; every warp waits for P(i - 1) . V(i - 1) on every page all the
       // same, so that no phase of its barrier is taken for another
       if (i > 0) {
         ok = lt_wait(o_done, (uint32_t)(i - 1) & 1u, abort_flag, 7);
@@ -408,7 +411,8 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
     if (ok) ok = lt_wait(o_done, (uint32_t)(n_pg - 1) & 1u, abort_flag, 8);
     if (__all_sync(0xffffffffu, ok)) {
       tc_fence_after();
-      const float inv = 1.0f / l;
+      // a sink only enters the denominator
+      const float inv = 1.0f / (a.sink != nullptr && valid ? l + exp2f(a.sink[r % a.heads] * 1.4426950408889634f - m) : l);
       float* orow = a.o + ((size_t)(first + t0) * a.heads + r) * LT_RANK + half * LT_HALF;
 #pragma unroll 2
       for (int c = 0; c < LT_HALF; c += 32) {
