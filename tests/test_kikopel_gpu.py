@@ -533,3 +533,61 @@ def test_latent_attention_of_prompts_is_as_near_to_64_bits_as_the_kernel_for_eve
     tc, every = (float((x - want).norm() / want.norm()) for x in outs)
     assert LatentBf16.get().take_error() == 0
     assert tc <= 1.01 * every, (tc, every)
+
+
+@pytest.mark.parametrize("heads,n,new,window", [(16, 300, 300, None), (16, 450, 300, 100), (1, 400, 333, 70), (128, 200, 150, 64),
+                                                (24, 200, 130, None), (16, 65, 65, 64), (32, 130, 2, 30)])
+@pytest.mark.parametrize("what", [float("nan"), float("inf")])
+def test_latent_attention_of_prompts_keeps_unseen_values_out(heads, n, new, window, what):
+    """Values that are not finite behind the sequence's end (a page's earlier owner left them) and before every window reach
+    nobody; one such value at a position that some tokens see makes those tokens' results what 64 bits give (NaN in every column,
+    or, for a score of minus infinity, in its own) and no other's.  Numbers in both halves of the latent and in the rotated part."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.latent_bf16 import LatentBf16
+    from torchless_rs_b200.parts.runtime import Workspace
+    o, ws, rank, rot = ops.core_ops(torch.bfloat16), Workspace(torch.device("cuda:0")), 512, 64
+    w, scale = rank + rot, (rank + rot) ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(n + heads)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    n_pg, first = -(-n // 64), n - new
+    lo = max(first - window + 1, 0) if window else 0
+    clean = torch.randn((n_pg * 64, w), device="cuda", generator=g).to(torch.bfloat16)
+    q = torch.randn((new, heads * w), device="cuda", generator=g)
+    batch = SimpleNamespace(is_decode=False, n_seqs=1, max_new=new, seq_start=i32([0, new]))
+    def run(rows):
+        out = torch.empty((new, heads, rank), device="cuda")
+        o.latent_attn(q, w, q, w, rank, rows.view(n_pg, 64, w).contiguous(), out, i32(list(range(first, n))), i32([0] * new), i32([0]),
+                      i32([list(range(n_pg))]), None, heads, rank, rot, 0, window, scale, max_keys=n, workspace=ws, batch=batch)
+        return out
+    keep, LatentBf16.FROM_ROWS = LatentBf16.FROM_ROWS, 0
+    try:
+        base = run(clean)
+        assert base.isfinite().all()
+        dirty = clean.clone()
+        dirty[n:] = what
+        dirty[:lo] = what
+        assert torch.equal(run(dirty), base)
+        pos = torch.arange(first, n, device="cuda")
+        for at in sorted({lo, first, first + 1, first + new // 2, n - 2, n - 1, max(first - 3, lo)}):
+            for col in (3, 300, 540):           # the first block's half, the second's, the rotated part
+                bad = dirty.clone()
+                bad[at, col] = what
+                got = run(bad)
+                sees = (pos >= at) & ((pos - at < window) if window else (pos >= 0))
+                assert torch.equal(got[~sees], base[~sees]), (at, col)
+                # the row's score of it: NaN, or the sign of the query's number times infinity
+                qc = (q.view(new, heads, w)[..., col] * scale * 1.4426950408889634).to(torch.bfloat16).float()
+                low = (qc < 0) if what == float("inf") else torch.zeros_like(qc, dtype=torch.bool)
+                s, l = sees[:, None].expand(new, heads), low
+                assert got[s & ~l].isnan().all(), (at, col)
+                rest = got[s & l]
+                if col < rank:
+                    assert rest[:, col].isnan().all()
+                    rest = torch.cat([rest[:, :col], rest[:, col + 1:]], 1)
+                alone = (torch.arange(new, device="cuda") + first == lo) & sees      # (a row that sees nothing else has no softmax)
+                if not bool(alone.any()):
+                    assert rest.isfinite().all(), (at, col)
+        assert LatentBf16.get().take_error() == 0
+    finally:
+        LatentBf16.FROM_ROWS = keep

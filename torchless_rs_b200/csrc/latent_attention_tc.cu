@@ -16,8 +16,8 @@
 // block, the exponentials, the weights' way back (the tensor core's part of a page is some 1100 cycles and overlaps it).
 // It is the exchange and not the exponentials: with two threads per row, each half of a page's keys, it took as long (before
 // the maximum below moved with every page).
-// Measured, 16 heads, on mma.sync with a token's heads per tile / here: one prompt of 2048 tokens 582 / 251 us, of 4096
-// 1941 / 711 us; 32 heads, 2048 tokens 1025 / 471 us.
+// Measured, 16 heads, on mma.sync with a token's heads per tile / here: one prompt of 2048 tokens 582 / 254 us, of 4096
+// 1941 / 723 us; 32 heads, 2048 tokens 1025 / 479 us.
 //
 // Every wait on an mbarrier is bounded; when a bound is hit the block records a code in tl_latent_tc_error, stops, frees
 // its tensor memory and returns.
@@ -131,9 +131,43 @@ __device__ __forceinline__ uint64_t lt_desc_k64(uint32_t saddr) {
          (uint64_t)4 << 61;
 }
 
+// The tensor core multiplies a weight of 0 like any other, and 0 x NaN is NaN.  So in a page that not every row of the tile sees
+// whole, a position outside [seen_lo, seen_hi] (what all rows see) whose values are not all finite is set to zero before P . V.
+// By the 128 softmax threads, eight to a position's 512 bytes; true if this thread cleared one that some row does see, in
+// [some_lo, some_hi].  Such a row's score of it is NaN or infinite, so its weight is NaN, which reaches the row's sum l, or 0,
+// and the caller puts in what 0 x the value gives.
+__device__ __forceinline__ bool lt_clear_unseen(uint8_t* page, int key0, int seen_lo, int seen_hi, int some_lo, int some_hi) {
+  const int row0 = (int)(threadIdx.x >> 3), chunk = (int)(threadIdx.x & 7);
+  bool found = false;
+#pragma unroll
+  for (int k = row0; k < PAGE; k += LT_ROWS / 8) {
+    const int key = key0 + k;
+    uint4* at = reinterpret_cast<uint4*>(page + k * 128 + chunk * 16);
+    uint32_t carry = 0;                    // an exponent of all ones carries into the bit above it
+    const bool look = key < seen_lo || key > seen_hi;
+    if (look) {
+#pragma unroll
+      for (int u = 0; u < LT_SUBS; ++u) {
+        const uint4 x = at[u * (PAGE * 128 / 16)];
+        carry |= ((x.x & 0x7f807f80u) + 0x00800080u) | ((x.y & 0x7f807f80u) + 0x00800080u) |
+                 ((x.z & 0x7f807f80u) + 0x00800080u) | ((x.w & 0x7f807f80u) + 0x00800080u);
+      }
+    }
+    const uint32_t any = __ballot_sync(0xffffffffu, (carry & 0x80008000u) != 0u) >> (threadIdx.x & 24u) & 0xffu;
+    if (look && any) {
+#pragma unroll
+      for (int u = 0; u < LT_SUBS; ++u) at[u * (PAGE * 128 / 16)] = make_uint4(0u, 0u, 0u, 0u);
+      found |= key >= some_lo && key <= some_hi;
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads the page as it is now
+  return found;
+}
+
 struct LatentArgs {
   const float* qa;
   const float* q;
+  const __nv_bfloat16* pages;
   float* o;                 // [tokens, heads, 512]
   const int* seq_start;
   const int* token_pos;
@@ -161,6 +195,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
   uint64_t* o_done = pv_done + 2;
   uint32_t* tmem_slot = (uint32_t*)(o_done + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  volatile int* cleared = abort_flag + 1;   // values that some row sees were set to zero (lt_clear_unseen)
 
   const int warp = threadIdx.x >> 5, tid = threadIdx.x;
   const uint32_t half = cluster_rank();
@@ -171,6 +206,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
   const int tokens = min(a.tokens, n_new - t0), rows = tokens * a.heads;
   const int p0 = a.token_pos[first + t0], p_last = p0 + tokens - 1;
   const int lo_all = a.window > 0 ? max(p0 - a.window + 1, 0) : 0;
+  const int lo_last = a.window > 0 ? max(p_last - a.window + 1, 0) : 0;     // [lo_last, p0]: what every row of the tile sees
   const int pg0 = lo_all / PAGE, n_pg = p_last / PAGE - pg0 + 1;
   const int* table = a.page_table + (size_t)a.seq_slot[b] * a.table_stride + pg0;
 
@@ -184,6 +220,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
     }
     mbar_init(o_done, 1);
     *abort_flag = 0;
+    *cleared = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int u = 0; u < 2 && u < n_pg; ++u) mbar_expect_tx(&x_full[u], LT_X);
   }
@@ -365,7 +402,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
       for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fmaxf(__uint_as_float(sa[j]), __uint_as_float(sb[j])));
       // The reference is the running maximum itself: the weight of the key that stands out is then 1, which bfloat16 holds
       // exactly.  (A reference that moves only when a score exceeds it by 2^8 spares most of the rescaling of O, but rounds
-      // that weight too while l sums weights as they are: 235 us instead of 251 for 2048 tokens, and up to 7 % further from 64
+      // that weight too while l sums weights as they are: 235 us instead of 251 for 2048 tokens (then), and up to 7 % further from 64
       // bits where few keys count.)
       const float m_new = fmaxf(m, mx);
       const float ref = m_new == -INFINITY ? 0.0f : m_new;
@@ -403,12 +440,18 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
           lt_wait_st();
         }
       }
+      if (key0 < lo_last || key0 + PAGE - 1 > p0) {   // (the page's scores are done: nobody else reads it now)
+        ok = lt_wait(&k_full[i % LT_PAGES], (uint32_t)(i / LT_PAGES) & 1u, abort_flag, 3);   // what TMA wrote is visible
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        if (lt_clear_unseen(k_s + (i % LT_PAGES) * LT_K, key0, lo_last, p0, lo_all, p_last)) *cleared = 1;
+      }
       lt_st32(t_s + u * PAGE, pk);   // this lane's row of P, keys 2c and 2c + 1 in column c
       lt_wait_st();
       tc_fence_before();
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_full[u])) : "memory");
     }
     if (ok) ok = lt_wait(o_done, (uint32_t)(n_pg - 1) & 1u, abort_flag, 8);
+    asm volatile("bar.sync 1, 128;" ::: "memory");   // `cleared` by any of these warps
     if (__all_sync(0xffffffffu, ok)) {
       tc_fence_after();
       // a sink only enters the denominator
@@ -425,6 +468,15 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm, const __grid_const
             *reinterpret_cast<float4*>(orow + c + j) =
                 make_float4(__uint_as_float(ov[j]) * inv, __uint_as_float(ov[j + 1]) * inv, __uint_as_float(ov[j + 2]) * inv,
                             __uint_as_float(ov[j + 3]) * inv);
+        }
+      }
+      if (valid && *cleared) {
+        for (int key = lo_all; key <= p_last; ++key) {
+          if (key >= lo_last && key <= p0) { key = p0; continue; }     // these were multiplied as they are
+          if (key < lo || key > pos) continue;
+          const __nv_bfloat16* v = a.pages + ((size_t)table[key / PAGE - pg0] * PAGE + key % PAGE) * (LT_RANK + a.rot) + half * LT_HALF;
+          for (int c = 0; c < LT_HALF; ++c)
+            if (!(fabsf(__bfloat162float(v[c])) < INFINITY)) orow[c] = NAN;
         }
       }
     }
@@ -479,7 +531,7 @@ extern "C" int tl_latent_attn_tc(const float* qa, int ld_qa, int qa_head, const 
   if (!make(&tm, box, CU_TENSOR_MAP_SWIZZLE_128B) || !make(&tm_r, box_r, CU_TENSOR_MAP_SWIZZLE_64B)) return -2;
   static const cudaError_t set = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
   if (set != cudaSuccess) return (int)set;
-  LatentArgs a = {qa, q, o, seq_start, token_pos, seq_slot, page_table, inv_freq, sink, ld_qa, qa_head, ldq, q_head, q_off,
+  LatentArgs a = {qa, q, (const __nv_bfloat16*)pages, o, seq_start, token_pos, seq_slot, page_table, inv_freq, sink, ld_qa, qa_head, ldq, q_head, q_off,
                   table_stride, heads, rot, dims, window, LT_ROWS / heads, scale * 1.4426950408889634f, amp};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * ((max_new + a.tokens - 1) / a.tokens), seqs);

@@ -16,8 +16,8 @@ build.register_library("latent_tc", ("latent_attention_tc.cu",), ())
 class LatentBf16:
     _inst = None
     # Rows (tokens of the sequence that brings most, times heads) from which on this kernel is the faster one.  16 heads, us
-    # here / by the kernel of latent_attention.cu: 128 tokens 30 / 24, 300 tokens 39 / 41, 1000 tokens 86 / 225, 2048 tokens
-    # 251 / 582, four prompts of 400 tokens 112 / 142; 32 tokens after 968 63 / 39 (that one cuts the keys into parts).
+    # here / by the kernel of latent_attention.cu: 128 tokens 30 / 24, 300 tokens 39 / 41, 1000 tokens 88 / 222, 2048 tokens
+    # 254 / 582, four prompts of 400 tokens 114 / 142; 32 tokens after 968 63 / 39 (that one cuts the keys into parts).
     FROM_ROWS = 4096
 
     @classmethod
