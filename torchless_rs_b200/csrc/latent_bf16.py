@@ -3,7 +3,7 @@ sizes it does not take; the caller then uses the kernels of latent_attention.cu.
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong, c_void_p
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -12,12 +12,38 @@ from .ops import _check, _stream, register_error_word
 
 build.register_library("latent_tc", ("latent_attention_tc.cu",), ())
 
+PAGE = build.PAGE_TOKENS
+
+
+def prompt_times(past_lens, new_lens, heads: int, window: Optional[int], sms: int) -> Tuple[float, float]:
+    """What a step's latent attention takes, in us, here and by the kernel for every step (latent_attention.cu), from what each
+    sequence holds before and after it.  Here a tile of 128 // heads tokens of one sequence takes a pair of SMs some 32 us
+    besides 2.1 us per page (27.5 the first round), however few of its rows are filled.  There a token's group of 16 heads takes
+    0.026 us and 0.0002 per key with four tokens to a block, more while the GPU is not full, and a block walks its
+    token's keys in order.  Measured, 16 heads, here / there: one prompt of 256 tokens 36 / 29, of 300 39 / 41, of 1000
+    88 / 222, of 2048 254 / 582; 32 prompts of 256 509 / 424, of 400 850 / 839, of 500 1109 / 1187, of 256 after 256 640 /
+    841; 512 tokens and 32 prompts of 50 161 / 97; 256 tokens and 63 sequences that bring one after 199 68 / 38, 15 that
+    bring one after 999 59 / 87; 64 prompts of 128 at 32 heads 928 / 612; 16 of 600 at 8 heads 366 / 788."""
+    W = window or 1 << 60
+    seen = lambda n: n * (n + 1) // 2 if n <= W else W * (W + 1) // 2 + (n - W) * W     # keys that the first n tokens see
+    per = 128 // heads
+    counts = [n - p for p, n in zip(past_lens, new_lens)]
+    T, tiles = sum(counts), sum(-(-c // per) for c in counts)
+    pairs = sum(seen(n) - seen(p) for p, n in zip(past_lens, new_lens))
+    longest = max(new_lens)
+    at_once = sms // 2
+    here = 32.0 * -(-tiles // at_once) - 4.5 + 2.1 * max(-(-min(longest, W + per) // PAGE), tiles / at_once * (pairs / T / PAGE + 0.5))
+    groups = -(-heads // 16)
+    rows, keys = T * groups, pairs * groups
+    there = 20.0 + 0.0002 * keys + 0.026 * rows if rows >= 1184 else min(12.0 + 0.0006 * keys, 25.0 + 0.0004 * keys)
+    return here, max(there, 5.2 * -(-min(longest, W) // PAGE))
+
 
 class LatentBf16:
     _inst = None
-    # Rows (tokens of the sequence that brings most, times heads) from which on this kernel is the faster one.  16 heads, us
-    # here / by the kernel of latent_attention.cu: 128 tokens 30 / 24, 300 tokens 39 / 41, 1000 tokens 88 / 222, 2048 tokens
-    # 254 / 582, four prompts of 400 tokens 114 / 142; 32 tokens after 968 63 / 39 (that one cuts the keys into parts).
+    # Rows (tokens of the sequence that brings most, times heads) below which this kernel is not considered.  16 heads, us
+    # here / by the kernel of latent_attention.cu: 128 tokens 30 / 24; 32 tokens after 968 63 / 39 (that one cuts the keys
+    # into parts).
     FROM_ROWS = 4096
 
     @classmethod
@@ -34,17 +60,34 @@ class LatentBf16:
             [c_float, c_float, P]
         self.lib.tl_latent_tc_take_error.restype = c_int
         register_error_word("latent_tc", self.take_error)
+        self._sms = {}
 
-    def run(self, qa, qa_head, q, q_head, q_off, pages, out, token_pos, seq_start, seq_slot, page_table, inv_freq, n_seqs,
-            max_new, heads, rank, rot, dims, window: Optional[int], scale, amplitude, sink: Optional[torch.Tensor]) -> bool:
-        if max_new * heads < self.FROM_ROWS:
+    def _faster(self, batch, heads: int, window: Optional[int], device) -> bool:
+        """Whether a step runs here (worked out once per step)."""
+        if batch.max_new * heads < self.FROM_ROWS or heads > 128:
+            return False
+        if getattr(batch, "past_lens", None) is None:
+            return True
+        key = ("latent", heads, window)
+        known = batch.plans.get(key)
+        if known is None:
+            at = device.index if device.index is not None else torch.cuda.current_device()
+            if at not in self._sms:
+                self._sms[at] = torch.cuda.get_device_properties(device).multi_processor_count
+            here, there = prompt_times(batch.past_lens, batch.new_lens, heads, window, self._sms[at])
+            known = batch.plans[key] = here < there
+        return known
+
+    def run(self, qa, qa_head, q, q_head, q_off, pages, out, token_pos, seq_slot, page_table, inv_freq, batch, heads, rank, rot,
+            dims, window: Optional[int], scale, amplitude, sink: Optional[torch.Tensor]) -> bool:
+        if not self._faster(batch, heads, window, qa.device):
             return False
         addr = lambda t: t.data_ptr() if t is not None else None
         st = self.lib.tl_latent_attn_tc(
             qa.data_ptr(), qa.stride(0), qa_head, q.data_ptr(), q.stride(0), q_head, q_off, pages.data_ptr(),
-            pages.shape[0], out.data_ptr(), seq_start.data_ptr(), token_pos.data_ptr(), seq_slot.data_ptr(),
-            page_table.data_ptr(), page_table.stride(0), addr(inv_freq if dims else None), addr(sink), n_seqs, max_new,
-            heads, rank, rot, dims, window or 0, scale, amplitude, _stream())
+            pages.shape[0], out.data_ptr(), batch.seq_start.data_ptr(), token_pos.data_ptr(), seq_slot.data_ptr(),
+            page_table.data_ptr(), page_table.stride(0), addr(inv_freq if dims else None), addr(sink), batch.n_seqs,
+            batch.max_new, heads, rank, rot, dims, window or 0, scale, amplitude, _stream())
         if st == -2:
             return False
         _check(st, "latent_attn_tc")

@@ -477,9 +477,8 @@ class CoreOps:
                 for t in (qa, q, pages, out):
                     if not t.is_cuda:
                         raise KernelError("kernel argument is not on a CUDA device; this package has no CPU path")
-                if LatentBf16.get().run(qa, qa_head, q, q_head, q_off, pages, out, token_pos, batch.seq_start, seq_slot,
-                                        page_table, inv_freq, batch.n_seqs, batch.max_new, heads, rank, rot, dims, window,
-                                        scale, amplitude, sink):
+                if LatentBf16.get().run(qa, qa_head, q, q_head, q_off, pages, out, token_pos, seq_slot, page_table, inv_freq,
+                                        batch, heads, rank, rot, dims, window, scale, amplitude, sink):
                     return
             from ctypes import byref, c_longlong
             n = c_longlong(0)

@@ -1,7 +1,7 @@
 """The tokens of one step and where they belong, as the kernels read them."""
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -37,6 +37,7 @@ class StepBatch:
     new_lens: List[int]
     token_src: Optional[torch.Tensor] = None   # device int32: tokens selected by the previous step
     total_bucket: Optional[int] = None           # the sum of the sequences' lengths after this step, rounded up
+    plans: dict = field(default_factory=dict)    # which kernels the step's lengths call for, as layers find it out
 
 
 def length_bucket(max_len: int) -> int:
