@@ -581,6 +581,40 @@ def test_attention_f32_keeps_unseen_values_out(poison):
     assert out[:bad].isfinite().all() and not out[bad:].isfinite().any()
 
 
+@pytest.mark.parametrize("poison", [float("inf"), float("nan")])
+@pytest.mark.parametrize("nh,nkv,hd,window", [(4, 2, 64, 70), (8, 1, 128, 64), (2, 2, 16, 33), (4, 1, 32, 1)])
+def test_attention_f32_decode_keeps_values_before_the_window_out(nh, nkv, hd, window, poison):
+    """Decode steps with a window whose edge lies inside a page, all values before it no numbers: the same bits as with
+    ordinary values there, in one block per sequence and in several; a value at the edge itself does reach the result."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc import attention_f32 as f32
+    from torchless_rs_b200.parts.runtime import Workspace
+    lens = [window, window + 1, 130, 191, 192, 193, 500]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(is_decode=True, n_seqs=len(lens), len_bucket=512, total_bucket=sum(lens), max_new=1,
+                            seq_start=i32(list(range(len(lens) + 1))), seq_len=i32(lens), max_len=max(lens))
+    q = _rand((len(lens), nh * hd), torch.float32, 6)
+    def run(spoil, split):
+        pc = Paged(lens, nkv, hd, torch.float32, 5)
+        for b, n in enumerate(lens):
+            for i in spoil(n):
+                pc.v_pages[int(pc.table[pc.slots[b], i // PAGE]), :, :, i % PAGE] = poison
+        batch.seq_slot = pc.seq_slot
+        out = torch.empty((len(lens), nh * hd), device=DEV)
+        view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
+        keep, f32.decode_split = f32.decode_split, lambda *a: split
+        try:
+            assert f32.AttentionF32.get(hd).run(q, view, out, batch, nh, nkv, window, 0.125, Workspace(torch.device(DEV)))
+        finally:
+            f32.decode_split = keep
+        return out
+    for split in ((8, 1), (1, 8)):
+        base = run(lambda n: (), split)
+        assert base.isfinite().all()
+        assert torch.equal(run(lambda n: range(max(n - window, 0)), split), base)
+        assert not run(lambda n: (max(n - window, 0),), split).isfinite().any()
+
+
 @pytest.mark.parametrize("kernel", ["prefill_bf16_tc", "prefill_bf16_tma", "prefill_bf16_plain", "generic_bf16",
                                     "generic_f32"])
 def test_attention_far_key_stands_out_in_every_kernel(kernel):

@@ -283,6 +283,8 @@ attn_f32_decode_kernel(const AttnArgs a) {
     const int at = (i - begin) & 1, key0 = (pg0 + i) * PAGE;
     cp_wait<1>();
     __syncthreads();
+    // values that have left the window must not reach the sum, whatever they are: 0 x NaN is NaN
+    for (int e = part; e < lo - key0; e += PARTS) Vs[at * Sizes<HD>::V + d * VLD + e] = 0.0f;
     {
       // a key and half of the dimensions per thread
       float s[GM];
