@@ -581,6 +581,35 @@ def test_attention_f32_keeps_unseen_values_out(poison):
     assert out[:bad].isfinite().all() and not out[bad:].isfinite().any()
 
 
+@pytest.mark.parametrize("window", [None, 90])
+def test_attention_f32_counts_a_seen_value_whose_weight_vanishes(window):
+    """A key far below the others has a weight of 0 in 32 bits; its value, if it is no number, makes the sum none all the same,
+    in the page of the token itself as in any other page (what the kernel for every head size gives)."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc.attention_f32 import AttentionF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    nh, nkv, hd, n = 8, 2, 64, 200
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(is_decode=False, n_seqs=1, len_bucket=256, total_bucket=256, max_new=n, seq_start=i32([0, n]),
+                            seq_len=i32([n]), max_len=n)
+    for bad in (5, 64, 130, 199):
+        pc = Paged([n], nkv, hd, torch.float32, 9)
+        batch.seq_slot = pc.seq_slot
+        page = int(pc.table[pc.slots[0], bad // PAGE])
+        q = _rand((n, nh * hd), torch.float32, 6).abs()
+        pc.k_pages[page, :, bad % PAGE] = -1e4
+        pc.v_pages[page, :, :, bad % PAGE] = float("nan")
+        view = SimpleNamespace(k_pages=pc.k_pages, v_pages=pc.v_pages, page_table=pc.table)
+        out, every = torch.empty((n, nh * hd), device=DEV), torch.empty((n, nh * hd), device=DEV)
+        assert AttentionF32.get(hd).run(q, view, out, batch, nh, nkv, window, 0.125, Workspace(torch.device(DEV)))
+        _ops(torch.float32).attn_generic(q, pc.k_pages, pc.v_pages, every, i32(list(range(n))), i32([0] * n), pc.seq_slot, pc.table,
+                                         nh, nkv, hd, window, 0.125)
+        sees = torch.zeros(n, dtype=torch.bool, device=DEV)
+        sees[bad:min(n, bad + window) if window else n] = True
+        for x in (out, every):
+            assert x[sees].isnan().all() and x[~sees].isfinite().all(), bad
+
+
 @pytest.mark.parametrize("poison", [float("inf"), float("nan")])
 @pytest.mark.parametrize("nh,nkv,hd,window", [(4, 2, 64, 70), (8, 1, 128, 64), (2, 2, 16, 33), (4, 1, 32, 1)])
 def test_attention_f32_decode_keeps_values_before_the_window_out(nh, nkv, hd, window, poison):

@@ -179,6 +179,15 @@ attn_f32_prompt_kernel(const AttnArgs a, int tokens_per_block) {
         Ps[(ty * 4 + i) * VLD + tx + 16 * j] = p;
       }
     }
+    if (masked) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = key0 + tx + 16 * j;
+          if (key > pos[i] || (a.window > 0 && key <= pos[i] - a.window)) Ps[(ty * 4 + i) * VLD + tx + 16 * j] = -1.0f;
+        }
+    }
     cp_wait<1>();          // the page's values
     __syncthreads();
 #pragma unroll 2
@@ -189,15 +198,16 @@ attn_f32_prompt_kernel(const AttnArgs a, int tokens_per_block) {
 #pragma unroll
       for (int j = 0; j < DJ; ++j) vv[j] = *reinterpret_cast<const float4*>(Vs + (tx + 16 * j) * VLD + k);
       if (masked) {
-        // a value that a row does not see must not reach it, whatever it is
+        // a value that a row does not see (weight -1) must not reach it, whatever it is; one that it does see counts, however
+        // small its weight
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < DJ; ++j) {
-            if (pv[i].x != 0.0f) acc[i][j] = fmaf(pv[i].x, vv[j].x, acc[i][j]);
-            if (pv[i].y != 0.0f) acc[i][j] = fmaf(pv[i].y, vv[j].y, acc[i][j]);
-            if (pv[i].z != 0.0f) acc[i][j] = fmaf(pv[i].z, vv[j].z, acc[i][j]);
-            if (pv[i].w != 0.0f) acc[i][j] = fmaf(pv[i].w, vv[j].w, acc[i][j]);
+            if (!(pv[i].x < 0.0f)) acc[i][j] = fmaf(pv[i].x, vv[j].x, acc[i][j]);
+            if (!(pv[i].y < 0.0f)) acc[i][j] = fmaf(pv[i].y, vv[j].y, acc[i][j]);
+            if (!(pv[i].z < 0.0f)) acc[i][j] = fmaf(pv[i].z, vv[j].z, acc[i][j]);
+            if (!(pv[i].w < 0.0f)) acc[i][j] = fmaf(pv[i].w, vv[j].w, acc[i][j]);
           }
       } else {
 #pragma unroll
