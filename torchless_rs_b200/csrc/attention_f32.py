@@ -52,10 +52,11 @@ class AttentionF32:
         self._sms = {}
 
     def _load(self) -> None:
-        self.lib = build.load_library("attn_f32")
+        lib = build.load_library("attn_f32")
         P, I = c_void_p, c_int
-        self.lib.tl_attn_f32.restype = c_int
-        self.lib.tl_attn_f32.argtypes = [P] * 8 + [I] * 7 + [c_float, I, P, I, I, P]
+        lib.tl_attn_f32.restype = c_int
+        lib.tl_attn_f32.argtypes = [P] * 8 + [I] * 7 + [c_float, I, P, I, I, P]
+        self.lib = lib        # last: another thread calls as soon as it is there
 
     def run(self, q: torch.Tensor, cache_view, out: torch.Tensor, batch, nh: int, nkv: int, window, scale: float,
             workspace) -> bool:

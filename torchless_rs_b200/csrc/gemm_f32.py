@@ -27,13 +27,14 @@ class GemmF32:
         self._sms = {}
 
     def _load(self) -> None:
-        self.lib = build.load_library("gemm_split")
+        lib = build.load_library("gemm_split")
         P, I = c_void_p, c_int
-        self.lib.tl_gemm_split.restype = c_int
-        self.lib.tl_gemm_split.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P, P]
-        self.lib.tl_gemm_split_scratch.restype = c_longlong
-        self.lib.tl_gemm_split_scratch.argtypes = [I, I]
-        self.lib.tl_gemm_split_take_error.restype = c_int
+        lib.tl_gemm_split.restype = c_int
+        lib.tl_gemm_split.argtypes = [P, I, P, I, P, I, I, I, I, I, I, P, P]
+        lib.tl_gemm_split_scratch.restype = c_longlong
+        lib.tl_gemm_split_scratch.argtypes = [I, I]
+        lib.tl_gemm_split_take_error.restype = c_int
+        self.lib = lib        # last: another thread calls as soon as it is there
         register_error_word("gemm_split", self.take_error)
 
     @staticmethod
