@@ -23,3 +23,20 @@ def test_a_library_is_seen_only_when_its_functions_know_their_types(make, monkey
     user._load()
     assert "argtypes" in declared and not any(early)
     assert isinstance(user.lib, Library)
+
+
+def test_error_words_are_read_while_another_library_is_loaded(monkeypatch):
+    """A library that another thread loads registers its error word while this one reads those that are there."""
+    from torchless_rs_b200.csrc import ops
+    words = {}
+    monkeypatch.setattr(ops, "_error_words", words)
+
+    def take():
+        ops.register_error_word("late", lambda: 0)
+        return 0
+    words["early"] = take
+    ops.check_kernel_errors()
+    assert set(words) == {"early", "late"}
+    words["late"] = lambda: 3
+    with pytest.raises(ops.KernelError, match="late: code 3"):
+        ops.check_kernel_errors()

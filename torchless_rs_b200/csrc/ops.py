@@ -40,7 +40,7 @@ def register_error_word(name: str, take: Callable[[], int]) -> None:
 def check_kernel_errors() -> None:
     """Reads every registered error word (this synchronises the device) and raises if one is
     set.  Callers use it where they wait for results anyway."""
-    bad = {name: code for name, code in ((n, take()) for n, take in _error_words.items()) if code}
+    bad = {name: code for name, code in ((n, take()) for n, take in list(_error_words.items())) if code}
     if bad:
         raise KernelError("a kernel ran out of a bounded wait, its results are not valid: " +
                           ", ".join(f"{n}: code {c}" for n, c in bad.items()))
