@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "pdl.cuh"
+#include "per_device.cuh"
 
 #define PAGE 64
 static_assert(TL_PAGE == PAGE, "the tiles are pages of 64 keys");
@@ -410,7 +411,7 @@ attn_f32_merge_kernel(const AttnArgs a) {
 template <int HD>
 static int run_prompt(const AttnArgs& a, int seqs, int max_new, cudaStream_t stream) {
   const int smem = (2 * P_ROWS * Sizes<HD>::KLD + Sizes<HD>::V + P_ROWS * Sizes<HD>::VLD) * 4;
-  static const cudaError_t set = cudaFuncSetAttribute(attn_f32_prompt_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t set = tl_allow_smem<attn_f32_prompt_kernel<HD>>(smem);
   if (set != cudaSuccess) return (int)set;
   const int per = P_ROWS / (a.nh / a.nkv);
   return tl_launch(attn_f32_prompt_kernel<HD>, dim3((max_new + per - 1) / per, a.nkv, seqs), dim3(P_THREADS), (size_t)smem, stream, a, per);
@@ -418,7 +419,7 @@ static int run_prompt(const AttnArgs& a, int seqs, int max_new, cudaStream_t str
 template <int HD, int GM>
 static int run_decode(const AttnArgs& a, int seqs, cudaStream_t stream) {
   const int smem = (2 * Sizes<HD>::K + 2 * Sizes<HD>::V + GM * (HD + 2 * PAGE + D_THREADS + 3)) * 4;
-  static const cudaError_t set = cudaFuncSetAttribute(attn_f32_decode_kernel<HD, GM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t set = tl_allow_smem<attn_f32_decode_kernel<HD, GM>>(smem);
   if (set != cudaSuccess) return (int)set;
   int rc = tl_launch(attn_f32_decode_kernel<HD, GM>, dim3(a.splits, a.nkv, seqs), dim3(D_THREADS), (size_t)smem, stream, a);
   if (rc == 0 && a.splits > 1) rc = tl_launch(attn_f32_merge_kernel<HD>, dim3(a.nh, seqs), dim3(HD), 0, stream, a);

@@ -50,6 +50,7 @@
 #include <stdint.h>
 
 #include "pdl.cuh"
+#include "per_device.cuh"
 #include "umma.cuh"
 
 #include <mutex>
@@ -506,8 +507,7 @@ static SpEncodeFn sp_encode() {
 
 template <bool SWIGLU>
 static cudaError_t sp_configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int splits) {
-  static const cudaError_t set =
-      cudaFuncSetAttribute(gemm_split_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM);
+  const cudaError_t set = tl_allow_smem<gemm_split_kernel<SWIGLU>>(SP_SMEM);
   cfg.blockDim = dim3(SP_THREADS);
   cfg.dynamicSmemBytes = SP_SMEM;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -520,13 +520,16 @@ static cudaError_t sp_configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&a
   cfg.numAttrs = 2;
   return set;
 }
-// How many clusters of `splits` blocks run at once (the GPCs differ in size: not the SMs divided by it).
+// How many clusters of `splits` blocks run at once on this device (the GPCs differ in size: not the SMs divided by it).
 template <bool SWIGLU>
 static int sp_clusters(int splits, int num_sms) {
-  static int known[SP_MAX_SPLITS + 1];
+  static int known_on[TL_DEVICES][SP_MAX_SPLITS + 1];
   static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
   if (splits == 1) return num_sms;
+  const int device = tl_device();
+  int unknown[SP_MAX_SPLITS + 1] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  int* known = device >= 0 ? known_on[device] : unknown;
   if (known[splits] == 0) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];

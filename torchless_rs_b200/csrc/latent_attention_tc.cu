@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include "pdl.cuh"
+#include "per_device.cuh"
 #include "umma.cuh"
 
 #include <mutex>
@@ -529,7 +530,7 @@ extern "C" int tl_latent_attn_tc(const float* qa, int ld_qa, int qa_head, const 
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   if (!make(&tm, box, CU_TENSOR_MAP_SWIZZLE_128B) || !make(&tm_r, box_r, CU_TENSOR_MAP_SWIZZLE_64B)) return -2;
-  static const cudaError_t set = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM);
+  const cudaError_t set = tl_allow_smem<latent_attn_tc_kernel>(LT_SMEM);
   if (set != cudaSuccess) return (int)set;
   LatentArgs a = {qa, q, (const __nv_bfloat16*)pages, o, seq_start, token_pos, seq_slot, page_table, inv_freq, sink, ld_qa, qa_head, ldq, q_head, q_off,
                   table_stride, heads, rot, dims, window, LT_ROWS / heads, scale * 1.4426950408889634f, amp};

@@ -12,6 +12,7 @@
 // FMAs and SCAN_COLS warp sums; the activations of a row are computed by every warp that needs
 // them rather than stored and read again.
 #include "common.cuh"
+#include "per_device.cuh"
 
 #define SCAN_COLS 4          // columns per warp (warp_sum4 is written for 4)
 #define SCAN_WARPS 4         // warps per block
@@ -322,8 +323,7 @@ extern "C" int TL_NAME(tl_gated_scan)(float* zq, float* zf, const float* zv, int
     const size_t smem = sizeof(float) * (WALK_STAGES * WALK_T * (2 * dim + WALK_COLS) + WALK_T * (WALK_GROUPS + 1) * WALK_COLS);
 #define WALK(RPT)                                                                                                       \
   do {                                                                                                                  \
-    static const cudaError_t set =                                                                                      \
-        cudaFuncSetAttribute(gated_walk_kernel<RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);           \
+    const cudaError_t set = tl_allow_smem<gated_walk_kernel<RPT>>(96 * 1024);                                           \
     if (set != cudaSuccess) return (int)set;                                                                            \
     return tl_launch(gated_walk_kernel<RPT>, walk, dim3(WALK_THREADS), smem, stream, (const float*)zq, (const float*)zf, zv, \
                      ld, state, o, ldo, seq_start, seq_slot, heads, vdim);                                              \

@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include "pdl.cuh"
+#include "per_device.cuh"
 #include "umma.cuh"
 
 #include <mutex>
@@ -292,7 +293,7 @@ static bool mt_map(CUtensorMap* m, const void* ptr, long long rows, int K, long 
 
 template <bool UP>
 static int run_moe(const CUtensorMap& tw, const CUtensorMap& tx, const MoeArgs& a, int smem, int blocks, cudaStream_t stream) {
-  static const cudaError_t set = cudaFuncSetAttribute(moe_tc_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  const cudaError_t set = tl_allow_smem<moe_tc_kernel<UP>>(227 * 1024);
   if (set != cudaSuccess) return (int)set;
   return tl_launch(moe_tc_kernel<UP>, dim3(blocks), dim3(MT_THREADS), (size_t)smem, stream, tw, tx, a);
 }
