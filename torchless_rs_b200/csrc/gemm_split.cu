@@ -206,26 +206,28 @@ __device__ __forceinline__ void sp_write(const SplitArgs& a, float (&v)[16], int
   if (bad) {            // (a branch and no function: the callers' register budgets differ)
     const float* x = a.X + (size_t)m * a.ldx;
     const float* w = a.W + (size_t)(up ? a.N + n : n) * a.ldw;
-    // a walk along K for eight of them (one after the other an activation tensor of NaN took 27 ms at 300 x 4096 x 4096, 45 times
-    // what the CUDA-core kernel takes; all sixteen at once spill); K, W and its rows allow 16-byte loads
+    // a walk along K for GROUP of them (one after the other an activation tensor of NaN took 27 ms at 300 x 4096 x 4096, 45 times
+    // what the CUDA-core kernel takes; more than two under the SiLU-gate spill, which cost finite products 2 %); K, W and
+    // its rows allow 16-byte loads
+    constexpr int GROUP = SWIGLU ? 2 : 8;
 #pragma unroll
-    for (int j0 = 0; j0 < 16; j0 += 8) {
-      if (!(bad >> j0 & 0xffu)) continue;
-      float sum[8];
+    for (int j0 = 0; j0 < 16; j0 += GROUP) {
+      if (!(bad >> j0 & ((1u << GROUP) - 1u))) continue;
+      float sum[GROUP];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) sum[j] = 0.0f;
-#pragma unroll 1
+      for (int j = 0; j < GROUP; ++j) sum[j] = 0.0f;
+#pragma unroll (SWIGLU ? 2 : 1)
       for (int k = 0; k < a.K; k += 4) {
         const float4 wv = *reinterpret_cast<const float4*>(w + k);
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < GROUP; ++j)
           if (bad >> (j0 + j) & 1) {
             const float* xj = x + (size_t)(j0 + j) * a.ldx + k;
             sum[j] = fmaf(xj[3], wv.w, fmaf(xj[2], wv.z, fmaf(xj[1], wv.y, fmaf(xj[0], wv.x, sum[j]))));
           }
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < GROUP; ++j)
         if (bad >> (j0 + j) & 1) v[j0 + j] = sum[j];
     }
   }
