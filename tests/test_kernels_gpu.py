@@ -167,6 +167,24 @@ def test_gemm_split_gives_what_the_cuda_core_kernel_gives_where_results_are_not_
             assert torch.allclose(c[ok], plain[ok], rtol=1e-4, atol=1e-3), (where, value, mode)
 
 
+@pytest.mark.parametrize("x_exp,w_exp", [(-90, 0), (-100, 10), (-118, 0), (-124, 0), (-130, 20), (0, -120), (-60, -50), (-70, -60)])
+def test_gemm_split_of_small_numbers_is_no_further_off_than_the_cuda_core_kernel(x_exp, w_exp):
+    """Numbers whose bfloat16 pieces fall below the smallest bfloat16 number, in activations or weights, down to results that
+    are themselves subnormal (there both round the last sum to a multiple of 2^-149)."""
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    g, o, ws = GemmF32.get(), _ops(torch.float32), Workspace(torch.device(DEV))
+    for M, N, K in ((9, 1024, 1024), (200, 1100, 1024)):
+        a, w = _rand((M, K), torch.float32, 3) * 2.0 ** x_exp, _rand((N, K), torch.float32, 4) * 2.0 ** w_exp
+        a[3] = 0.0
+        want = a.double() @ w.double().T
+        c, plain = torch.empty((M, N), device=DEV), torch.empty((M, N), device=DEV)
+        assert g.run(a, w, c, 0, ws)
+        o.gemm_generic(a, w, plain, 0)
+        err = [float(((y.double() - want) * 2.0 ** -(x_exp + w_exp)).norm()) for y in (c, plain)]
+        assert (c[3] == 0).all() and err[0] <= 1.2 * err[1], err
+
+
 def test_gemm_split_of_activations_that_are_no_numbers_is_not_slow():
     """Results that are not finite are computed again; with all of them so, a product stays within some times what the
     CUDA-core kernel takes (measured: 3 to 4; one result after the other it was 45)."""

@@ -16,7 +16,10 @@
 //
 // A result that is not finite (an infinity or a NaN in an operand, a number that rounds to infinity in bfloat16, an
 // overflow of one of the products) is computed again as the plain sequence of multiply-adds, so such operands give what
-// they give there.
+// they give there.  So is one below 2^-90 that is not 0: what a number below 2^-117 loses, up to 2^-134, counts in results
+// that small (operands of size 2^-118 and 1 were 9e-6 off, of 2^-124 6e-4).  In larger results it counts only where numbers
+// below 2^-117 meet some above 2^20.  A product whose results are all of these kinds takes some four times what the
+// CUDA-core kernel does.
 //
 // One block computes 128 rows of W (the M operand of tcgen05.mma) times up to 192 tokens.
 //   warps 0-3   sums in registers, epilogue
@@ -76,6 +79,8 @@
 #define SP_COST_STAGE 750.0
 #define SP_COST_ROUND 8000.0
 #define SP_COST_REDUCE 40.0
+
+#define SP_LEAST ((127u - 90u) << 23)   // 2^-90 as its bits
 
 #define MODE_ACCUM_F32 1
 #define MODE_SWIGLU 2
@@ -199,10 +204,12 @@ __device__ __forceinline__ void sp_write(const SplitArgs& a, float (&v)[16], int
                                          int turn, int group) {
   const bool up = SWIGLU && row >= 64;
   const int n = n0 + (SWIGLU ? (row & 63) : row);
-  uint32_t bad = 0;   // results that are not finite: the plain sequence of multiply-adds
+  uint32_t bad = 0;   // results that are not finite, or so small that the operands may have lost bits: the plain sequence of multiply-adds
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
-    if (!(fabsf(v[j]) <= 3.402823466e38f) && n < a.N && j < tokens) bad |= 1u << j;
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t size = __float_as_uint(v[j]) & 0x7fffffffu;       // ordered as the absolute values are, infinities and NaN last
+    if (size != 0u && size - SP_LEAST >= 0x7f800000u - SP_LEAST && n < a.N && j < tokens) bad |= 1u << j;
+  }
   if (bad) {            // (a branch and no function: the callers' register budgets differ)
     const float* x = a.X + (size_t)m * a.ldx;
     const float* w = a.W + (size_t)(up ? a.N + n : n) * a.ldw;
