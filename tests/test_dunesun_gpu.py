@@ -766,3 +766,30 @@ def test_blocks_that_take_no_addend_work_in_repeated_passes():
     s2 = eng.start_sequences(1)
     one = np.concatenate([eng.step(s2, [[t]], "last").cpu().numpy().copy() for t in toks])
     assert np.allclose(whole, one, atol=2e-4 * np.abs(whole).max())
+
+
+def test_experts_input_rows_take_no_buffer_of_their_own():
+    """The rows in the grouped order lie where the second product's output will be: a step's buffers for experts are the
+    router's, the plan's, the activations and that output, however many tokens it has; and a room that is too small is refused."""
+    tm = DModel("C", "bfloat16", seed=0, max_tokens=1024)
+    toks = tokens_of(np.random.default_rng(3), 500, tm.cfg["vocab"])
+    s = tm.engine.start_sequences(1)
+    tm.step_np([s[0]], [toks], "all")
+    held = {k[0]: b.numel() * b.element_size() for k, b in tm.engine.rt.workspace._bufs.items() if k[0].startswith("moe_")}
+    known = {"moe_logits", "moe_idx", "moe_wt", "moe_offsets", "moe_row_token", "moe_row_of", "moe_expert_out", "moe_act",
+             "moe_shared_act", "moe_shared_out"}
+    assert "moe_expert_out" in held and set(held) <= known, held
+    o, E, N, K, T = _ops(torch.bfloat16), 3, 40, 64, 70
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", generator=g).to(torch.bfloat16)
+    a, w = rnd(T, K), rnd(E, 2 * N, K)
+    off, row_token = _i32([0, 30, 30, T]), _i32(np.random.default_rng(2).permutation(T))
+    outs = []
+    for room in (None, torch.full((T, K), float("nan"), device="cuda"), rnd(T * K), torch.empty(2 * T * K, dtype=torch.uint8, device="cuda")):
+        c = torch.zeros((T, N), device="cuda", dtype=torch.bfloat16)
+        o.moe_gemm(a, row_token, w, c, off, up=True, act=0, room=room, most=T)
+        outs.append(c)
+    assert all(torch.equal(outs[0], c) for c in outs) and outs[0].abs().sum() > 0
+    from torchless_rs_b200.csrc.ops import KernelError
+    with pytest.raises(KernelError):
+        o.moe_gemm(a, row_token, w, c, off, up=True, act=0, room=rnd(T * K - 1), most=T)

@@ -997,12 +997,12 @@ class CoreOps:
 
     def moe_gemm(self, a: torch.Tensor, row_token: Optional[torch.Tensor], w: torch.Tensor, c: torch.Tensor,
                  offsets: torch.Tensor, up: bool, limit: float = 0.0, alpha: float = 0.0,
-                 act: int = ACT_CLAMPED_GLU, grouped: Optional[torch.Tensor] = None, most: Optional[int] = None) -> None:
+                 act: int = ACT_CLAMPED_GLU, room: Optional[torch.Tensor] = None, most: Optional[int] = None) -> None:
         """The experts' products over rows grouped by expert.  up: c[row] = act(gate, up) of a[row_token[row]]
         with w [experts, 2 N, K] (`act`: ACT_CLAMPED_GLU with `limit` and `alpha`, or ACT_PLAIN, silu(gate) * up);
-        else c[row] (32-bit) = a[row] . w[expert] with w [experts, N, K].  `grouped` [rows of c, K]: room for the
-        rows of `a` in the grouped order (up, bfloat16; made here if not given).  `most`: no expert has more rows
-        (a token chooses an expert once, so the number of tokens)."""
+        else c[row] (32-bit) = a[row] . w[expert] with w [experts, N, K].  `room` (up, bfloat16): a contiguous tensor of any
+        type with 2 K bytes for each row of c, where the rows of `a` in the grouped order are put for the product (made here if
+        not given).  `most`: no expert has more rows (a token chooses an expert once, so the number of tokens)."""
         if act not in (ACT_PLAIN, ACT_CLAMPED_GLU):
             raise KernelError(f"moe_gemm: no such activation ({act})")
         _need(a, self.act_dtype, "expert input")
@@ -1015,13 +1015,13 @@ class CoreOps:
         if self.act_dtype == torch.bfloat16:
             # the tensor-core kernel, where alignments allow it
             from .moe_bf16 import MoeBf16
-            if up and grouped is None:
-                grouped = torch.empty((c.shape[0], K), dtype=a.dtype, device=a.device)
-            if up and (grouped.shape != (c.shape[0], K) or grouped.dtype != a.dtype or not grouped.is_contiguous()):
+            if up and room is None:
+                room = torch.empty((c.shape[0], K), dtype=a.dtype, device=a.device)
+            if up and (not room.is_contiguous() or room.numel() * room.element_size() < 2 * c.shape[0] * K):
                 raise KernelError("moe_gemm: the room for the grouped rows does not fit")
             if most is None:
                 most = a.shape[0] if up else c.shape[0]
-            if MoeBf16.get().run(a, row_token, grouped, w, c, offsets, min(most, c.shape[0]), N, up, act, limit, alpha):
+            if MoeBf16.get().run(a, row_token, room, w, c, offsets, min(most, c.shape[0]), N, up, act, limit, alpha):
                 return
         _check(self._tl_moe_gemm(_ptr(a), c_int(a.stride(0)), _ptr(row_token), _ptr(w), _ptr(c), c_int(c.stride(0)),
                                  _ptr(offsets), c_int(E), c_int(c.shape[0]), c_int(N), c_int(K), c_int(1 if up else 0), c_int(act),

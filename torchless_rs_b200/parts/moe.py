@@ -7,7 +7,8 @@
     expert e >= experts: y_e = h
     output = sum over the chosen of weight * y_e
 The (token, expert) pairs are grouped by expert on the device; the experts' products run over the
-groups (no host value is read, so decode steps replay from CUDA graphs)."""
+groups (no host value is read, so decode steps replay from CUDA graphs).  The first product brings its input rows into the
+grouped order; they lie, for that long, where the second product's 32-bit output will be."""
 from __future__ import annotations
 
 from typing import Dict, Optional
@@ -20,11 +21,6 @@ from ..weights.loader import TensorSpec
 from .linear import Matmul
 from .registry import register_feed_forward
 from .runtime import Runtime
-
-
-def _grouped_rows(rt: Runtime, rows: int, hidden: int) -> Optional[torch.Tensor]:
-    """Room for the experts' input rows in the grouped order; the 32-bit kernel reads them where they lie."""
-    return None if rt.is_f32 else rt.workspace.get("moe_rows", (rows, hidden), rt.act_dtype)
 
 
 @register_feed_forward("moe_clamped")
@@ -85,7 +81,7 @@ class ClampedMoE:
         if E:
             act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
             rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, limit=self.limit,
-                            alpha=self.gate_alpha, grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+                            alpha=self.gate_alpha, room=yk, most=T)
             rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         rt.ops.moe_combine(yk, row_of, wt, xn, residual, accumulate=not overwrite)
 
@@ -168,7 +164,7 @@ class GroupedSigmoidMoE:
         yk = ws.get("moe_expert_out", (T * top, self.hidden), torch.float32)
         act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
         rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, limit=self.limit, alpha=self.gate_alpha,
-                        grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+                        room=yk, most=T)
         rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         rt.ops.moe_combine(yk, row_of, wt, xn, residual, accumulate=not overwrite)
         if self.shared_ff:
@@ -259,7 +255,7 @@ class SoftmaxChosenMoE:
         yk = ws.get("moe_expert_out", (T * top, self.hidden), torch.float32)
         act = ws.get("moe_act", (T * top, self.ff), rt.act_dtype)
         rt.ops.moe_gemm(xn, row_token, self.w_up, act, offsets, up=True, act=ops.ACT_PLAIN,
-                        grouped=_grouped_rows(rt, T * top, self.hidden), most=T)
+                        room=yk, most=T)
         rt.ops.moe_gemm(act, None, self.w_down, yk, offsets, up=False, most=T)
         if not self.shared_ff:
             return (yk, row_of, wt), None
