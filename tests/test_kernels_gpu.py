@@ -185,6 +185,38 @@ def test_gemm_split_of_small_numbers_is_no_further_off_than_the_cuda_core_kernel
         assert (c[3] == 0).all() and err[0] <= 1.2 * err[1], err
 
 
+def test_gemm_split_holds_a_bounded_buffer_and_does_without(monkeypatch):
+    """Many rows go in several launches with the pieces of some at a time, the last one ragged, with strided rows and in every
+    mode; without memory for the pieces the product is left to the CUDA-core kernel."""
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    g, M, N, K = GemmF32.get(), 1000, 1030, 1024
+    a, w = _rand((M, K + 4), torch.float32, 3)[:, :K], _rand((2 * N, K), torch.float32, 4, 1.0 / math.sqrt(K))
+    base = _rand((M, N + 3), torch.float32, 5)
+    outs = []
+    for bound in (g.SCRATCH, 300 * 6 * K):
+        monkeypatch.setattr(GemmF32, "SCRATCH", bound)
+        ws = Workspace(torch.device(DEV))
+        row = []
+        for mode in (ops.MODE_STORE_F32, ops.MODE_ACCUM_F32, ops.MODE_SWIGLU):
+            c = base.clone()
+            before = ops.launch_counts().get("gemm_split", 0)
+            assert g.run(a, w if mode == ops.MODE_SWIGLU else w[:N], c[:, :N], mode, ws)
+            assert ops.launch_counts()["gemm_split"] - before == (6 if outs else 1)
+            assert torch.equal(c[:, N:], base[:, N:])
+            row.append(c)
+        assert ws.bytes_held() <= bound + 16
+        outs.append(row)
+    for x, y in zip(*outs):     # the tiles may differ, so may the order of 32-bit sums
+        assert (x - y).norm() <= 1e-6 * x.norm()
+
+    class Full(Workspace):
+        def get(self, *args):
+            raise torch.cuda.OutOfMemoryError("none left")
+    assert not g.run(a, w[:N], base[:, :N].clone(), 0, Full(torch.device(DEV)))
+
+
 def test_gemm_split_of_activations_that_are_no_numbers_is_not_slow():
     """Results that are not finite are computed again; with all of them so, a product stays within some times what the
     CUDA-core kernel takes (measured: 3 to 4; one result after the other it was 45)."""

@@ -15,6 +15,11 @@ build.register_library("gemm_split", ("gemm_split.cu",), ())
 class GemmF32:
     _inst = None
     LEAST = 1 << 20       # no product with a smaller matrix is taken
+    # Most bytes of pieces (6 for each number of the activations) that are held: 65,536 tokens of 14336 columns would be 5.6
+    # GB, half as much again as the step's largest activation.  At the bound a launch has 6208 rows and more of these
+    # columns, 7 rounds of blocks and more over 4096 outputs.
+    SCRATCH = 1 << 29
+    ROWS = 192            # rows of a launch: a multiple of the kernel's largest tile
 
     @classmethod
     def get(cls) -> "GemmF32":
@@ -66,14 +71,22 @@ class GemmF32:
         key = a.device.index if a.device.index is not None else torch.cuda.current_device()
         if key not in self._sms:
             self._sms[key] = torch.cuda.get_device_properties(a.device).multi_processor_count
-        n = int(self.lib.tl_gemm_split_scratch(M, K))
-        scratch = workspace.get("gemm_split_pieces", ((n + 3) // 4,), torch.int32)
-        st = self.lib.tl_gemm_split(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0),
-                                    M, N, K, mode, self._sms[key], scratch.data_ptr(), _stream())
-        if st == -2:
-            return False
-        _check(st, "gemm_split")
-        _check(0, "split_rows")      # the kernel before it counts too
+        # many rows in several launches, so that the pieces of all rows are never held at once
+        most = max(self.SCRATCH // self.lib.tl_gemm_split_scratch(self.ROWS, K), 1) * self.ROWS
+        parts = -(-M // most)
+        rows = M if parts == 1 else -(-M // (parts * self.ROWS)) * self.ROWS
+        try:
+            scratch = workspace.get("gemm_split_pieces", ((int(self.lib.tl_gemm_split_scratch(rows, K)) + 3) // 4,), torch.int32)
+        except torch.cuda.OutOfMemoryError:
+            return False              # the CUDA-core kernel needs no room
+        for m in range(0, M, rows):
+            st = self.lib.tl_gemm_split(a.data_ptr() + 4 * m * a.stride(0), a.stride(0), w.data_ptr(), w.stride(0),
+                                        out.data_ptr() + 4 * m * out.stride(0), out.stride(0), min(rows, M - m), N, K, mode,
+                                        self._sms[key], scratch.data_ptr(), _stream())
+            if st == -2 and m == 0:
+                return False
+            _check(st, "gemm_split")
+            _check(0, "split_rows")      # the kernel before it counts too
         return True
 
     def take_error(self) -> int:
