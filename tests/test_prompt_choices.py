@@ -1,7 +1,7 @@
 """Host rules that choose a kernel from a step's sizes (no device needed), at sizes where both sides were timed."""
 import pytest
 
-from torchless_rs_b200.csrc.latent_bf16 import prompt_times
+from torchless_rs_b200.csrc import attention_f32, latent_bf16
 
 
 @pytest.mark.parametrize("past,new,heads,window,tiles", [
@@ -15,5 +15,21 @@ from torchless_rs_b200.csrc.latent_bf16 import prompt_times
     ([0], [33], 128, 4096, False), ([1000] * 4, [1033] * 4, 128, 4096, True), ([0] * 32, [600] * 32, 8, 4096, True),
     ([0], [4096], 1, 4096, True)])
 def test_latent_attention_of_prompts_runs_where_it_was_faster(past, new, heads, window, tiles):
-    here, there = prompt_times(past, new, heads, window, 148)
+    here, there = latent_bf16.prompt_times(past, new, heads, window, 148)
     assert (here < there) == tiles, (here, there)
+
+
+@pytest.mark.parametrize("past,new,nh,nkv,hd,window,tiles", [
+    ([2000], [2002], 32, 8, 128, None, False), ([2000], [2008], 32, 8, 128, None, True), ([8000], [8004], 32, 8, 128, None, False),
+    ([500], [508], 32, 8, 128, None, True), ([500], [504], 32, 8, 128, None, False), ([100], [108], 32, 8, 128, None, False),
+    ([100], [116], 32, 8, 128, None, True), ([0], [400], 32, 8, 128, None, True), ([0, 0], [400, 131], 32, 8, 128, None, True),
+    ([0], [42], 32, 8, 128, None, True), ([0] * 64, [5] * 64, 32, 8, 128, None, False), ([100] * 64, [102] * 64, 32, 8, 128, None, True),
+    ([999] * 4, [1000] * 3 + [1001], 32, 8, 128, None, True), ([3999, 3998], [4000, 4000], 32, 8, 128, None, False),
+    ([100] * 64, [102] * 64, 32, 32, 128, None, False), ([0] * 16, [64] * 16, 32, 32, 128, None, True),
+    ([2000], [2008], 32, 8, 128, 200, False), ([2000], [2016], 32, 8, 128, 200, True),
+    ([500], [508], 16, 4, 64, None, False), ([500], [532], 16, 4, 64, None, True), ([2000], [2064], 64, 8, 64, None, True),
+    ([500], [502], 8, 8, 32, None, True), ([0] * 64, [5] * 64, 8, 8, 32, None, False), ([2000], [2002], 4, 2, 16, None, True),
+    ([500], [564], 4, 2, 16, 200, False), ([500], [628], 32, 8, 16, 200, True)])
+def test_32_bit_prompt_attention_runs_where_it_was_faster(past, new, nh, nkv, hd, window, tiles):
+    in_tiles, by_rows = attention_f32.prompt_times(past, new, nh, nkv, hd, window, 148)
+    assert (in_tiles < by_rows) == tiles, (in_tiles, by_rows)

@@ -14,10 +14,8 @@ build.register_library("attn_f32", ("attention_f32.cu",), ())
 
 HEAD_DIMS = (16, 32, 64, 128)
 MAX_GROUP_DECODE, MAX_GROUP_PROMPT = 8, 64      # query heads per key/value head
-# Rows (tokens x heads) times the longest sequence's keys from which on a prompt step's tiles are faster than a block per
-# row: a tile takes its page's time however few of its 64 rows are filled.  Device time, tiles / blocks: 32 heads of
-# 128, 3 tokens after 97 24 / 15 us (9600), 42 tokens 15 / 20 us (31,000), 20 tokens after 980 161 / 440 us; 4 heads of 16, 60
-# tokens 5.7 / 3.7 us (14,400).
+# Rows (tokens x heads) times the longest sequence's keys below which a prompt step runs by a block per row without a second
+# look: 4 heads of 16, 60 tokens 3.7 us so and 5.7 in tiles (14,400).
 PROMPT_FROM = 16384
 PAGE = build.PAGE_TOKENS
 
@@ -34,6 +32,38 @@ def decode_split(n_seqs: int, nkv: int, len_bucket: int, total_bucket: int, wind
         longest, pages = min(longest, seen), min(pages, n_seqs * seen)
     per = longest if longest <= 4 else max(1, min(16, -(-pages * nkv // sms)))
     return per, -(-longest // per)
+
+
+# us of a prompt step by head size: a tile's page; a block per row's key of its longest row, key of any row, row
+PAGE_US = {16: 2.6, 32: 3.7, 64: 5.8, 128: 10.1}
+CHAIN_US = {16: 0.061, 32: 0.079, 64: 0.088, 128: 0.1205}
+KEY_US = {16: 0.085e-3, 32: 0.17e-3, 64: 0.33e-3, 128: 0.65e-3}
+ROW_US = {16: 1.4e-3, 32: 1.6e-3, 64: 2.4e-3, 128: 3.4e-3}
+
+
+def prompt_times(past_lens, new_lens, nh: int, nkv: int, hd: int, window: Optional[int], sms: int) -> Tuple[float, float]:
+    """What a prompt step takes, in us, in tiles of 64 rows and by a block per row (attention_generic.cu), from what each
+    sequence holds before and after it.  A tile takes its pages' time however few of its rows are filled (more per page at
+    a window's edges); a block per row takes its keys' time one after the other, half as long again where two share an SM, until the
+    rows are so many that all their keys count.  Measured, tiles / blocks: 32 heads over 8 of 128, 2 tokens after 2000
+    314 / 242 us, 8 314 / 365, 8 after 500 83 / 94, 8 after 100 26 / 22, 64 sequences of 5 tokens 57 / 38, of 2 after 100 98 /
+    260; 16 over 4 of 64, 8 tokens after 500 49 / 47, 16 after 500 56 / 60; 8 heads of 32, 2 tokens after 500 32 / 41, 32
+    after 100 15.0 / 14.4; 4 heads over 2 of 16 with a window of 200, 64 after 500 20 / 15."""
+    w = window or 1 << 60
+    seen = lambda n: n * (n + 1) // 2 if n <= w else w * (w + 1) // 2 + (n - w) * w     # keys that the first n tokens see
+    per = 64 * nkv // nh
+    counts = [n - p for p, n in zip(past_lens, new_lens)]
+    T, rows, longest = sum(counts), sum(counts) * nh, max(new_lens)
+    pairs = sum(seen(n) - seen(p) for p, n in zip(past_lens, new_lens))
+    rounds = sum(-(-c // per) for c in counts) * nkv / sms
+    pages = -(-longest // PAGE)
+    if longest > w:
+        pages = min(pages, (w + min(per, max(counts)) - 2) // PAGE + 2)
+    tiles = (3.0 + hd / 64) * (max(1.0, rounds) if hd == 128 else 1.0) + \
+        PAGE_US[hd] * max(pages, rounds * max(1.0, pairs / T / PAGE + 0.5)) + (0.7 * min(pages, 5) if longest > w else 0.0)
+    shared = 1.0 if rows <= sms else 1.5 if hd == 128 else 1.15
+    blocks = 3.0 + max(CHAIN_US[hd] * min(longest, w) * shared, KEY_US[hd] * pairs * nh, ROW_US[hd] * rows)
+    return tiles, blocks
 
 
 class AttentionF32:
@@ -58,12 +88,32 @@ class AttentionF32:
         lib.tl_attn_f32.argtypes = [P] * 8 + [I] * 7 + [c_float, I, P, I, I, P]
         self.lib = lib        # last: another thread calls as soon as it is there
 
+    def _sm_count(self, device) -> int:
+        key = device.index if device.index is not None else torch.cuda.current_device()
+        if key not in self._sms:
+            self._sms[key] = torch.cuda.get_device_properties(device).multi_processor_count
+        return self._sms[key]
+
+    def _tiles(self, batch, rows: int, nh: int, nkv: int, hd: int, window, device) -> bool:
+        """Whether a prompt step runs in tiles (worked out once per step)."""
+        longest = getattr(batch, "max_len", None) or batch.len_bucket
+        keys = min(longest, window + batch.max_new) if window else longest
+        if rows * keys < PROMPT_FROM or nh // nkv > MAX_GROUP_PROMPT:
+            return False
+        if getattr(batch, "past_lens", None) is None:
+            return True
+        key = ("attn_f32", nh, nkv, hd, window)
+        known = batch.plans.get(key)
+        if known is None:
+            tiles, blocks = prompt_times(batch.past_lens, batch.new_lens, nh, nkv, hd, window, self._sm_count(device))
+            known = batch.plans[key] = tiles < blocks
+        return known
+
     def run(self, q: torch.Tensor, cache_view, out: torch.Tensor, batch, nh: int, nkv: int, window, scale: float,
             workspace) -> bool:
+        hd = q.shape[1] // nh
         if not batch.is_decode:
-            longest = getattr(batch, "max_len", None) or batch.len_bucket
-            keys = min(longest, window + batch.max_new) if window else longest
-            if q.shape[0] * nh * keys < PROMPT_FROM or nh // nkv > MAX_GROUP_PROMPT:
+            if not self._tiles(batch, q.shape[0] * nh, nh, nkv, hd, window, q.device):
                 return False
         elif nh // nkv > MAX_GROUP_DECODE:
             return False
@@ -75,14 +125,10 @@ class AttentionF32:
         _need(c.page_table, torch.int32, "page table")
         if self.lib is None:
             self._load()
-        hd = q.shape[1] // nh
         per, splits, part = 1, 1, None
         if batch.is_decode:
-            key = q.device.index if q.device.index is not None else torch.cuda.current_device()
-            if key not in self._sms:
-                self._sms[key] = torch.cuda.get_device_properties(q.device).multi_processor_count
             total = getattr(batch, "total_bucket", None) or batch.n_seqs * batch.len_bucket
-            per, splits = decode_split(batch.n_seqs, nkv, batch.len_bucket, total, window, self._sms[key])
+            per, splits = decode_split(batch.n_seqs, nkv, batch.len_bucket, total, window, self._sm_count(q.device))
             if splits > 1:
                 part = workspace.get("attn_f32_part", (batch.n_seqs * nh * splits * (hd + 2),), torch.float32)
         st = self.lib.tl_attn_f32(
