@@ -793,3 +793,49 @@ def test_experts_input_rows_take_no_buffer_of_their_own():
     from torchless_rs_b200.csrc.ops import KernelError
     with pytest.raises(KernelError):
         o.moe_gemm(a, row_token, w, c, off, up=True, act=0, room=rnd(T * K - 1), most=T)
+
+
+@pytest.mark.parametrize("act", [0, 2])
+@pytest.mark.parametrize("N,K,counts", [
+    (2990, 1032, [257, 0, 700, 513, 40]), (1500, 2048, [0, 600, 0, 0, 300, 1, 17]), (48, 64, [900, 0, 333]), (64, 128, [2000, 1, 0, 31]),
+    (40, 104, [(7 * e) % 23 * ((e % 3) > 0) for e in range(300)]), (129, 72, [1]), (130, 1024, [16, 33, 256, 255])])
+def test_experts_products_on_tensor_cores_alone(N, K, counts, act):
+    """Experts cut into several row tiles, tiles without rows, empty experts between full ones, more tiles than two rounds of
+    blocks take, a ring of stages that wraps, rows and columns that end inside a tile, few experts of small matrices and many;
+    against 64 bits.  Bound of a sum: the tensor core cuts what falls off at each of K / 16 additions, 2^-23 of the sum of
+    the sizes each, and up to 16 products inside one; after the activation also the rounding to bfloat16."""
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.moe_bf16 import MoeBf16
+    o, E, R = _ops(torch.bfloat16), len(counts), sum(counts)
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)
+    T = R // 2 + 3
+    x = rnd(T, K).to(torch.bfloat16)
+    row_token = _i32(np.random.default_rng(K).integers(0, T, R))
+    off = _i32(np.concatenate([[0], np.cumsum(counts)]))
+    w_up, w_down = (rnd(E, n, K).mul_(K ** -0.5).to(torch.bfloat16) for n in (2 * N, N))
+    up = torch.full((R, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    down = torch.full((R, N), float("nan"), device="cuda")
+    before = ops.launch_counts()
+    o.moe_gemm(x, row_token, w_up, up, off, up=True, act=act, limit=2.0, alpha=1.3, most=max(counts))
+    grouped = x[row_token.long()].contiguous()
+    o.moe_gemm(grouped, None, w_down, down, off, up=False, most=max(counts))
+    assert ops.counts_since(before).get("moe_gemm_tc") == 2 and MoeBf16.get().take_error() == 0
+    at = 0
+    for e, n in enumerate(counts):
+        if n == 0:
+            continue
+        h, rows = grouped[at:at + n].double(), slice(at, at + n)
+        at += n
+        cut = (K / 16 + 16) * 2.0 ** -23
+        wu, wd = w_up[e].double(), w_down[e].double()
+        assert ((down[rows].double() - h @ wd.T).abs() <= cut * (h.abs() @ wd.abs().T)).all(), e
+        gate, lin = h @ wu[:N].T, h @ wu[N:].T
+        off_by = cut * (h.abs() @ wu.abs().T)
+        off_by = off_by[:, :N] + off_by[:, N:]
+        if act == 0:
+            want = gate * torch.sigmoid(gate) * lin
+        else:
+            gate, lin = gate.clamp(max=2.0), lin.clamp(-2.0, 2.0)
+            want = gate * torch.sigmoid(1.3 * gate) * (lin + 1)
+        assert ((up[rows].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2 * (gate.abs() + lin.abs() + 2) * off_by).all(), e

@@ -12,9 +12,11 @@
 // double-buffered in tensor memory.
 //
 // Bound by the tensor cores on prompts and by the experts' weights on decode steps.  On mma.sync, 64 x 64 tiles (which this
-// replaces), 2900 tokens of four choices among 16 experts of 1408 at width 2048 took 514 us up and 309 us down; here 161 and 77
-// us (84 and 42 at the bfloat16 rate).  Four tokens: 56 and 32 us; here 29 and 15 (19 and 10 at the copy rate of the experts
-// that are chosen).  Width 4096, experts of 3584, 16 tokens: 263 and 151 us; here 146 and 75 (143 and 72).
+// replaces), 3000 tokens of four choices among 16 experts of 1408 at width 2048 took 529 us up and 316 us down; here 157 and 78
+// us (87 and 43 at the bfloat16 rate).  Four tokens: 59 and 32 us; here 24 and 13 (19 and 10 at the copy rate of the experts
+// that are chosen).  Width 4096, experts of 3584, 16 tokens: 262 and 150 us; here 147 and 76 (143 and 72).  256 experts of 256 at
+// width 1024, one token of eight choices: 38 and 62 us; here 10 and 6.  Only where a few experts of some fifty at widths of some
+// fifty get thousands of rows was that faster (four of 48 at 64, 3000 tokens of two choices: 6.8 and 3.7 us; here 9.0 and 6.8).
 //
 // Every wait on an mbarrier is bounded; when a bound is hit the kernel records a code in tl_moe_tc_error, stops waiting
 // everywhere, frees its tensor memory and returns.
@@ -52,16 +54,16 @@ __device__ __forceinline__ void mt_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// rows[r] = X[row_token[r]] for the grouped rows r < offsets[E]; 16 bytes per thread.
+// rows[r] = X[row_token[r]] for the grouped rows r < offsets[E]; 16 bytes per thread, 1 << row_log threads per row.
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const uint4* __restrict__ X, int ldx16, const int* __restrict__ row_token, const int* __restrict__ offsets,
-                  int E, int per_row, uint4* __restrict__ rows) {
+                  int E, int per_row, int row_log, uint4* __restrict__ rows) {
   pdl_wait();
   pdl_launch_dependents();
-  const int n = offsets[E];
-  for (int r = blockIdx.x; r < n; r += gridDim.x) {
+  const int n = offsets[E], threads = 1 << row_log, per_block = 256 >> row_log;
+  for (int r = blockIdx.x * per_block + (threadIdx.x >> row_log); r < n; r += gridDim.x * per_block) {
     const uint4* src = X + (size_t)row_token[r] * ldx16;
-    for (int i = threadIdx.x; i < per_row; i += 256) rows[(size_t)r * per_row + i] = src[i];
+    for (int i = threadIdx.x & (threads - 1); i < per_row; i += threads) rows[(size_t)r * per_row + i] = src[i];
   }
 }
 
@@ -81,28 +83,36 @@ __device__ __forceinline__ float mt_act(const MoeArgs& a, float g, float u) {
 }
 
 // The tiles of a block, in order: expert by expert, inside an expert all row tiles of one strip of W, then the next
-// strip.
+// strip.  `first[e]`: the number of expert e's first tile, for e <= E.  (Walking from expert to expert with a division each
+// took 40 us of 48 with 300 experts.)
 struct MoeWalk {
   const int* off;
-  int E, cap, n_tiles;
-  int e = 0, first = 0;            // expert, and the number of its first tile
+  const int* first;
+  int E, cap;
+  int e = 0;                       // expert
   int r0 = 0, rows = 0, bn = 0, strip = 0;
   __device__ bool find(int tile) {
-    for (; e < E; ++e) {
-      const int n = off[e + 1] - off[e];
-      const int m_tiles = (n + cap - 1) / cap;
-      const int here = m_tiles * n_tiles;
-      if (tile < first + here) {
-        const int t = tile - first, m = t % m_tiles;
-        bn = ((n + m_tiles - 1) / m_tiles + 15) / 16 * 16;
-        strip = t / m_tiles;
-        r0 = off[e] + m * bn;
-        rows = min(bn, off[e + 1] - r0);      // (0 or less: the tiles before took all rows)
-        return true;
-      }
-      first += here;
+    if (tile >= first[E]) return false;
+    int hi = E;                    // the last expert whose first tile is not beyond; tiles rise, so it is not before e
+    while (hi - e > 1) {
+      const int mid = (e + hi) >> 1;
+      if (first[mid] <= tile) e = mid;
+      else hi = mid;
     }
-    return false;
+    const int n = off[e + 1] - off[e], t = tile - first[e];
+    int m_tiles = 1, m = 0;
+    strip = t;
+    bn = n;
+    if (n > cap) {
+      m_tiles = (n + cap - 1) / cap;
+      m = t % m_tiles;
+      strip = t / m_tiles;
+      bn = (n + m_tiles - 1) / m_tiles;
+    }
+    bn = (bn + 15) / 16 * 16;
+    r0 = off[e] + m * bn;
+    rows = min(bn, off[e + 1] - r0);      // (0 or less: the tiles before took all rows)
+    return true;
   }
 };
 
@@ -121,6 +131,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* off = (int*)((uint8_t*)full + MT_TAIL);  // [E + 1]
+  int* first = off + args.E + 1;                // [E + 1]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int TILE_N = UP ? 64 : 128;         // columns of C per tile
@@ -137,12 +148,28 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ 
   if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   pdl_wait();
   for (int i = threadIdx.x; i <= args.E; i += MT_THREADS) off[i] = args.offsets[i];
+  __syncthreads();
+  if (warp == 1) {
+    int before = 0;
+    for (int e0 = 0; e0 < args.E; e0 += 32) {
+      const int e = e0 + lane;
+      int v = e < args.E ? (off[e + 1] - off[e] + args.bn_cap - 1) / args.bn_cap * n_tiles : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (e < args.E) first[e + 1] = before + v;
+      before += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) first[0] = 0;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   if (threadIdx.x == 0) pdl_launch_dependents();
-  MoeWalk walk{off, args.E, args.bn_cap, n_tiles};
+  MoeWalk walk{off, first, args.E, args.bn_cap};
 
   if (warp == 4 && elect_one()) {
     // ---- TMA
@@ -309,21 +336,30 @@ extern "C" int tl_moe_tc(const void* X, int ldx, const int* row_token, void* gro
     return -2;
   if ((long long)E * N * (up ? 2 : 1) > 0x7fffffffll) return -2;
   MoeArgs a = {C, offsets, ldc, E, N, K, 0, 0, kind, limit, alpha};
+  const int tile_n = up ? 64 : 128, n_tiles = (N + tile_n - 1) / tile_n;
   a.bn_cap = most >= MT_BN ? MT_BN : (most + MT_BOX - 1) / MT_BOX * MT_BOX;
-  const int stage = MT_W + a.bn_cap * 128, fixed = 1024 + MT_XCHG + MT_TAIL + (E + 1) * 4;
+  if ((long long)E * n_tiles < num_sms) {
+    // few experts with small matrices: tiles of as few rows as give every SM one (6000 rows, four experts of 48 at width 64: 9.0
+    // us up and 6.8 down; with tiles of 256 rows 22.7 and 13.4)
+    const long long share = ((long long)max_rows * n_tiles + num_sms - 1) / num_sms;
+    if (share < a.bn_cap) a.bn_cap = (int)((share + MT_BOX - 1) / MT_BOX * MT_BOX);
+  }
+  const int stage = MT_W + a.bn_cap * 128, fixed = 1024 + MT_XCHG + MT_TAIL + 2 * (E + 1) * 4;
   a.stages = (227 * 1024 - fixed) / stage;
   if (a.stages > MT_MAX_STAGES) a.stages = MT_MAX_STAGES;
   CUtensorMap tw, tx;
   if (!mt_map(&tw, W, (long long)E * N * (up ? 2 : 1), K, K, 64)) return -2;
   if (!mt_map(&tx, up ? grouped : X, max_rows, K, up ? K : ldx, MT_BOX)) return -2;
   if (up) {
-    const int rc = tl_launch(moe_gather_kernel, dim3(max_rows < 4096 ? max_rows : 4096), dim3(256), 0, stream, (const uint4*)X,
-                             ldx / 8, row_token, offsets, E, K / 8, (uint4*)grouped);
+    int row_log = 0;
+    while (row_log < 8 && (1 << row_log) < K / 8) ++row_log;
+    const int want = (max_rows + (256 >> row_log) - 1) / (256 >> row_log);
+    const int rc = tl_launch(moe_gather_kernel, dim3(want < 4096 ? want : 4096), dim3(256), 0, stream, (const uint4*)X,
+                             ldx / 8, row_token, offsets, E, K / 8, row_log, (uint4*)grouped);
     if (rc != 0) return rc;
   }
   // no more blocks than there can be tiles
-  const int tile_n = up ? 64 : 128;
-  const long long tiles = ((long long)max_rows / 16 + E) * ((N + tile_n - 1) / tile_n);
+  const long long tiles = ((long long)max_rows / 16 + E) * n_tiles;
   const int blocks = tiles < num_sms ? (int)tiles : num_sms, smem = fixed + a.stages * stage;
   return up ? run_moe<true>(tw, tx, a, smem, blocks, stream) : run_moe<false>(tw, tx, a, smem, blocks, stream);
 }
