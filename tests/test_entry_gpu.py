@@ -242,3 +242,15 @@ def test_a_cluster_of_blocks_samples_what_one_block_samples(rows, V):
                 s.sample(y, t, k, p, u, a)
                 s.sample(y, t, k, p, u, b, walk=True)
                 assert a.tolist() == b.tolist(), (V, pad, t, k, p)
+
+
+@pytest.mark.parametrize("rows,V,k,p,blocks", [
+    (8, 131072, 0, 0.95, 8), (300, 200000, 0, 0.95, 8), (64, 131072, 50, 0.0, 4), (148, 131072, 50, 0.0, 0), (148, 131072, 50, 0.9, 4),
+    (148, 200000, 0, 0.0, 0), (148, 200000, 50, 0.0, 0), (148, 200000, 50, 0.9, 0), (64, 200000, 0, 0.0, 8), (75, 200000, 50, 0.9, 8),
+    (600, 40000, 50, 0.0, 0), (64, 32000, 50, 0.0, 2), (300, 32000, 50, 0.9, 1), (1000, 5000, 0, 0.0, 1), (1, 262145, 0, 0.95, 0),
+    (148, 32000, 200000, 0.0, 1)])
+def test_rows_are_sampled_by_clusters_where_they_were_faster(rows, V, k, p, blocks):
+    """The rule between clusters of blocks and one block per row, at sizes where both were timed (0: one block per row)."""
+    import ctypes
+    from torchless_rs_b200.csrc import ops
+    assert ops.sampling_ops().lib.tl_sample_route(rows, V, k, ctypes.c_float(p)) == blocks

@@ -769,29 +769,63 @@ extern "C" int tl_sample_walk(const float* logits, int ld, int rows, int V, floa
                    temperature, top_k, top_p, uniform, out);
 }
 
-// temperature must be > 0; rows with temperature <= 0 go through tl_argmax.
+// Whether walking the rows with one block each is faster than clusters of `blocks` blocks, `per` entries per thread.  What more
+// clusters than run at once cost, they cost in rounds, while a row's walk takes its SM as long whatever the others do;
+// top-p alone, whose walk takes many passes, always gains, and so do 16 entries per thread and fewer.  us (temperature alone /
+// top-k / both): a round of clusters 17 / 55 / 84; a walk 5 + 0.00058 V / 22 + 0.00138 V / 78 + 0.00254 V, some more per row beyond
+// 148 rows and beyond what the L2 cache holds.  Measured, clusters / walk: 148 rows of 200,000 entries 185 / 153, 609 / 382 and
+// 928 / 740 us, 100 rows 130 / 125, 423 / 295, 643 / 586, 64 rows 92 / 122, 294 / 294, 452 / 591; 148 rows of 131,072 77 / 86, 268 /
+// 206, 410 / 416; 300 of 32,000 53 / 49, 135 / 160, 222 / 399; 1000 of 5000 45 / 54, 116 / 213, 203 / 615.
+static bool sample_walks(int rows, int V, int blocks, int per, bool use_k, bool use_p) {
+  if ((use_p && !use_k) || per <= 16) return false;
+  const int kind = use_p ? 2 : use_k ? 1 : 0;
+  static const double round[3] = {17, 55, 84}, fixed[3] = {5, 22, 78}, entry[3] = {0.58e-3, 1.38e-3, 2.54e-3};
+  const int at_once = blocks == 1 ? 148 : blocks == 2 ? 74 : blocks == 4 ? 33 : 15;
+  double clusters = blocks == 1 && kind == 1 ? 50.0 : round[kind];
+  clusters *= (rows + at_once - 1) / at_once * (blocks == 8 ? 1.08 : blocks == 4 ? 0.96 : 1.0);
+  double walk = fixed[kind] + entry[kind] * V;
+  if (rows > 148) walk *= kind == 0 ? 0.35 + 0.9 * rows / 148 : 0.47 + 0.95 * rows / 148;
+  if ((double)rows * V > 2.2e7) walk *= 1.2;
+  return walk < clusters;
+}
+
 #define SAMPLE_MAX_CLUSTER 8   // portable cluster size
+// The blocks per row and the entries per thread, or false if the rows are walked.
+// As many blocks per row as give a thread four entries, at most 8 and no more than run at once (a block fills an
+// SM), but enough that 32 entries per thread cover the row: a pass costs what a thread holds, a barrier of eight
+// blocks little more than one of two, and a second round of blocks as much as the first.
+static bool sample_plan(int rows, int V, int top_k, float top_p, int* blocks, int* per) {
+  int n = 1;
+  while (n < SAMPLE_MAX_CLUSTER && n * SAMPLE_THREADS * 4 < V &&
+         (n * SAMPLE_THREADS * 32 < V || (long long)rows * n * 2 <= 148))
+    n *= 2;
+  *blocks = n;
+  *per = (V + n * SAMPLE_THREADS - 1) / (n * SAMPLE_THREADS);
+  return *per <= 32 && !sample_walks(rows, V, n, *per, top_k > 0 && top_k < V, top_p > 0.0f && top_p < 1.0f);
+}
+
+// temperature must be > 0; rows with temperature <= 0 go through tl_argmax.
 extern "C" int tl_sample(const float* logits, int ld, int rows, int V, float temperature,
                          int top_k, float top_p, const float* uniform, int* out,
                          cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (V <= 0 || !(temperature > 0.0f)) return -1;
-  // As many blocks per row as give a thread four entries, at most 8 and no more than run at once (a block fills an
-  // SM), but enough that 32 entries per thread cover the row: a pass costs what a thread holds, a barrier of eight
-  // blocks little more than one of two, and a second round of blocks as much as the first.
-  int blocks = 1;
-  while (blocks < SAMPLE_MAX_CLUSTER && blocks * SAMPLE_THREADS * 4 < V &&
-         (blocks * SAMPLE_THREADS * 32 < V || (long long)rows * blocks * 2 <= 148))
-    blocks *= 2;
-  const int per = (V + blocks * SAMPLE_THREADS - 1) / (blocks * SAMPLE_THREADS);
+  int blocks, per;
+  if (!sample_plan(rows, V, top_k, top_p, &blocks, &per))
+    return tl_sample_walk(logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream);
 #define SAMPLE_CLUSTER(EPT_) \
   return launch_sample_cluster<EPT_>(blocks, logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream)
   if (per <= 4) SAMPLE_CLUSTER(4);
   if (per <= 8) SAMPLE_CLUSTER(8);
   if (per <= 16) SAMPLE_CLUSTER(16);
-  if (per <= 32) SAMPLE_CLUSTER(32);
+  SAMPLE_CLUSTER(32);
 #undef SAMPLE_CLUSTER
-  return tl_sample_walk(logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream);
+}
+
+// Blocks per row, or 0 if the rows are walked (for the test of the rule).
+extern "C" int tl_sample_route(int rows, int V, int top_k, float top_p) {
+  int blocks, per;
+  return sample_plan(rows, V, top_k, top_p, &blocks, &per) ? blocks : 0;
 }
 
 TL_TRACE_EXPORT(sampling)
