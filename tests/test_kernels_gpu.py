@@ -99,7 +99,8 @@ def test_gemm_generic(dtype, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(4, 1024, 1024), (8, 200, 5120), (16, 1100, 1024), (96, 1027, 1056), (97, 1027, 1056), (17, 1027, 1500), (64, 640, 2052), (65, 640, 2048),
-                                   (192, 1028, 1024), (193, 700, 1600), (531, 320, 4096), (300, 96, 14336)])
+                                   (192, 1028, 1024), (193, 700, 1600), (531, 320, 4096), (300, 96, 14336),
+                                   (531, 6144, 1024), (192, 20000, 1056), (4, 14336, 1024)])
 def test_gemm_split_is_no_further_off_than_the_cuda_core_kernel(M, N, K):
     """32-bit products on tensor cores, at the edges of tiles (64 and 128 rows of weights, 16 to 192 tokens), of K
     (stages of 32, several splits) and with strided rows.  Bound, per output: a sum of 16 leading products is cut 16 times,
@@ -108,7 +109,6 @@ def test_gemm_split_is_no_further_off_than_the_cuda_core_kernel(M, N, K):
     from torchless_rs_b200.csrc.gemm_f32 import GemmF32
     from torchless_rs_b200.parts.runtime import Workspace
     g, o, ws = GemmF32.get(), _ops(torch.float32), Workspace(torch.device(DEV))
-    assert GemmF32.takes(M, N, K) or N * K < 20 << 20
     g_takes, GemmF32.takes = GemmF32.takes, staticmethod(lambda *a: True)
     try:
         for pad in (0, 3):       # rows of X and C that do not start on 16 bytes
@@ -138,6 +138,41 @@ def test_gemm_split_is_no_further_off_than_the_cuda_core_kernel(M, N, K):
         assert g.take_error() == 0
     finally:
         GemmF32.takes = staticmethod(g_takes)
+
+
+def test_gemm_split_tests_reach_every_way_of_cutting_a_product():
+    """What the shapes of the test above are for: tiles of up to 192 tokens, one block per tile in one round and in several, K
+    over clusters, narrow tiles (two sums in tensor memory) and wide ones; in both forms of the kernel."""
+    import ctypes
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    g = GemmF32.get()
+    if g.lib is None:
+        g._load()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    def plan(M, N, K, mode):
+        v = [ctypes.c_int() for _ in range(3)]
+        g.lib.tl_gemm_split_plan(M, N, K, mode, sms, *(ctypes.byref(x) for x in v))
+        return tuple(x.value for x in v)      # tokens per tile, splits of K, tiles
+    for mode in (ops.MODE_STORE_F32, ops.MODE_SWIGLU):
+        bn, splits, tiles = plan(531, 6144, 1024, mode)
+        assert bn > 96 and splits == 1
+        bn, splits, tiles = plan(192, 20000, 1056, mode)
+        assert splits == 1 and tiles > sms
+        bn, splits, tiles = plan(16, 1100, 1024, mode)
+        assert bn == 16 and splits > 1
+    assert plan(531, 6144, 1024, ops.MODE_STORE_F32)[0] == 192
+    assert plan(4, 14336, 1024, ops.MODE_SWIGLU)[1:] == (1, 224) and plan(300, 96, 14336, ops.MODE_STORE_F32)[1] == 8
+
+
+def test_gemm_split_takes_the_products_it_is_faster_at():
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    takes = GemmF32.takes
+    million = 1 << 20
+    assert takes(9, 1024, 1024) and not takes(9, 1023, 1024) and not takes(9, 1 << 20, 1023) and takes(1000, 1024, 1024)
+    assert takes(8, 6 * million // 1024, 1024) and not takes(8, 6 * million // 1024 - 1, 1024) and takes(5, 6144, 1024)
+    assert takes(4, 20 * million // 1024, 1024) and not takes(4, 20 * million // 1024 - 1, 1024)
+    assert not takes(3, 14336, 4096) and not takes(1, 1 << 20, 4096)
 
 
 def test_gemm_split_gives_what_the_cuda_core_kernel_gives_where_results_are_not_finite():

@@ -580,23 +580,12 @@ static int run_split(const CUtensorMap& tw, const CUtensorMap& tx, const SplitAr
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// Bytes of scratch that tl_gemm_split needs for X's pieces.
-extern "C" long long tl_gemm_split_scratch(int M, int K) { return 6ll * M * ((K + 7) / 8 * 8); }
-
-// Returns 0, a CUDA error, or -2 when these sizes or alignments are not taken (the caller then uses the CUDA-core
-// kernel).  N counts output columns; in mode 2 W has 2N rows.  `scratch`: tl_gemm_split_scratch bytes, on 16 bytes.
-extern "C" int tl_gemm_split(const float* X, int ldx, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
-                             int mode, int num_sms, void* scratch, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return 0;
-  if (mode < 0 || mode > 3) return -1;
-  if (K <= 0 || K % 4 || ldw % 4 || ((uintptr_t)W & 15) || ((uintptr_t)scratch & 15)) return -2;
-  const bool swiglu = mode == MODE_SWIGLU;
-  const int n_tiles = (N + (swiglu ? 64 : 128) - 1) / (swiglu ? 64 : 128);
-  const int Kp = (K + 7) / 8 * 8, k_all = (K + SP_K - 1) / SP_K;
-  SplitArgs a = {X, W, C, ldx, ldw, ldc, M, N, K, mode, 0, 0, 1, k_all};
-  // Tokens per tile and splits of K: the choice that takes the fewest cycles.  A stage takes SP_COST_TOKEN per token
-  // for its instructions and SP_COST_STAGE for splitting W at the least; a round of blocks SP_COST_ROUND besides, and
-  // the reduction over a cluster SP_COST_REDUCE per token of the tile.
+// Tokens per tile and splits of K into `a`: the choice that takes the fewest cycles.  A stage takes SP_COST_TOKEN per token
+// for its instructions and SP_COST_STAGE for splitting W at the least; a round of blocks SP_COST_ROUND besides, and
+// the reduction over a cluster SP_COST_REDUCE per token of the tile.  Returns the tiles along N.
+static int sp_plan(SplitArgs& a, int num_sms) {
+  const bool swiglu = a.mode == MODE_SWIGLU;
+  const int n_tiles = (a.N + (swiglu ? 64 : 128) - 1) / (swiglu ? 64 : 128), k_all = (a.K + SP_K - 1) / SP_K, M = a.M;
   double best = -1.0;
   for (int mt = (M + SP_BN - 1) / SP_BN, tries = 0; tries < 8 && mt <= M; ++mt, ++tries) {
     const int bn = ((M + mt - 1) / mt + 15) / 16 * 16;
@@ -613,6 +602,31 @@ extern "C" int tl_gemm_split(const float* X, int ldx, const float* W, int ldw, f
     }
   }
   a.m_tiles = (M + a.bn - 1) / a.bn;
+  return n_tiles;
+}
+
+// Tokens per tile, splits of K and tiles of a product, for the tests.
+extern "C" void tl_gemm_split_plan(int M, int N, int K, int mode, int num_sms, int* bn, int* splits, int* tiles) {
+  SplitArgs a = {nullptr, nullptr, nullptr, 0, 0, 0, M, N, K, mode, 0, 0, 1, 0};
+  *tiles = sp_plan(a, num_sms) * a.m_tiles;
+  *bn = a.bn;
+  *splits = a.splits;
+}
+
+// Bytes of scratch that tl_gemm_split needs for X's pieces.
+extern "C" long long tl_gemm_split_scratch(int M, int K) { return 6ll * M * ((K + 7) / 8 * 8); }
+
+// Returns 0, a CUDA error, or -2 when these sizes or alignments are not taken (the caller then uses the CUDA-core
+// kernel).  N counts output columns; in mode 2 W has 2N rows.  `scratch`: tl_gemm_split_scratch bytes, on 16 bytes.
+extern "C" int tl_gemm_split(const float* X, int ldx, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
+                             int mode, int num_sms, void* scratch, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (mode < 0 || mode > 3) return -1;
+  if (K <= 0 || K % 4 || ldw % 4 || ((uintptr_t)W & 15) || ((uintptr_t)scratch & 15)) return -2;
+  const bool swiglu = mode == MODE_SWIGLU;
+  const int Kp = (K + 7) / 8 * 8;
+  SplitArgs a = {X, W, C, ldx, ldw, ldc, M, N, K, mode, 0, 0, 1, 0};
+  const int n_tiles = sp_plan(a, num_sms);
   const long long tiles = (long long)n_tiles * a.m_tiles;
   if (tiles * a.splits > 0x7fffffffll) return -2;
   SpEncodeFn fn = sp_encode();
