@@ -100,7 +100,7 @@ class AttentionF32:
         keys = min(longest, window + batch.max_new) if window else longest
         if rows * keys < PROMPT_FROM or nh // nkv > MAX_GROUP_PROMPT:
             return False
-        if getattr(batch, "past_lens", None) is None:
+        if getattr(batch, "plans", None) is None:      # not a step of the engine's
             return True
         key = ("attn_f32", nh, nkv, hd, window)
         known = batch.plans.get(key)

@@ -66,7 +66,7 @@ class LatentBf16:
         """Whether a step runs here (worked out once per step)."""
         if batch.max_new * heads < self.FROM_ROWS or heads > 128:
             return False
-        if getattr(batch, "past_lens", None) is None:
+        if getattr(batch, "plans", None) is None:      # not a step of the engine's
             return True
         key = ("latent", heads, window)
         known = batch.plans.get(key)
