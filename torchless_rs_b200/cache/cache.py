@@ -132,8 +132,8 @@ class PagedGroup:
 
     def truncate(self, slot: int, new_len: int) -> None:
         """Gives back the whole pages beyond `new_len` positions.  What lies beyond `new_len`
-        in the last kept page stays there; no kernel reads past a sequence's length, and the
-        next tokens overwrite it."""
+        in the last kept page stays there; kernels that read whole pages give it no weight, and
+        the next tokens overwrite it."""
         keep = pages_for(new_len)
         f, c = self.first_live[slot], self.n_cols[slot]
         if keep >= c:

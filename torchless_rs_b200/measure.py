@@ -26,6 +26,13 @@ import math
 import torch
 
 
+def _step_of(seqs: int, per: int, past: int, start: torch.Tensor):
+    """What the kernels that choose by a step's lengths ask of it: `seqs` sequences that bring `per` tokens each after `past`."""
+    from types import SimpleNamespace
+    return SimpleNamespace(is_decode=per == 1, n_seqs=seqs, max_new=per, seq_start=start, past_lens=[past] * seqs,
+                           new_lens=[past + per] * seqs, plans={})
+
+
 def _time(fn, iters: int) -> float:
     """Mean microseconds per call.  The calls are recorded into one CUDA graph and the graph
     is replayed, so the host's launch cost (some ten microseconds per call from Python) does
@@ -248,7 +255,7 @@ def kikopel_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None) 
         q = torch.randn((n_tok, H * width), device=dev) * 0.1
         mix = torch.empty((n_tok, H, rank), device=dev)
         us = _time(lambda: o.latent_attn(q, width, q, width, rank, pages, mix, pos, seq, slot, table, inv, H, rank,
-                                         rot, rot, z["window"], 0.04), max(2, iters // 8) if n_tok > 64 else iters)
+                                         rot, rot, z["window"], 0.04, batch=_step_of(seqs, per, past, start)), max(2, iters // 8) if n_tok > 64 else iters)
         cache_b = 2.0 * seqs * min(past + per, z["window"]) * width
         report("latent_attn", case, us, cache_b + n_tok * H * (width + rank) * 4.0, 2.0 * H * seen * (width + rank))
         nkv = max(1, H // 4)
@@ -891,10 +898,12 @@ def fezolorn_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None)
         all_seen = sum(p + 1 for p in range(past, past + per)) * seqs
         lat_b = 2.0 * seqs * (past + per) * width + n_tok * mh * (width + rank) * 4.0
         us = _time(lambda: o.latent_attn(ql, width, ql, width, rank, pages, mix, pos, seq, slot, ltab, inv2, mh, rank,
-                                         rot, rot, None, 0.04, max_keys=past + per, workspace=ws, sink=lsink), few)
+                                         rot, rot, None, 0.04, max_keys=past + per, workspace=ws, sink=lsink,
+                                         batch=_step_of(seqs, per, past, start)), few)
         report("latent_attn (sink, no window)", case, us, lat_b, 2.0 * mh * all_seen * (width + rank))
         us = _time(lambda: o.latent_attn(ql, width, ql, width, rank, pages, mix, pos, seq, slot, ltab, inv2, mh, rank,
-                                         rot, rot, None, 0.04, max_keys=past + per, workspace=ws), few)
+                                         rot, rot, None, 0.04, max_keys=past + per, workspace=ws,
+                                         batch=_step_of(seqs, per, past, start)), few)
         report("  like: latent_attn (second design)", case, us, lat_b, 2.0 * mh * all_seen * (width + rank))
         wuv = torch.randn((mh, mv, rank), device=dev, dtype=bf) * 0.02
         og = torch.empty((n_tok, mh * mv), device=dev, dtype=bf)
@@ -1270,12 +1279,14 @@ def beralix_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None) 
                mh * mv * rank * 2.0 + n_tok * mh * (rank * 4.0 + mv * 6.0), 2.0 * n_tok * mh * mv * rank)
         seen = sum(p + 1 for p in range(past, past + per)) * seqs
         us = _time(lambda: o.latent_attn(qa, rank, s, md + rot, md, pages, mix, pos, seq, slot, ltab, inv2, mh, rank, rot, rot,
-                                         None, 0.04, max_keys=past + per, workspace=ws, amplitude=1.2), few)
+                                         None, 0.04, max_keys=past + per, workspace=ws, amplitude=1.2,
+                                         batch=_step_of(seqs, per, past, start)), few)
         byts = 2.0 * seqs * (past + per) * width + n_tok * mh * (width + rank) * 4.0
         report("latent_attn", case, us, byts, 2.0 * mh * seen * (width + rank))
         ql = torch.randn((n_tok, mh * width), device=dev)
         us = _time(lambda: o.latent_attn(ql, width, ql, width, rank, pages, mix, pos, seq, slot, ltab, inv2, mh, rank, rot,
-                                         rot, None, 0.04, max_keys=past + per, workspace=ws), few)
+                                         rot, None, 0.04, max_keys=past + per, workspace=ws,
+                                         batch=_step_of(seqs, per, past, start)), few)
         report("  like: latent_attn (folded queries)", case, us, byts, 2.0 * mh * seen * (width + rank))
         del ql, mix, s2, gate
         # --- the selective scan, beside the second design's recurrence and the sixth's, each at an equal state
