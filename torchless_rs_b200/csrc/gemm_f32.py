@@ -16,8 +16,8 @@ class GemmF32:
     _inst = None
     LEAST = 1 << 20       # no product with a smaller matrix is taken
     # Most bytes of pieces (6 for each number of the activations) that are held: 65,536 tokens of 14336 columns would be 5.6
-    # GB, half as much again as the step's largest activation.  At the bound a launch has 6208 rows and more of these
-    # columns, 7 rounds of blocks and more over 4096 outputs.
+    # GB, half as much again as the step's largest activation.  At the bound a launch has 6144 rows of these
+    # columns, seven rounds of blocks over 4096 outputs.
     SCRATCH = 1 << 29
     ROWS = 192            # rows of a launch: a multiple of the kernel's largest tile
 
