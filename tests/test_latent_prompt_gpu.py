@@ -1,0 +1,188 @@
+"""Latent attention of steps whose sequences start with them: keys and values formed per head (latent_prompt_tc.cu)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DIM = 128
+BF, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def _step(lens):
+    return SimpleNamespace(is_decode=False, n_seqs=len(lens), max_new=max(lens), past_lens=[0] * len(lens), new_lens=list(lens),
+                           seq_start=_i32([sum(lens[:b]) for b in range(len(lens) + 1)]))
+
+
+def _inputs(lens, heads, rot, dims, seed, size=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T, rank = sum(lens), 72
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)
+    ang = rnd(T, max(dims // 2, 1)) * 3
+    turn = torch.stack([ang.cos() * 1.1, ang.sin() * 1.1], -1).contiguous() if dims else None
+    return dict(q=rnd(T, heads * (DIM + rot) + 8) * size, turn=turn, kv=rnd(T, heads * 2 * DIM).to(BF), latents=rnd(T, rank + rot).to(BF),
+                gate=rnd(T, heads * DIM + 4) * 2, sink=rnd(heads)), rank
+
+
+def _run(x, rank, lens, heads, rot, dims, window, gate, sink, scale):
+    from torchless_rs_b200.csrc.latent_bf16 import LatentPrompt
+    T = sum(lens)
+    gates = {None: None, "entry": x["gate"][:, 4:], "head": x["gate"][:, :heads]}[gate]
+    out = torch.full((T, heads * DIM), float("nan"), device="cuda", dtype=BF)
+    assert LatentPrompt.get().run(x["q"], x["turn"], x["kv"], x["latents"], out, gates, x["sink"] if sink else None, _step(lens), heads,
+                                  rank, rot, dims, window, scale)
+    assert LatentPrompt.get().take_error() == 0
+    return out.view(T, heads, DIM), gates
+
+
+def _reference(x, rank, lens, heads, rot, dims, window, gates, sink, scale):
+    """(result in 64 bits, the weighted sum of the values' magnitudes), the queries rounded where the kernel rounds them."""
+    f = torch.tensor(scale * 1.4426950408889634, dtype=F32, device="cuda")
+    out, size, at = [], [], 0
+    for n in lens:
+        q = x["q"][at:at + n, :heads * (DIM + rot)].view(n, heads, DIM + rot).clone()
+        if dims:
+            p, (c, s) = dims // 2, x["turn"][at:at + n].unbind(-1)
+            u, w = q[..., DIM:DIM + p].clone(), q[..., DIM + p:DIM + dims].clone()
+            c, s = c[:, None], s[:, None]
+            q[..., DIM:DIM + p], q[..., DIM + p:DIM + dims] = u * c - w * s, w * c + u * s
+        q = (q * f).to(BF).to(F64)
+        kv = x["kv"][at:at + n].to(F64).view(n, 2, heads, DIM)
+        r = x["latents"][at:at + n, rank:].to(F64)
+        i = torch.arange(n, device="cuda")
+        hidden = (i[:, None] < i) | ((i[:, None] - i >= window) if window else (i[:, None] < i))
+        for h in range(heads):
+            sc = q[:, h, :DIM] @ kv[:, 0, h].T + q[:, h, DIM:] @ r.T
+            sc.masked_fill_(hidden, -float("inf"))
+            m = sc.max(-1, keepdim=True).values
+            e = torch.exp2(sc - m)
+            l = e.sum(-1, keepdim=True) + (torch.exp2(x["sink"][h].double() * 1.4426950408889634 - m) if sink else 0.0)
+            out.append((e / l) @ kv[:, 1, h])
+            size.append((e / l) @ kv[:, 1, h].abs())
+        at += n
+    def whole(parts):
+        rows, k = [], 0
+        for n in lens:
+            rows.append(torch.stack(parts[k:k + heads], 1))
+            k += heads
+        return torch.cat(rows)
+    y, a = whole(out), whole(size)
+    if gates is not None:
+        g = torch.sigmoid(gates.double())
+        g = g[:, :, None] if gates.shape[1] == heads else g.reshape(-1, heads, DIM)
+        y, a = y * g, a * g
+    return y, a
+
+
+@pytest.mark.parametrize("lens,heads,rot,dims,window,gate,sink", [
+    ([17], 2, 64, 64, None, "entry", False), ([128], 1, 64, 32, None, None, True), ([129, 1, 64], 3, 64, 64, None, "head", False),
+    ([300, 65, 63], 2, 32, 32, 100, "entry", True), ([513], 2, 0, 0, 64, None, False), ([1, 2, 700], 1, 16, 6, 1, "head", True),
+    ([400, 257], 2, 64, 64, 300, "entry", False), ([1030], 1, 48, 48, 129, None, True)])
+def test_against_64_bits(lens, heads, rot, dims, window, gate, sink):
+    """Edges of tiles (128) and chunks (64), one-token sequences, windows around both, partial rotations, every gate.  From
+    rounded queries on the kernel rounds weights and results: 2^-9 of each weight and of the result, so at most 2^-8 of the
+    weighted magnitudes; as much again for queries that round the other way at a tie and 32-bit sums."""
+    scale = (DIM + rot) ** -0.5
+    x, rank = _inputs(lens, heads, rot, dims, sum(lens))
+    got, gates = _run(x, rank, lens, heads, rot, dims, window, gate, sink, scale)
+    want, size = _reference(x, rank, lens, heads, rot, dims, window, gates, sink, scale)
+    assert ((got.double() - want).abs() <= 2.0 ** -7 * size + 1e-6).all()
+    assert (got.double() - want).norm() <= 4e-3 * want.norm()
+
+
+@pytest.mark.parametrize("n,window", [(300, None), (65, 64), (450, 100), (130, 1)])
+@pytest.mark.parametrize("what", [float("nan"), float("inf")])
+def test_values_that_are_not_finite_reach_those_who_see_them(n, window, what):
+    """A key's or a value's number that is not finite, in the sequence itself or in its neighbour: nobody's results change
+    who does not see the position, and those who do get NaN (a value of the position: in its column)."""
+    heads, rot, dims = 2, 64, 0
+    lens = [n, 70]
+    x, rank = _inputs(lens, heads, rot, dims, n)
+    args = (rank, lens, heads, rot, dims, window, None, False, (DIM + rot) ** -0.5)
+    base, _ = _run(x, *args)
+    assert base.isfinite().all()
+    pos = torch.arange(n + 70, device="cuda")
+    seq = (pos >= n).int()
+    for at in (0, 1, 63, 64, n // 2, n - 1, n, n + 69):
+        sees = (pos >= at) & (seq == int(at >= n)) & ((pos - at < window) if window else (pos >= 0))
+        bad = dict(x, kv=x["kv"].clone())
+        bad["kv"][at, heads * DIM + DIM + 5] = what          # head 1's value
+        got, _ = _run(bad, *args)
+        same = torch.ones_like(base, dtype=torch.bool)
+        same[:, 1, 5] = ~sees
+        assert torch.equal(got[same], base[same]), at
+        assert (~got[:, 1, 5][sees].isfinite()).all(), at
+        bad = dict(x, kv=x["kv"].clone())
+        bad["kv"][at, 3] = what                              # head 0's key
+        got, _ = _run(bad, *args)
+        assert torch.equal(got[:, 1], base[:, 1]) and torch.equal(got[~sees], base[~sees]), at
+        if what != what:
+            assert got[sees, 0].isnan().all(), at
+
+
+@pytest.mark.parametrize("heads,lens,window,sink,q_rank", [(4, [300, 33], None, False, 96), (4, [200], 90, True, None)])
+def test_a_step_is_as_near_to_64_bits_as_on_the_cached_vectors(heads, lens, window, sink, q_rank):
+    """The mixer on a step that starts its sequences, with the keys formed and without.  Each way rounds a query and one more
+    number per key or result to bfloat16, so their errors are alike; a fifth is left for the draw."""
+    from torchless_rs_b200.config.spec import PartSpec
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.parts import latent_attention
+    from torchless_rs_b200.parts.runtime import Runtime
+    rt = Runtime("cuda:0", BF)
+    W, rank, rot = 256, 128, 64
+    spec = PartSpec("latent_attention", {"hidden_size": W, "heads": heads, "dim": DIM, "rot_dim": rot, "vdim": DIM, "q_rank": q_rank,
+                                         "kv_rank": rank, "window": window, "eps": 1e-5, "sink": sink, "gate": "entry"})
+    part = latent_attention.LatentAttention(spec, "m", rt, None)
+    g = torch.Generator(device="cuda").manual_seed(heads + sum(lens))
+    w = {}
+    for name, t in part.expected_tensors(spec, "m").items():
+        w[name] = torch.randn(tuple(t.shape), device="cuda", generator=g) * (t.shape[1] ** -0.5 if len(t.shape) == 2 else 1.0)
+        w[name] = w[name].to(BF)
+    part.load(w)
+    T, B = sum(lens), len(lens)
+    need = [-(-n // 64) for n in lens]
+    table = torch.full((B, max(need)), -1, dtype=torch.int32)
+    for b in range(B):
+        table[b, :need[b]] = torch.arange(sum(need[:b]), sum(need[:b + 1]))
+    part.bind_cache(SimpleNamespace(pages=torch.zeros((sum(need), 64, rank + rot), device="cuda", dtype=BF), page_table=table.cuda()))
+    batch = _step(lens)
+    batch.token_pos, batch.token_seq = _i32(sum([list(range(n)) for n in lens], [])), _i32(sum([[b] * n for b, n in enumerate(lens)], []))
+    batch.seq_slot, batch.len_bucket, batch.plans = _i32(list(range(B))), 1024, {}
+    xn = torch.randn((T, W), device="cuda", generator=g).to(BF)
+
+    def run():
+        out = torch.zeros((T, W), device="cuda")
+        part.forward(xn, out, batch, overwrite=True)
+        return out.double()
+    before = ops.launch_counts().get("latent_prompt_tc", 0)
+    formed = run()
+    assert ops.launch_counts().get("latent_prompt_tc", 0) == before + 1
+    part.prompt = None
+    latent = run()
+    assert ops.launch_counts().get("latent_prompt_tc", 0) == before + 1
+    d = {k[2:]: v.double() for k, v in w.items()}
+    rms = lambda t: t / torch.sqrt((t * t).mean(-1, keepdim=True) + 1e-5)
+    h, want, at = xn.double(), [], 0
+    q = (rms(h @ d["dq"].T) * d["dq.norm"]) @ d["uq"].T if q_rank else h @ d["q"].T
+    down = h @ d["dkv"].T
+    c = rms(down[:, :rank]) * d["dkv.norm"]
+    for n in lens:
+        s_ = slice(at, at + n)
+        qs = q[s_].view(n, heads, DIM + rot)
+        k = torch.cat([(c[s_] @ d["uk"].T).view(n, heads, DIM), down[s_, None, rank:].expand(n, heads, rot)], -1)
+        v = (c[s_] @ d["uv"].T).view(n, heads, DIM)
+        sc = torch.einsum("thd,shd->hts", qs, k) * part.scale
+        i = torch.arange(n, device="cuda")
+        sc.masked_fill_((i[:, None] < i) | ((i[:, None] - i >= window) if window else (i[:, None] < i)), -float("inf"))
+        if sink:
+            sc = torch.cat([sc, d["sink"][:, None, None].expand(heads, n, 1)], -1)
+        want.append(torch.einsum("hts,shd->thd", torch.softmax(sc, -1)[..., :n], v).reshape(n, -1))
+        at += n
+    want = (torch.cat(want) * torch.sigmoid(h @ d["g"].T)) @ d["o"].T
+    a, b = (float((x - want).norm() / want.norm()) for x in (formed, latent))
+    print(f"error against 64 bits: formed {a:.3e}, latent {b:.3e}")
+    assert a <= 1.2 * b and a < 2e-2, (a, b)

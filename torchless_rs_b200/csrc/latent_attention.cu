@@ -17,7 +17,8 @@
 // Per token, from the 32-bit down-projections:
 //   cq[t, :]  = dq[t, :] / rms * wq                          (query latent, activation type)
 //   page row  = [ dkv[t, :rank] / rms * wc | rotate(dkv[t, rank:rank+rot]) ]   at the token's place
-// Without a query latent (q_rank = 0) only the page row is written.
+// Without a query latent (q_rank = 0) only the page row is written.  `flat` (or null) gets the page rows in token order,
+// `turn` (or null) the cosine and sine of every (token, pair).
 // Rotation: entry i of the rot part pairs with entry i + dims/2 (i < dims/2), angle =
 // position * inv_freq[i], sine and cosine times `amp`; entries from `dims` on pass unchanged.
 // ---------------------------------------------------------------------------
@@ -27,7 +28,8 @@ __global__ void latent_prep_kernel(const float* __restrict__ dq, int ld_dq, cons
                                    const int* __restrict__ token_pos, const int* __restrict__ token_seq,
                                    const int* __restrict__ seq_slot, const int* __restrict__ page_table,
                                    int table_stride, const float* __restrict__ inv_freq, int q_rank, int rank,
-                                   int rot, int dims, float amp) {
+                                   int rot, int dims, float amp, act_t* __restrict__ flat,
+                                   float2* __restrict__ turn) {
   __shared__ float scratch[33];
   pdl_wait();
   pdl_launch_dependents();
@@ -46,7 +48,12 @@ __global__ void latent_prep_kernel(const float* __restrict__ dq, int ld_dq, cons
   const int page = page_table[(size_t)seq_slot[token_seq[t]] * table_stride + pos / TL_PAGE];
   const int width = rank + rot;
   act_t* row = pages + ((size_t)page * TL_PAGE + (pos % TL_PAGE)) * width;
-  for (int i = threadIdx.x; i < rank; i += blockDim.x) row[i] = from_f32<act_t>((b[i] / rc) * wc[i]);
+  act_t* copy = flat != nullptr ? flat + (size_t)t * width : nullptr;
+  for (int i = threadIdx.x; i < rank; i += blockDim.x) {
+    const act_t y = from_f32<act_t>((b[i] / rc) * wc[i]);
+    row[i] = y;
+    if (copy != nullptr) copy[i] = y;
+  }
   const int half = dims >> 1;
   const float* r = b + rank;
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
@@ -55,22 +62,29 @@ __global__ void latent_prep_kernel(const float* __restrict__ dq, int ld_dq, cons
     sn *= amp;
     cs *= amp;
     const float u = r[i], v = r[i + half];
-    row[rank + i] = from_f32<act_t>(u * cs - v * sn);
-    row[rank + i + half] = from_f32<act_t>(v * cs + u * sn);
+    const act_t y0 = from_f32<act_t>(u * cs - v * sn), y1 = from_f32<act_t>(v * cs + u * sn);
+    row[rank + i] = y0;
+    row[rank + i + half] = y1;
+    if (copy != nullptr) { copy[rank + i] = y0; copy[rank + i + half] = y1; }
+    if (turn != nullptr) turn[(size_t)t * half + i] = make_float2(cs, sn);
   }
-  for (int i = dims + threadIdx.x; i < rot; i += blockDim.x) row[rank + i] = from_f32<act_t>(r[i]);
+  for (int i = dims + threadIdx.x; i < rot; i += blockDim.x) {
+    const act_t y = from_f32<act_t>(r[i]);
+    row[rank + i] = y;
+    if (copy != nullptr) copy[rank + i] = y;
+  }
 }
 
 extern "C" int TL_NAME(tl_latent_prep)(const float* dq, int ld_dq, const float* dkv, int ld_dkv, const float* wq,
                                        const float* wc, float eps, void* cq, void* pages, const int* token_pos,
                                        const int* token_seq, const int* seq_slot, const int* page_table,
                                        int table_stride, const float* inv_freq, int T, int q_rank, int rank,
-                                       int rot, int dims, float amp, cudaStream_t stream) {
+                                       int rot, int dims, float amp, void* flat, void* turn, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (q_rank < 0 || rank <= 0 || rot < 0 || dims < 0 || dims > rot || (dims & 1)) return TL_ERR_BAD_ARG;
   return tl_launch(latent_prep_kernel, dim3(T), dim3(128), 0, stream, dq, ld_dq, dkv, ld_dkv, wq, wc, eps,
                    (act_t*)cq, (act_t*)pages, token_pos, token_seq, seq_slot, page_table, table_stride, inv_freq,
-                   q_rank, rank, rot, dims, amp);
+                   q_rank, rank, rot, dims, amp, (act_t*)flat, (float2*)turn);
 }
 
 // ---------------------------------------------------------------------------

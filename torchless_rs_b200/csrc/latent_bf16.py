@@ -1,5 +1,6 @@
-"""Prompts of the latent attention on tensor cores (kernel in latent_attention_tc.cu).  `run` returns False for steps and
-sizes it does not take; the caller then uses the kernels of latent_attention.cu."""
+"""Prompts of the latent attention on tensor cores.  `LatentBf16` (kernel in latent_attention_tc.cu) works on the cached
+vectors themselves, `LatentPrompt` (kernel in latent_prompt_tc.cu) on keys and values that are formed for the step.  `run`
+returns False for steps and sizes that are not taken; the caller then uses the kernels of latent_attention.cu."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -8,9 +9,10 @@ from typing import Optional, Tuple
 import torch
 
 from . import build
-from .ops import _check, _stream, register_error_word
+from .ops import KernelError, _check, _stream, register_error_word
 
 build.register_library("latent_tc", ("latent_attention_tc.cu",), ())
+build.register_library("latent_prompt", ("latent_prompt_tc.cu",), ())
 
 PAGE = build.PAGE_TOKENS
 
@@ -96,3 +98,75 @@ class LatentBf16:
     def take_error(self) -> int:
         """Nonzero if the kernel gave up on a bounded wait since the last call (synchronises)."""
         return int(self.lib.tl_latent_tc_take_error())
+
+
+class LatentPrompt:
+    _inst = None
+    DIM, VDIM, MOST_ROT = 128, 128, 64      # the sizes of a head that the kernel is written for
+
+    @classmethod
+    def get(cls) -> "LatentPrompt":
+        if cls._inst is None:
+            cls._inst = cls()
+        return cls._inst
+
+    def __init__(self):
+        self.lib = build.load_library("latent_prompt")
+        P, I = c_void_p, c_int
+        self.lib.tl_latent_prompt_tc.restype = c_int
+        self.lib.tl_latent_prompt_tc.argtypes = [P, I, P, P, P, P, P, I, I, P, P] + [I] * 10 + [c_float, P]
+        self.lib.tl_latent_prompt_take_error.restype = c_int
+        register_error_word("latent_prompt", self.take_error)
+
+    @classmethod
+    def fits(cls, dim: int, vdim: int, rank: int, rot: int) -> bool:
+        return dim == cls.DIM and vdim == cls.VDIM and rank % 8 == 0 and rot % 8 == 0 and rot <= cls.MOST_ROT
+
+    @staticmethod
+    def takes(batch) -> bool:
+        """Whether a step's keys are the ones it brings (every sequence starts with it), and more than four a sequence: a
+        block per head and 128 tokens of a sequence costs some 8 us however few of its rows are filled.  The whole mixer
+        with the keys formed / on the cached vectors, 16 heads, query latent of 768, us: 17 tokens 38 / 62, 100 61 / 84,
+        300 72 / 107, 1000 107 / 181, 2048 154 / 393, 4096 283 / 963; 20 sequences of 1 token 45 / 63, 64 of 3 95 / 92,
+        16 of 17 59 / 86, 32 of 50 126 / 186, 32 of 500 750 / 1852; 32 heads: 2048 tokens 298 / 773, 64 sequences of 3
+        148 / 133."""
+        past = getattr(batch, "past_lens", None)
+        if batch.is_decode or past is None or any(past):
+            return False
+        return sum(batch.new_lens) > 4 * len(past)
+
+    def run(self, q: torch.Tensor, turn: Optional[torch.Tensor], kv: torch.Tensor, latents: torch.Tensor, out: torch.Tensor,
+            gate: Optional[torch.Tensor], sink: Optional[torch.Tensor], batch, heads: int, rank: int, rot: int, dims: int,
+            window: Optional[int], scale: float) -> bool:
+        """out[t, h] = softmax over the tokens that t sees of ((q . k_h) + (rotated q . r)) * scale times their v_h, times
+        sigmoid(gate).  `q`: [T, >= heads * (128 + rot)] 32-bit, before the rotation by `turn` ([T, dims / 2, 2], cosine and
+        sine); `kv`: [T, 2, heads, 128]; `latents`: [T, rank + rot], whose last columns are r; `gate`: [T, heads * 128] or
+        [T, heads] 32-bit, or None."""
+        T = out.shape[0]
+        width = heads * (self.DIM + self.VDIM)
+        for t, n, dtype, cols in ((q, "queries", torch.float32, heads * (self.DIM + rot)), (kv, "keys and values", out.dtype, width),
+                                  (latents, "latents", out.dtype, rank + rot), (out, "out", torch.bfloat16, heads * self.VDIM)):
+            if not t.is_cuda or t.dtype != dtype or t.dim() != 2 or t.shape[0] != T or t.stride(1) != 1 or t.shape[1] < cols or \
+                    (t is not q and t.stride(0) != cols):
+                raise KernelError(f"latent_prompt: {n} {tuple(t.shape)} {t.dtype} do not fit")
+        if gate is not None and (gate.dtype != torch.float32 or gate.shape not in ((T, heads), (T, heads * self.VDIM)) or
+                                 gate.stride(1) != 1):
+            raise KernelError("latent_prompt: the gate must be [tokens, heads] or [tokens, heads * 128]")
+        if dims and (turn is None or turn.dtype != torch.float32 or turn.numel() != T * dims or not turn.is_contiguous()):
+            raise KernelError("latent_prompt: the turns must be [tokens, dims / 2, 2]")
+        if sink is not None and (sink.dtype != torch.float32 or sink.numel() != heads):
+            raise KernelError("latent_prompt: one sink per head is needed")
+        addr = lambda t: t.data_ptr() if t is not None else None
+        st = self.lib.tl_latent_prompt_tc(
+            q.data_ptr(), q.stride(0), addr(turn if dims else None), kv.data_ptr(), latents.data_ptr(), out.data_ptr(), addr(gate),
+            gate.stride(0) if gate is not None else 0, int(gate is not None and gate.shape[1] == heads), addr(sink),
+            batch.seq_start.data_ptr(), T, batch.n_seqs, batch.max_new, heads, self.DIM, self.VDIM, rank, rot, dims, window or 0,
+            scale, _stream())
+        if st == -2:
+            return False
+        _check(st, "latent_prompt_tc")
+        return True
+
+    def take_error(self) -> int:
+        """Nonzero if the kernel gave up on a bounded wait since the last call (synchronises)."""
+        return int(self.lib.tl_latent_prompt_take_error())

@@ -371,9 +371,11 @@ class CoreOps:
     def latent_prep(self, dq: Optional[torch.Tensor], dkv: torch.Tensor, wq: Optional[torch.Tensor], wc: torch.Tensor,
                     eps: float, cq: Optional[torch.Tensor], pages: torch.Tensor, token_pos: torch.Tensor, token_seq: torch.Tensor,
                     seq_slot: torch.Tensor, page_table: torch.Tensor, inv_freq: Optional[torch.Tensor],
-                    rank: int, rot: int, dims: int, amplitude: float = 1.0) -> None:
+                    rank: int, rot: int, dims: int, amplitude: float = 1.0, flat: Optional[torch.Tensor] = None,
+                    turn: Optional[torch.Tensor] = None) -> None:
         """cq = norm(dq) * wq (none of the three: no query latent); the token's page row =
-        [norm(dkv[:, :rank]) * wc | rotate(dkv[:, rank:])], sine and cosine times `amplitude`."""
+        [norm(dkv[:, :rank]) * wc | rotate(dkv[:, rank:])], sine and cosine times `amplitude`.  `flat` ([T, rank + rot])
+        also gets the rows in token order, `turn` ([T, dims / 2, 2], 32-bit) the cosines and sines."""
         for t, n in ((dq, "query down-projection"), (dkv, "key/value down-projection")):
             if t is None and dq is None:
                 continue
@@ -399,11 +401,19 @@ class CoreOps:
             _need(inv_freq, torch.float32, "inv_freq")
             if inv_freq.numel() != dims // 2:
                 raise KernelError("latent_prep: inv_freq must have dims/2 entries")
+        if flat is not None:
+            _need(flat, self.act_dtype, "latents in token order")
+            if flat.shape != (T, rank + rot):
+                raise KernelError("latent_prep: sizes do not match")
+        if turn is not None:
+            _need(turn, torch.float32, "turns")
+            if turn.numel() != T * dims:
+                raise KernelError("latent_prep: sizes do not match")
         _check(self._tl_latent_prep(
             _ptr(dq), c_int(dq.stride(0) if dq is not None else 0), _ptr(dkv), c_int(dkv.stride(0)), _ptr(wq), _ptr(wc), c_float(eps),
             _ptr(cq), _ptr(pages), _ptr(token_pos), _ptr(token_seq), _ptr(seq_slot), _ptr(page_table),
             c_int(page_table.stride(0)), _ptr(inv_freq if dims else None), c_int(T), c_int(q_rank), c_int(rank),
-            c_int(rot), c_int(dims), c_float(amplitude), _stream()), "latent_prep")
+            c_int(rot), c_int(dims), c_float(amplitude), _ptr(flat), _ptr(turn), _stream()), "latent_prep")
 
     def headwise_gemm(self, a: torch.Tensor, a_head: int, w: torch.Tensor, c: torch.Tensor, c_head: int,
                       gate: Optional[torch.Tensor] = None, act_out: bool = False) -> None:

@@ -9,10 +9,11 @@ With h the mixer's input, per token:
     k_h = [W_uk,h c | r],  v_h = W_uv,h c,  score = (q_h . k_h) * scale over the window
     p(i, j) = exp(score(i, j)) / (sum over visible j' of exp(score(i, j')) [+ exp(sink_h)])
     out = W_o ((heads' weighted values, concatenated) [* sigmoid(W_g h)])
-Only [c | r] is cached, one vector per position (`PagedLatentRequest`).  Keys and values are
-never formed: q's plain part is carried into the latent space (W_uk,h^T q_h), the weighted sum
-is taken over the c's, and W_uv,h is applied to the sum, so prefill and decode run the same
-kernels on the same pages and a position's result does not depend on the step that computes it.
+Only [c | r] is cached, one vector per position (`PagedLatentRequest`).  Steps that go on with a
+sequence never form keys and values: q's plain part is carried into the latent space (W_uk,h^T q_h), the
+weighted sum is taken over the c's, and W_uv,h is applied to the sum, straight from the pages.  In bfloat16
+a step whose sequences all start with it forms the keys and values of its own tokens, where its kernel takes the
+head's sizes (`LatentPrompt`): the same sums, rounded at k_h and v_h instead of at W_uk,h^T q_h and the sum of c's.
 The projections of h (W_dq or W_q, W_dkv and, with a gate, W_g) are one stacked product.
 
 The rotated parts of a query and of the shared key only ever meet in their dot product, which does
@@ -28,7 +29,7 @@ import torch
 
 from ..cache.requests import PagedLatentRequest
 from ..config.spec import PartSpec
-from ..csrc import ops
+from ..csrc import latent_bf16, ops
 from ..weights.loader import TensorSpec
 from .linear import Matmul
 from .registry import register_mixer
@@ -143,6 +144,10 @@ class LatentAttention:
         self.w_uk_t = rt.matrix(uk)                                          # [heads, rank, dim]
         self.w_uv = rt.matrix(weights[f"{p}.uv"].reshape(self.heads, self.vdim, self.rank))
         self.w_o = rt.matrix(weights[f"{p}.o"])
+        self.prompt = None
+        if not rt.is_f32 and latent_bf16.LatentPrompt.fits(self.dim, self.vdim, self.rank, self.rot):
+            self.prompt = latent_bf16.LatentPrompt.get()
+            self.w_kv = rt.stack([weights[f"{p}.uk"], weights[f"{p}.uv"]])
         f32 = lambda t: t.to(device=rt.device, dtype=torch.float32).contiguous()
         self.norm_q = f32(weights[f"{p}.dq.norm"]) if self.q_rank else None
         self.norm_c = f32(weights[f"{p}.dkv.norm"])
@@ -178,9 +183,17 @@ class LatentAttention:
         self.matmul(xn, self.w_in, s, ops.MODE_STORE_F32)
         dkv = s[:, n_q:g_off]
         cq = ws.get("latent_cq", (T, q_rank), rt.act_dtype) if q_rank else None
+        gate = s[:, g_off:g_off + self.gate_rows] if self.gate_rows else None
+        forms = self.prompt is not None and T > self.FEW_TOKENS and self.prompt.takes(batch)
+        flat = ws.get("latent_flat", (T, rank + rot), rt.act_dtype) if forms else None
+        turn = ws.get("latent_turn", (T, self.rot_dims), torch.float32) if forms and self.rot_dims else None
         o.latent_prep(s[:, :q_rank] if q_rank else None, dkv, self.norm_q, self.norm_c, self.eps, cq, c.pages,
                       batch.token_pos, batch.token_seq, batch.seq_slot, c.page_table, inv_freq, rank, rot,
-                      self.rot_dims, amplitude=self.amplitude)
+                      self.rot_dims, amplitude=self.amplitude, flat=flat, turn=turn)
+        gated = ws.get("latent_gated", (T, H * vdim), rt.act_dtype)
+        if forms and self._form_and_attend(s, cq, flat, turn, gate, gated, batch):
+            self.matmul(gated, self.w_o, residual, ops.MODE_STORE_F32 if overwrite else ops.MODE_ACCUM_F32)
+            return
         mix = ws.get("latent_mix", (T, H, rank), torch.float32)
         if not q_rank or T <= self.FEW_TOKENS:
             # without a query latent, or for few tokens (two small matrices are fewer bytes to stream than the
@@ -200,7 +213,18 @@ class LatentAttention:
                       c.page_table, inv_freq, H, rank, rot, self.rot_dims, self.window, self.scale,
                       max_keys=batch.len_bucket, workspace=ws, sink=self.sink, amplitude=self.amplitude,
                       batch=batch)
-        gated = ws.get("latent_gated", (T, H * vdim), rt.act_dtype)
-        o.headwise_gemm(mix.view(T, H * rank), rank, self.w_uv, gated, vdim,
-                        gate=s[:, g_off:g_off + self.gate_rows] if self.gate_rows else None, act_out=True)
+        o.headwise_gemm(mix.view(T, H * rank), rank, self.w_uv, gated, vdim, gate=gate, act_out=True)
         self.matmul(gated, self.w_o, residual, ops.MODE_STORE_F32 if overwrite else ops.MODE_ACCUM_F32)
+
+    def _form_and_attend(self, s, cq, latents, turn, gate, gated, batch) -> bool:
+        """The step's keys and values from its latents, and the attention over them, gated.  False if its kernel does not
+        take the step."""
+        ws, T, H = self.rt.workspace, gated.shape[0], self.heads
+        q = s
+        if self.q_rank:
+            q = ws.get("latent_q", (T, H * (self.dim + self.rot)), torch.float32)
+            self.matmul(cq, self.w_uq, q, ops.MODE_STORE_F32)
+        kv = ws.get("latent_kv", (T, H * (self.dim + self.vdim)), self.rt.act_dtype)
+        self.matmul(latents[:, :self.rank], self.w_kv, kv, ops.MODE_STORE_ACT)
+        return self.prompt.run(q, turn, kv, latents, gated, gate, self.sink, batch, H, self.rank, self.rot, self.rot_dims,
+                               self.window, self.scale)
