@@ -927,3 +927,29 @@ def test_weight_conversion_on_the_device(dtype, stored):
     assert got.dtype == dtype and got.shape == (42, 72) and got.is_cuda
     assert torch.equal(got.cpu(), torch.cat([a, b]).to(dtype))
     assert torch.equal(rt.matrix(b).cpu(), b.to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 100, 127, 128, 129, 140, 300])
+@pytest.mark.parametrize("nh,nkv,hd,pad", [(32, 8, 128, 0), (5, 3, 128, 4), (48, 8, 128, 0), (33, 9, 64, 0), (70, 3, 32, 0), (17, 1, 256, 0)])
+def test_rope_cache_write_of_one_to_four_passes(dtype, T, nh, nkv, hd, pad):
+    """Head counts that need one to several passes of a block, filled and not, on both sides of the lines between its forms,
+    against the kernel of a warp per head (which rows off a 16-byte boundary take): the same operations, so the same bits."""
+    o = _ops(dtype)
+    cols, pages = (nh + 2 * nkv) * hd, (T + 63) // 64
+    x = _rand((T, cols + pad), torch.float32, T + nh)
+    odd = torch.empty((T, cols + 1), dtype=torch.float32, device=DEV)
+    odd[:, :cols] = x[:, :cols]
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    seq, slot = torch.zeros_like(pos), torch.zeros(1, dtype=torch.int32, device=DEV)
+    table = torch.arange(pages - 1, -1, -1, dtype=torch.int32, device=DEV)[None].contiguous()
+    inv = (1e4 ** (-torch.arange(hd // 2, dtype=torch.float64) * 2 / hd)).float().to(DEV)
+    got = []
+    for qkv in (x, odd):
+        q = torch.empty((T, nh * hd), dtype=dtype, device=DEV)
+        kp, vp = (torch.zeros((pages, nkv, 64, hd), dtype=dtype, device=DEV).view(s)
+                  for s in ((pages, nkv, 64, hd), (pages, nkv, hd, 64)))
+        o.rope_cache_write(qkv, q, kp, vp, pos, seq, slot, table, inv, 0, nh, nkv, hd)
+        got.append((q, kp, vp))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

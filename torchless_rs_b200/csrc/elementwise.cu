@@ -295,24 +295,30 @@ __global__ void rope_cache_write_kernel(const float* __restrict__ qkv, int ld,
   }
 }
 
-// The same for steps of many tokens, half-split pairs (style 0) and head sizes of 32, 64,
-// 128 or 256.  Two kinds of block in one launch:
-//  - blockIdx.y < rot_groups: one token; its query and key heads are rotated four pairs per
-//    lane with 16-byte loads, hd/8 lanes per head and 256/hd heads per warp at a time;
-//  - blockIdx.y == rot_groups: 32 consecutive tokens of one value head; the tile is turned
-//    in shared memory, so that the transposed value pages are written in runs of positions.
+// The same for half-split pairs (style 0) and head sizes of 32, 64, 128 or 256.  Three kinds of block in one launch:
+//  - blockIdx.y < rot_groups: one token; a pass of the block turns 1024 / hd of its query and key heads, four pairs per
+//    thread with 16-byte loads, PASSES of them, whose loads are all issued before the angles are worked out;
+//  - blockIdx.y == rot_groups, `turned`: 32 consecutive tokens of one value head; the tile is turned in shared memory, so
+//    that the transposed value pages are written in runs of positions;
+//  - blockIdx.y == rot_groups otherwise: one token's value heads, written as they are read.
+// What bounds it is the chain of a block (position, angle, sine; sequence, slot, page) beside few bytes, hence the loads
+// first.  Bfloat16, 32 + 8 heads of 128, a warp per head below 256 tokens and loads after the angles from there on / now: in
+// decode steps of 64 sequences 7.0 / 4.2 us, in prompts of 100 tokens 7.1 / 4.2 us, of 2048 20.6 / 19.3 us; alone 200 tokens
+// 10.4 / 4.2 us, 2048 14.3 / 12.5 us, 8192 63 / 54 us (302 MB).
+#define ROPE_PASSES 4
+template <int PASSES>
 __global__ void __launch_bounds__(128)
 rope_cache_write_vec_kernel(const float* __restrict__ qkv, int ld, act_t* __restrict__ q_out,
                             act_t* __restrict__ k_pages, act_t* __restrict__ v_pages,
                             const int* __restrict__ token_pos, const int* __restrict__ token_seq,
                             const int* __restrict__ seq_slot, const int* __restrict__ page_table,
                             int table_stride, const float* __restrict__ inv_freq, int T, int nh,
-                            int nkv, int hd, int rot_groups) {
+                            int nkv, int hd, int rot_groups, int turned) {
   extern __shared__ float vt[];   // [32 tokens][hd + 1]
   pdl_wait();
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if ((int)blockIdx.y == rot_groups) {
+  if ((int)blockIdx.y == rot_groups && turned) {
     const int tiles_t = (T + 31) / 32;
     for (int tile = blockIdx.x; tile < tiles_t * nkv; tile += gridDim.x) {
       const int t0 = (tile / nkv) * 32, kvh = tile % nkv;
@@ -331,7 +337,8 @@ rope_cache_write_vec_kernel(const float* __restrict__ qkv, int ld, act_t* __rest
         const int pos = token_pos[t];
         const int page = page_table[(size_t)seq_slot[token_seq[t]] * table_stride + pos / TL_PAGE];
         act_t* dst = v_pages + ((size_t)page * nkv + kvh) * (size_t)(TL_PAGE * hd) + (pos % TL_PAGE);
-        for (int d = warp; d < hd; d += 4) dst[(size_t)d * TL_PAGE] = from_f32<act_t>(vt[lane * (hd + 1) + d]);
+        if (page >= 0)
+          for (int d = warp; d < hd; d += 4) dst[(size_t)d * TL_PAGE] = from_f32<act_t>(vt[lane * (hd + 1) + d]);
       }
       __syncthreads();
     }
@@ -339,43 +346,58 @@ rope_cache_write_vec_kernel(const float* __restrict__ qkv, int ld, act_t* __rest
   }
   const int t = blockIdx.x;
   const int pos = token_pos[t];
-  const int half = hd >> 1;
-  const int lph = hd >> 3;            // lanes per head
-  const int hpp = 32 / lph;           // heads per warp pass
-  const int sub = lane / lph, i0 = (lane % lph) * 4;
   const int page = page_table[(size_t)seq_slot[token_seq[t]] * table_stride + pos / TL_PAGE];
-  // cosine and sine of the token's angles: each once per block (a thread per pair of dimensions),
-  // then read by every lane that turns that pair; the full-precision sine is most of this
-  // kernel's arithmetic otherwise
+  if ((int)blockIdx.y == rot_groups) {
+    const float* row = qkv + (size_t)t * ld + (size_t)(nh + nkv) * hd;
+    act_t* dst = v_pages + (size_t)page * nkv * (size_t)(TL_PAGE * hd) + (pos % TL_PAGE);
+    if (page < 0) return;
+#pragma unroll 2
+    for (int d = threadIdx.x * 4; d < nkv * hd; d += 512) {     // (the heads of a page follow one another)
+      float v[4];
+      load4(row + d, v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[(size_t)(d + j) * TL_PAGE] = from_f32<act_t>(v[j]);
+    }
+    return;
+  }
+  const int half = hd >> 1;
+  const int lph = hd >> 3;            // threads per head
+  const int hpp = 128 / lph;          // heads per pass
+  const int sub = threadIdx.x / lph, i0 = (threadIdx.x % lph) * 4;
+  const int rot_heads = nh + nkv, h0 = (int)blockIdx.y * PASSES * hpp + sub;
+  const float* row = qkv + (size_t)t * ld + i0;
+  float a[PASSES][4], b[PASSES][4];
+#pragma unroll
+  for (int u = 0; u < PASSES; ++u) {
+    const int h = h0 + u * hpp;
+    if (h < rot_heads) {
+      load4(row + (size_t)h * hd, a[u]);
+      load4(row + (size_t)h * hd + half, b[u]);
+    }
+  }
+  // each angle's cosine and sine once per block, while the loads are under way
   float2* cs_s = reinterpret_cast<float2*>(vt);   // [hd / 2]; the value blocks use `vt` otherwise
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+  if ((int)threadIdx.x < half) {
     float s_ = 0.0f, c_ = 1.0f;
-    if (inv_freq) sincosf((float)pos * inv_freq[i], &s_, &c_);
-    cs_s[i] = make_float2(c_, s_);
+    if (inv_freq) sincosf((float)pos * inv_freq[threadIdx.x], &s_, &c_);
+    cs_s[threadIdx.x] = make_float2(c_, s_);
   }
   __syncthreads();
   float cs[4], sn[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) { cs[j] = cs_s[i0 + j].x; sn[j] = cs_s[i0 + j].y; }
-  const int rot_heads = nh + nkv;
-  const int passes = (rot_heads + hpp - 1) / hpp;
-  const int per_group = (passes + rot_groups - 1) / rot_groups;
-  const int p_end = min(((int)blockIdx.y + 1) * per_group, passes);
-#pragma unroll 2
-  for (int p = (int)blockIdx.y * per_group + warp; p < p_end; p += 4) {
-    const int h = p * hpp + sub;
-    if (h >= rot_heads) continue;
-    const float* row = qkv + (size_t)t * ld + (size_t)h * hd;
+#pragma unroll
+  for (int u = 0; u < PASSES; ++u) {
+    const int h = h0 + u * hpp;
+    if (h >= rot_heads || (h >= nh && page < 0)) continue;
     act_t* dst = h < nh ? q_out + ((size_t)t * nh + h) * hd
                         : k_pages + ((size_t)page * nkv + (h - nh)) * (size_t)(TL_PAGE * hd) +
                               (size_t)(pos % TL_PAGE) * hd;
-    float a[4], b[4], lo[4], hi[4];
-    load4(row + i0, a);
-    load4(row + half + i0, b);
+    float lo[4], hi[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      lo[j] = a[j] * cs[j] - b[j] * sn[j];
-      hi[j] = a[j] * sn[j] + b[j] * cs[j];
+      lo[j] = a[u][j] * cs[j] - b[u][j] * sn[j];
+      hi[j] = a[u][j] * sn[j] + b[u][j] * cs[j];
     }
     store4(dst + i0, lo);
     store4(dst + half + i0, hi);
@@ -391,15 +413,26 @@ extern "C" int TL_NAME(tl_rope_cache_write)(const float* qkv, int ld, void* q_ou
   if (T <= 0) return 0;
   if ((hd & 1) || hd > 256) return TL_ERR_BAD_ARG;
   const int heads = nh + (k_pages ? 2 * nkv : 0);
-  if (T >= 256 && style == 0 && k_pages && v_pages && (hd == 32 || hd == 64 || hd == 128 || hd == 256) &&
-      ld % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && nkv <= 65535) {
-    const int passes = (nh + nkv + 256 / hd - 1) / (256 / hd);
-    int rot_groups = (passes + 7) / 8;   // at most two passes for each of a block's four warps
+  if (style == 0 && k_pages && v_pages && (hd == 32 || hd == 64 || hd == 128 || hd == 256) && ld % 4 == 0 &&
+      (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pages) & 15) == 0) {
+    const int passes = (nh + nkv + 1024 / hd - 1) / (1024 / hd);
+    // while the GPU has few blocks a pass to a block, then as many as a thread's registers take
+    const int rot_groups = (long long)T * passes < 640 ? passes : (passes + ROPE_PASSES - 1) / ROPE_PASSES;
+    const int per_group = (passes + rot_groups - 1) / rot_groups;
     if (rot_groups > 65534) return TL_ERR_UNSUPPORTED;
-    dim3 grid(T, rot_groups + 1);
-    return tl_launch(rope_cache_write_vec_kernel, grid, dim3(128), (size_t)32 * (hd + 1) * sizeof(float),
-                     stream, qkv, ld, (act_t*)q_out, (act_t*)k_pages, (act_t*)v_pages, token_pos,
-                     token_seq, seq_slot, page_table, table_stride, inv_freq, T, nh, nkv, hd, rot_groups);
+    const int turned = T >= 128;
+    const size_t smem = (turned ? (size_t)32 * (hd + 1) : (size_t)hd) * sizeof(float);
+#define ROPE(P)                                                                                                          \
+  return tl_launch(rope_cache_write_vec_kernel<P>, dim3(T, rot_groups + 1), dim3(128), smem, stream, qkv, ld,            \
+                   (act_t*)q_out, (act_t*)k_pages, (act_t*)v_pages, token_pos, token_seq, seq_slot, page_table,          \
+                   table_stride, inv_freq, T, nh, nkv, hd, rot_groups, turned)
+    switch (per_group) {
+      case 1: ROPE(1);
+      case 2: ROPE(2);
+      case 3: ROPE(3);
+      default: ROPE(4);
+    }
+#undef ROPE
   }
   // few tokens: one warp per (token, head), for parallelism; many tokens: one block per token
   const int per_block = T >= 256 ? heads : 1;
