@@ -124,7 +124,7 @@ def test_values_that_are_not_finite_reach_those_who_see_them(n, window, what):
             assert got[sees, 0].isnan().all(), at
 
 
-@pytest.mark.parametrize("heads,lens,window,sink,q_rank", [(4, [300, 33], None, False, 96), (4, [200], 90, True, None)])
+@pytest.mark.parametrize("heads,lens,window,sink,q_rank", [(4, [600, 33], None, False, 96), (4, [512], 90, True, None)])
 def test_a_step_is_as_near_to_64_bits_as_on_the_cached_vectors(heads, lens, window, sink, q_rank):
     """The mixer on a step that starts its sequences, with the keys formed and without.  Each way rounds a query and one more
     number per key or result to bfloat16, so their errors are alike; a fifth is left for the draw."""

@@ -36,9 +36,9 @@ def test_32_bit_prompt_attention_runs_where_it_was_faster(past, new, nh, nkv, hd
 
 
 @pytest.mark.parametrize("past,new,decode,formed", [
-    ([0], [17], False, True), ([0] * 64, [3] * 64, False, False), ([0] * 64, [5] * 64, False, True), ([0, 1], [400, 9], False, False),
-    ([0], [5], True, False), ([0] * 2, [1, 900], False, True)])
-def test_latent_attention_forms_keys_for_steps_that_start_their_sequences(past, new, decode, formed):
+    ([0], [511], False, False), ([0], [512], False, True), ([0] * 300, [600] + [1] * 299, False, False),
+    ([0] * 100, [600] + [1] * 99, False, True), ([0, 1], [700, 9], False, False), ([0], [512], True, False), ([0] * 2, [1, 900], False, True)])
+def test_latent_attention_forms_keys_for_long_steps_that_start_their_sequences(past, new, decode, formed):
     from types import SimpleNamespace
     assert latent_bf16.LatentPrompt.takes(SimpleNamespace(is_decode=decode, past_lens=past, new_lens=new)) == formed
     assert not latent_bf16.LatentPrompt.takes(SimpleNamespace(is_decode=False))     # a step whose lengths nobody says

@@ -122,18 +122,21 @@ class LatentPrompt:
     def fits(cls, dim: int, vdim: int, rank: int, rot: int) -> bool:
         return dim == cls.DIM and vdim == cls.VDIM and rank % 8 == 0 and rot % 8 == 0 and rot <= cls.MOST_ROT
 
-    @staticmethod
-    def takes(batch) -> bool:
-        """Whether a step's keys are the ones it brings (every sequence starts with it), and more than four a sequence: a
-        block per head and 128 tokens of a sequence costs some 8 us however few of its rows are filled.  The whole mixer
-        with the keys formed / on the cached vectors, 16 heads, query latent of 768, us: 17 tokens 38 / 62, 100 61 / 84,
-        300 72 / 107, 1000 107 / 181, 2048 154 / 393, 4096 283 / 963; 20 sequences of 1 token 45 / 63, 64 of 3 95 / 92,
-        16 of 17 59 / 86, 32 of 50 126 / 186, 32 of 500 750 / 1852; 32 heads: 2048 tokens 298 / 773, 64 sequences of 3
-        148 / 133."""
+    # Tokens of the longest sequence from which a step runs here.  The whole mixer with the keys formed / on the cached vectors, 16
+    # heads, query latent of 768, us: one prompt of 100 tokens 61 / 84, 300 72 / 107, 512 94 / 134, 1000 107 / 181, 2048 154 / 393,
+    # 4096 283 / 963; 16 prompts of 100 120 / 199, 64 of 3 95 / 92 (a block per head and 128 tokens of a sequence costs some
+    # 8 us however few of its rows are filled); 32 heads, 2048 tokens 298 / 773.  It would be faster from some 20 tokens on, but
+    # rounds at other places, which moves logits by 5e-3 of their size either way and a greedy choice in forty: short
+    # prompts, where that buys some 30 us a layer, keep the numbers that they and the steps after them always had.
+    FROM_TOKENS = 512
+
+    @classmethod
+    def takes(cls, batch) -> bool:
+        """Whether a step's keys are the ones it brings (every sequence starts with it), and enough of them."""
         past = getattr(batch, "past_lens", None)
         if batch.is_decode or past is None or any(past):
             return False
-        return sum(batch.new_lens) > 4 * len(past)
+        return max(batch.new_lens) >= cls.FROM_TOKENS and sum(batch.new_lens) > 4 * len(past)
 
     def run(self, q: torch.Tensor, turn: Optional[torch.Tensor], kv: torch.Tensor, latents: torch.Tensor, out: torch.Tensor,
             gate: Optional[torch.Tensor], sink: Optional[torch.Tensor], batch, heads: int, rank: int, rot: int, dims: int,

@@ -12,8 +12,8 @@ With h the mixer's input, per token:
 Only [c | r] is cached, one vector per position (`PagedLatentRequest`).  Steps that go on with a
 sequence never form keys and values: q's plain part is carried into the latent space (W_uk,h^T q_h), the
 weighted sum is taken over the c's, and W_uv,h is applied to the sum, straight from the pages.  In bfloat16
-a step whose sequences all start with it forms the keys and values of its own tokens, where its kernel takes the
-head's sizes (`LatentPrompt`): the same sums, rounded at k_h and v_h instead of at W_uk,h^T q_h and the sum of c's.
+a long step whose sequences all start with it forms the keys and values of its own tokens, where its kernel takes
+the head's sizes (`LatentPrompt`): the same sums, rounded at k_h and v_h instead of at W_uk,h^T q_h and the sum of c's.
 The projections of h (W_dq or W_q, W_dkv and, with a gate, W_g) are one stacked product.
 
 The rotated parts of a query and of the shared key only ever meet in their dot product, which does
@@ -184,7 +184,7 @@ class LatentAttention:
         dkv = s[:, n_q:g_off]
         cq = ws.get("latent_cq", (T, q_rank), rt.act_dtype) if q_rank else None
         gate = s[:, g_off:g_off + self.gate_rows] if self.gate_rows else None
-        forms = self.prompt is not None and T > self.FEW_TOKENS and self.prompt.takes(batch)
+        forms = self.prompt is not None and self.prompt.takes(batch)
         flat = ws.get("latent_flat", (T, rank + rot), rt.act_dtype) if forms else None
         turn = ws.get("latent_turn", (T, self.rot_dims), torch.float32) if forms and self.rot_dims else None
         o.latent_prep(s[:, :q_rank] if q_rank else None, dkv, self.norm_q, self.norm_c, self.eps, cq, c.pages,
