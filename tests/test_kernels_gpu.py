@@ -953,3 +953,26 @@ def test_rope_cache_write_of_one_to_four_passes(dtype, T, nh, nkv, hd, pad):
         got.append((q, kp, vp))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M", [17, 33, 48, 64, 65, 100, 128])
+@pytest.mark.parametrize("N,K,mode,tiles", [(6144, 4096, 0, 32), (1024, 2048, 0, 33), (2048, 1024, 2, 40), (4096, 512, 3, 3), (28672, 512, 0, 100)])
+def test_gemm_scales_rows_by_their_partial_sums(M, N, K, mode, tiles):
+    """The folded norm's 1/rms from any number of partial sums (a thread or a warp per row), with and without K splits, against the
+    same product without it: the scale is one factor per row, so the results agree to the rounding of one 32-bit product per
+    step (and of the result where it is bfloat16)."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc.gemm_bf16 import GemmBf16
+    a, w = _rand((M, K), torch.bfloat16, 1), _rand(((2 * N if mode == 2 else N), K), torch.bfloat16, 2) * 0.05
+    ss = torch.rand((M, tiles), device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)) * 9
+    carry = SimpleNamespace(xw=a, ss=ss, tiles=tiles, size=tiles * 128, eps=1e-5)
+    out = torch.empty((M, N), device=DEV, dtype=torch.float32 if mode == 0 else torch.bfloat16)
+    assert GemmBf16.get().run(a, w, out, mode, scaled=carry)
+    rinv = 1.0 / torch.sqrt(ss.double().sum(1) / (tiles * 128) + 1e-5)
+    want = (a.double() @ w.double().T) * rinv[:, None]
+    if mode == 2:
+        g, u = want[:, :N], want[:, N:]
+        want = g * torch.sigmoid(g) * u
+    tol = 1e-5 if mode == 0 else 2.0 ** -8
+    assert ((out.double() - want).abs() <= tol * (want.abs() + want.square().mean().sqrt())).all()
+    assert GemmBf16.get().take_error() == 0

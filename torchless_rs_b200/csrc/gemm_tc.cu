@@ -134,7 +134,44 @@ __device__ __forceinline__ float* tail_ssw(uint8_t* tail) { return (float*)tail 
 __device__ __forceinline__ float* tail_rinv(uint8_t* tail) { return (float*)tail + 64 + 256; }
 __device__ __forceinline__ float2* tail_cossin(uint8_t* tail) { return (float2*)(tail + TAIL_BYTES); }
 
-// 1 / sqrt(mean(x^2) + eps) of input row m from the partial sums the producer left.
+// 1 / sqrt(mean(x^2) + eps) of the `cols` input rows from m0 on, from the partial sums the producer left: a thread per row,
+// 32 sums' loads under way at once, since a round trip takes some 2 us beside the weights' stream.  For tiles of 64 tokens
+// and more.  (A warp per row is what smaller tiles take: its sum across lanes, root and quotient are a chain of 250 cycles, row
+// after row, and from 48 rows on that took longer than the product: q/k/v of 64 tokens 16.7 us, now 14.)  The sums are
+// added as a warp's exchange adds them, so the result does not depend on which of the two ran.
+__device__ __forceinline__ void rows_rinv(const GemmArgs& a, int m0, int cols, float* rinv) {
+  const int n = a.ss_in_tiles;
+#pragma unroll 1
+  for (int c = threadIdx.x; c < cols; c += 128) {
+    const float* src = a.ss_in + (size_t)(m0 + c) * n;
+    float v[32];
+#pragma unroll
+    for (int l = 0; l < 32; ++l) v[l] = 0.0f;
+    int t = 0;
+    if ((n & 3) == 0) {                 // (the sums' buffer starts on a 16-byte boundary)
+#pragma unroll 1
+      for (; t + 32 <= n; t += 32) {
+        float4 x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = __ldcg(reinterpret_cast<const float4*>(src + t) + k);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { v[4 * k] += x[k].x; v[4 * k + 1] += x[k].y; v[4 * k + 2] += x[k].z; v[4 * k + 3] += x[k].w; }
+      }
+    }
+#pragma unroll 1
+    for (; t < n; t += 32) {
+#pragma unroll
+      for (int l = 0; l < 32; ++l)
+        if (t + l < n) v[l] += __ldcg(src + t + l);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int l = 0; l < o; ++l) v[l] += v[l + o];
+    rinv[c] = 1.0f / sqrtf(v[0] / (float)a.norm_h + a.eps_in);
+  }
+}
+// The same of one row, by one thread.
 __device__ __forceinline__ float row_rinv(const GemmArgs& a, int m) {
   float ss = 0.0f;
   for (int t = 0; t < a.ss_in_tiles; ++t) ss += __ldcg(a.ss_in + (size_t)m * a.ss_in_tiles + t);
@@ -156,6 +193,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   constexpr uint32_t B_BYTES = BN * TILE_K * 2;
   constexpr uint32_t STAGE_BYTES = KS * (A_BYTES * (SWIGLU ? 2 : 1) + B_BYTES);
   constexpr uint32_t B_OFF = KS * A_BYTES * (SWIGLU ? 2 : 1);
+  constexpr bool MANY = BN >= 64;
   constexpr uint32_t ACC_COLS = BN * (SWIGLU ? 2 : 1);
   constexpr uint32_t TMEM_COLS = ACC_COLS < 32 ? 32 : ACC_COLS;   // a power of two >= 32
   constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
@@ -197,12 +235,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // ---- TMA producer.  The weights do not depend on earlier kernels, so the tiles of the
     // first stages are requested before the wait for those kernels; the activations after it.
     const int pre = n_kb < stages ? n_kb : stages;
+    uint64_t once = 0;
+    if (MANY) once = l2_evict_first();   // every weight goes to one block
+    auto load_tile = [&](uint8_t* dst, uint64_t* bar, int k, int row) {
+      if (MANY) tma_load_2d_once(dst, &tm_w, bar, k, row, once);
+      else tma_load_2d(dst, &tm_w, bar, k, row);
+    };
     auto load_w = [&](uint8_t* st, uint64_t* bar, int kb) {
 #pragma unroll
       for (int h = 0; h < KS; ++h) {
         const int k = kb * KSTEP + h * TILE_K;   // past K the tile is filled with zeros
-        tma_load_2d(st + h * A_BYTES, &tm_w, bar, k, n0);
-        if (SWIGLU) tma_load_2d(st + A_BYTES, &tm_w, bar, k, args.N + n0);
+        load_tile(st + h * A_BYTES, bar, k, n0);
+        if (SWIGLU) load_tile(st + A_BYTES, bar, k, args.N + n0);
       }
     };
     auto load_x = [&](uint8_t* st, uint64_t* bar, int kb) {
@@ -263,11 +307,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // ---- epilogue: thread = one weight row = one column of C
     pdl_wait();   // C may be read and written by earlier kernels
     TL_TRACE_RELEASED();
+    // What the way out needs besides the sums: now, while the weights stream and these warps have nothing else to do.
+    if (MANY && args.ss_in) rows_rinv(args, m0, min(BN, args.M - m0), tail_rinv(smem + (size_t)stages * STAGE_BYTES));
     if (splits > 1) {
-      // What the reduction after the cluster barrier needs and the product does not: done now,
-      // while the weights stream and these warps have nothing else to do.
       const int cols = min(BN, args.M - m0);
-      if (args.ss_in) {   // 1/rms of every token: a warp per token, the partial sums spread over its lanes
+      if (!MANY && args.ss_in) {   // 1/rms of every token: a warp per token, the partial sums spread over its lanes
         float* rinv_c = tail_rinv(smem + (size_t)stages * STAGE_BYTES);
         for (int c = warp; c < cols; c += 4) {
           float ss = 0.0f;
@@ -295,10 +339,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const int n = n0 + row;
     const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16);
     float* red = (float*)smem;   // partial tile [columns][128 rows]; the stages are free by now
-    float* rinv_s = (float*)smem;   // without a split the same place holds the row scales
+    float* rinv_s = MANY ? tail_rinv(smem + (size_t)stages * STAGE_BYTES) : (float*)smem;   // without a split (the stages are free)
     if (ok && splits == 1 && args.ss_in) {
-      for (int c = threadIdx.x; c < BN; c += 128)
-        rinv_s[c] = m0 + c < args.M ? row_rinv(args, m0 + c) : 0.0f;
+      if (!MANY)
+        for (int c = threadIdx.x; c < BN; c += 128)
+          rinv_s[c] = m0 + c < args.M ? row_rinv(args, m0 + c) : 0.0f;
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }
     if (ok) {
@@ -1419,7 +1464,7 @@ extern "C" int tl_gemm_tc_act(const void* X, int ldx, const void* W, int ldw, vo
   const size_t budget = !two_per_sm ? 224 * 1024 : (!swiglu && bn <= 32) ? 88 * 1024 : 112 * 1024;
   const long long slots = (long long)num_sms * (two_per_sm ? 2 : 1);
   int splits = 1;
-  if (tiles < slots && (two_per_sm || !ss_in)) {
+  if (tiles < slots) {
     // a power of two (clusters of 3, 5, 6 or 7 blocks do not tile the GPCs evenly, and a
     // cluster that has to wait for a second wave doubles the kernel's time), as large as
     // keeps every block resident at once
