@@ -175,6 +175,38 @@ def test_gemm_split_takes_the_products_it_is_faster_at():
     assert not takes(3, 14336, 4096) and not takes(1, 1 << 20, 4096)
 
 
+@pytest.mark.parametrize("M,N,K", [(4, 6144, 4096), (32, 6144, 4160), (33, 6144, 4096), (17, 14336, 1056), (9, 4096, 14336), (4, 300, 1000)])
+def test_gemm_split_of_few_rows_under_load(M, N, K):
+    """Products back to back whose weights come from memory at its full rate (odd and even numbers of blocks of K per split, tiles on
+    either side of 32 tokens): every launch gives the bits of the first, alone on the device, and it those of the bound above."""
+    from torchless_rs_b200.csrc import ops
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    from torchless_rs_b200.parts.runtime import Workspace
+    g, ws = GemmF32.get(), Workspace(torch.device(DEV))
+    g_takes, GemmF32.takes = GemmF32.takes, staticmethod(lambda *a: True)
+    try:
+        a = _rand((M, K), torch.float32, 5)
+        w = [_rand((2 * N, K), torch.float32, 6 + i, 1.0 / math.sqrt(K)) for i in range(3)]
+        for mode, x in ((ops.MODE_STORE_F32, lambda i: w[i][:N]), (ops.MODE_SWIGLU, lambda i: w[i])):
+            alone = []
+            for i in range(3):
+                torch.cuda.synchronize()
+                alone.append(torch.zeros((M, N), device=DEV))
+                assert g.run(a, x(i), alone[-1], mode, ws)
+            torch.cuda.synchronize()
+            many = [torch.zeros((M, N), device=DEV) for _ in range(18)]
+            for i, y in enumerate(many):
+                g.run(a, x(i % 3), y, mode, ws)
+            assert all(torch.equal(y, alone[i % 3]) for i, y in enumerate(many))
+            if mode == ops.MODE_STORE_F32:
+                for i in range(3):
+                    ref, size = a.double() @ w[i][:N].double().T, a.double().abs() @ w[i][:N].double().abs().T
+                    assert ((alone[i].double() - ref).abs() <= (24 + K / 64 + 5 * K / 4096) * 2.0 ** -23 * size).all()
+        assert g.take_error() == 0
+    finally:
+        GemmF32.takes = staticmethod(g_takes)
+
+
 def test_gemm_split_gives_what_the_cuda_core_kernel_gives_where_results_are_not_finite():
     from torchless_rs_b200.csrc import ops
     from torchless_rs_b200.csrc.gemm_f32 import GemmF32

@@ -44,12 +44,12 @@ class GemmF32:
 
     @staticmethod
     def takes(M: int, N: int, K: int) -> bool:
-        """Up to three rows the CUDA-core kernel reads the weights at the copy rate or near it (three rows of 6144 x
-        4096: 30 us here and there; four rows of 4096 x 4096 19 us there, 21 here, of 6144 x 4096 38 and 32; eight rows of
-        4096 x 1024 16 and 17, of 4096 x 2048 26 and 18).  From nine rows on it is several times slower, until the
-        launch more that is made here costs what the product does.  Below 1024 elements its sums are so short that
-        they are nearer to the exact result."""
-        least = GemmF32.LEAST if M > 8 else (6 << 20 if M > 4 else 20 << 20)
+        """Up to three rows the CUDA-core kernel reads the weights at the copy rate or near it.  Four rows (there / here, us):
+        4096 x 1024 7.0 / 9.8, 4096 x 2048 11.5 / 12.8, and where K is long, so that its blocks are few, 1024 x 4096 18.5 / 12.1,
+        4096 x 4096 21.7 / 17.8, 6144 x 4096 40.6 / 25.0, 4096 x 14336 87 / 44.  Eight rows: 4096 x 1024 15.1 / 9.9, of 4096 x
+        2048 28 / 13.  From nine rows on it is several times slower, until the launch more that is made here costs what the
+        product does.  Below 1024 elements its sums are so short that they are nearer to the exact result."""
+        least = GemmF32.LEAST if M > 8 else (6 << 20 if M > 4 else (4 << 20 if K >= 4096 else 20 << 20))
         return M >= 4 and K >= 1024 and N * K >= least
 
     def run(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, workspace) -> bool:

@@ -26,7 +26,7 @@
 //   warps 4-11  take W as stored from shared memory, a row per thread, and write its three pieces into tensor memory;
 //               two groups of four warps in turn
 //   warp 12     TMA of W as stored (four tiles in flight)
-//   warp 13     issues the instructions
+//   warp 13     issues the instructions (with few tokens warp 15 those of the leading products)
 //   warp 14     TMA of the pieces of X, which a kernel before has made
 // W's pieces are operands from tensor memory because an instruction that reads both operands from shared memory is
 // bound by that: with W's pieces there a stage of 192 tokens took 2900 cycles where its arithmetic takes 1152.  While
@@ -36,11 +36,11 @@
 // through distributed shared memory (the same bits every run).
 //
 // What bounds it: the tensor core's six products per multiply-add with many tokens (265 TFLOP/s at the bfloat16 rate;
-// 231 at 531 x 6144 x 4096, whose tiles fill one round of blocks), with few the waits and hand-overs of a stage, some
-// 700 cycles for 16 KB of W.  Measured, from the CUDA-core kernels to this: 16 tokens 356 / 282 / 826 / 1275 us -> 30 /
-// 19 / 113 / 53 us for 6144 x 4096, 4096 x 4096, 14336 x 4096 with the SiLU-gate and 4096 x 14336 (W at the copy rate: 15 /
+// 231 at 531 x 6144 x 4096, whose tiles fill one round of blocks), with few W's way through a block (struct Sp).
+// Measured, from the CUDA-core kernels to this: 16 tokens 356 / 282 / 826 / 1275 us -> 25 /
+// 18 / 94 / 45 us for 6144 x 4096, 4096 x 4096, 14336 x 4096 with the SiLU-gate and 4096 x 14336 (W at the copy rate: 15 /
 // 10 / 72 / 36), 531 tokens 1192 / 1061 / 4355 / 3705 -> 116 / 91 / 579 / 303 us, 5 tokens 75 / 40 / 200 / 287 ->
-// 31 / 21 / 112 / 53 us.
+// 25 / 18 / 92 / 44 us.
 //
 // Output modes as in gemm_generic.cu: 0 store, 1 add into C, 2 SiLU-gate (W holds N gate rows, then N up rows; a tile
 // is 64 rows of each, and the halves of the rows exchange values through shared memory), 3 store.
@@ -61,17 +61,34 @@
 #define SP_THREADS 512
 #define SP_ROWS 128             // rows of W per tile
 #define SP_BN 192               // most tokens per tile
-#define SP_GROUPS (SP_BN / 16)  // groups of 16 tokens
 #define SP_K 32                 // K elements per stage
-#define SP_XSTAGES 4
-#define SP_RAW 4                // tiles of W as stored in flight
-#define SP_WSTAGES 2            // pieces of W in tensor memory
-#define SP_XSTAGE (SP_BN * 192) // bytes of X's three pieces, each rows of 32 bfloat16
 #define SP_RAW_BYTES (SP_ROWS * SP_K * 4)
-#define SP_TAIL 256
-#define SP_TWO (SP_BN / 2)      // tiles of up to this many tokens have two accumulators for the leading sums
-#define SP_COL_SMALL SP_BN      // tensor memory columns: the leading sums, the small products' sums, W's pieces
-#define SP_COL_W (2 * SP_BN)    // 16 columns per piece
+#define SP_TAIL 512
+#define SP_FEW 32               // most tokens of a tile that leaves its room to W
+
+// What a block's memory is shared out to.  A tile of many tokens: four stages of X's pieces and of W as stored, two of W's pieces
+// in tensor memory.  A tile of few, whose time is W's way through the block: 780 cycles for 16 KB of W so, of which the
+// splitting is 700 for either group of warps and the issuing thread's waits and hand-overs 700 too (clock64 stamps); a
+// stage of 64 K-elements halves what is paid per stage and puts twice the bytes under way, and the leading products have an
+// issuing thread of their own.  4 tokens, before / now: 6144 x 4096 31 / 25 us, 4096 x 4096 20.8 / 17.8, 14336 x 4096 with the
+// SiLU-gate 113 / 92, 4096 x 14336 52 / 44; 32 tokens 33 / 26, 21 / 18.5, 117 / 96, 55 / 46.  The bits are the same.  What is left
+// of the SiLU-gate's is its second round of blocks, which fills half of the SMs.
+template <bool FEW>
+struct Sp {
+  static constexpr int BN = FEW ? SP_FEW : SP_BN, GROUPS = BN / 16;
+  static constexpr int SUBS = FEW ? 2 : 1;        // blocks of SP_K elements per stage
+  static constexpr int XSTAGES = 4, RAW = 4, WSTAGES = FEW ? 4 : 2;
+  static constexpr int XSUB = BN * 192;           // bytes of X's three pieces of SP_K elements, each rows of 32 bfloat16
+  static constexpr int TWO = FEW ? BN : BN / 2;   // tiles of up to this many tokens have two accumulators for the leading sums
+  // tensor memory columns: the leading sums, the small products' sums, W's pieces of 16 columns each
+  static constexpr int COL_SMALL = FEW ? 2 * BN : BN, COL_W = FEW ? 3 * BN : 2 * BN;
+  static constexpr int SMEM = 1024 + SUBS * (XSTAGES * XSUB + RAW * SP_RAW_BYTES) + SP_TAIL;
+  static_assert(COL_W + 48 * SUBS * WSTAGES <= 512 && XSTAGES >= WSTAGES, "W's pieces fit, and a stage of X outlives them");
+  // A group of warps takes every second stage, and a wait for a barrier's phase means that phase only to one who has waited
+  // for the one before: a slot has to stay with its group.
+  static_assert(RAW % 2 == 0 && WSTAGES % 2 == 0 && XSTAGES % 2 == 0, "a slot belongs to one group of the splitting warps");
+  static_assert(8 * (2 * RAW + 2 * XSTAGES + 5) + 16 <= SP_TAIL, "the barriers fit");
+};
 #define SP_MAX_SPLITS 8         // portable cluster size
 
 // What a stage, a round of blocks and a reduction take, in cycles, for the choice of tiles (tl_gemm_split)
@@ -267,18 +284,19 @@ __device__ __forceinline__ void sp_write(const SplitArgs& a, float (&v)[16], int
   }
 }
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool FEW>
 __global__ void __launch_bounds__(SP_THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                   const SplitArgs args) {
+  typedef Sp<FEW> P;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* raw = smem + SP_XSTAGES * SP_XSTAGE;
-  uint64_t* raw_full = (uint64_t*)(raw + SP_RAW * SP_RAW_BYTES);   // [SP_RAW]
-  uint64_t* raw_empty = raw_full + SP_RAW;                         // [SP_RAW]
-  uint64_t* full = raw_empty + SP_RAW;      // [SP_XSTAGES]: X's pieces (their bytes) and W's (a warp each) are there
-  uint64_t* empty = full + SP_XSTAGES;      // [SP_XSTAGES]: the stage's instructions are done
-  uint64_t* main_full = empty + SP_XSTAGES;   // [2]
+  uint8_t* raw = smem + P::XSTAGES * P::SUBS * P::XSUB;
+  uint64_t* raw_full = (uint64_t*)(raw + P::RAW * P::SUBS * SP_RAW_BYTES);   // [RAW]
+  uint64_t* raw_empty = raw_full + P::RAW;                         // [RAW]
+  uint64_t* full = raw_empty + P::RAW;      // [XSTAGES]: X's pieces (their bytes) and W's (a warp each) are there
+  uint64_t* empty = full + P::XSTAGES;      // [XSTAGES]: the stage's instructions are done
+  uint64_t* main_full = empty + P::XSTAGES;   // [2]
   uint64_t* main_empty = main_full + 2;       // [2]
   uint64_t* small_full = main_empty + 2;
   uint32_t* tmem_slot = (uint32_t*)(small_full + 1);
@@ -292,18 +310,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
   const int n0 = (tile / args.m_tiles) * TILE_N;
   const int k_all = (args.K + SP_K - 1) / SP_K;
   const int k_first = split * args.k_per_split;
-  const int n_k = min(args.k_per_split, k_all - k_first);   // stages of this block
+  const int n_blocks = min(args.k_per_split, k_all - k_first);       // blocks of SP_K elements
+  const int n_k = (n_blocks + P::SUBS - 1) / P::SUBS;               // stages of this block; the last may not be full
   // Stages whose leading products are summed in tensor memory.  A narrow tile has two accumulators, so that handing a
   // sum over costs the instructions nothing, and takes 64 elements (error of 1024 / 4096 / 14336 elements: 0.9e-7 / 1.1e-7 /
   // 1.7e-7; the kernel for few rows of gemm_generic.cu, which sums K / 32 in a row, 1.2e-7 / 2.1e-7 / 3.8e-7); a wide one
   // takes 256 (2.4e-7 at 4096, where the kernel for many rows is at 1.15e-6).
-  const bool two = bn <= SP_TWO;
-  const int chunk = two ? 2 : 8;
+  const bool two = bn <= P::TWO;
+  const int chunk = (two ? 2 : 8) / P::SUBS;
   auto hands_over = [&](int i) { return i == n_k - 1 || (i + 1) % chunk == 0; };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < SP_RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4); }
-    for (int s = 0; s < SP_XSTAGES; ++s) { mbar_init(&full[s], 5); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < P::RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4); }
+    for (int s = 0; s < P::XSTAGES; ++s) { mbar_init(&full[s], 5); mbar_init(&empty[s], FEW ? 2 : 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&main_full[b], 1); mbar_init(&main_empty[b], 128); }
     mbar_init(small_full, 1);
     *abort_flag = 0;
@@ -347,13 +366,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     if (args.splits > 1) cluster_sync_all();   // nobody leaves while others still read its shared memory
   };
 
-  // registers per thread: 240 + 2 x 96 + 80 = 512 = 4 x the 128 that the block was launched with
+  // Registers per thread of a tile of many tokens: 240 + 2 x 96 + 80 = 512 = 4 x the 128 that the block was launched with.  Those
+  // suffice every role of a tile of few.
   if (warp < 4) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
+    if (!FEW) asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
     const uint32_t t_main = tmem + ((uint32_t)(warp * 32) << 16);
-    float acc[SP_GROUPS][16];
+    float acc[P::GROUPS][16];
 #pragma unroll
-    for (int g = 0; g < SP_GROUPS; ++g)
+    for (int g = 0; g < P::GROUPS; ++g)
 #pragma unroll
       for (int j = 0; j < 16; ++j) acc[g][j] = 0.0f;
     bool ok = true;
@@ -365,9 +385,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
       ++sums;
       tc_fence_after();
-      const uint32_t t_sum = t_main + buf * SP_TWO;
+      const uint32_t t_sum = t_main + buf * P::TWO;
 #pragma unroll
-      for (int g = 0; g < SP_GROUPS; g += 2) {
+      for (int g = 0; g < P::GROUPS; g += 2) {
         if (g * 16 < bn) {
           uint32_t r[16], q[16];       // (the second may lie past the tile: what it holds is not used)
           tmem_ld16(t_sum + g * 16, r);
@@ -389,11 +409,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
       tc_fence_after();
       const int tokens = min(bn, args.M - m0);
 #pragma unroll
-      for (int g = 0; g < SP_GROUPS; ++g) {
+      for (int g = 0; g < P::GROUPS; ++g) {
         const int c0 = g * 16;
         if (c0 < tokens) {
           uint32_t r[16];
-          tmem_ld16(t_main + SP_COL_SMALL + c0, r);
+          tmem_ld16(t_main + P::COL_SMALL + c0, r);
           tmem_ld_wait();
           float* part = (float*)smem + (size_t)c0 * SP_ROWS + row;   // [tokens][128 rows]; X's stages are free by now
 #pragma unroll
@@ -405,100 +425,133 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     reduce();
   } else if (warp < 12) {
     // ---- W as stored -> its pieces, a row per thread, the two groups of warps in turn
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
-    const uint32_t t_w = tmem + ((uint32_t)((warp & 3) * 32) << 16) + SP_COL_W;
+    if (!FEW) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+    const uint32_t t_w = tmem + ((uint32_t)((warp & 3) * 32) << 16) + P::COL_W;
     const uint8_t* own = raw + row * 128;
     for (int i = group - 1; i < n_k; i += 2) {
-      const int r = i % SP_RAW, before = i - SP_WSTAGES;
-      bool ok = sp_wait(&raw_full[r], (i / SP_RAW) & 1, abort_flag, 1);
+      const int r = i % P::RAW, before = i - P::WSTAGES;
+      bool ok = sp_wait(&raw_full[r], (i / P::RAW) & 1, abort_flag, 1);
       if (!__all_sync(0xffffffffu, ok)) break;
-      const uint8_t* src = own + r * SP_RAW_BYTES;
-      float4 x[8];
+      const uint8_t* src = own + r * (P::SUBS * SP_RAW_BYTES);
+      const uint32_t at = t_w + (i % P::WSTAGES) * (48 * P::SUBS);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
-      uint32_t p1[16], p2[16], p3[16];
+      for (int b = 0; b < P::SUBS; ++b) {
+        float4 x[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        split3(x[c].x, x[c].y, p1[2 * c], p2[2 * c], p3[2 * c]);
-        split3(x[c].z, x[c].w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
+        for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(src + b * SP_RAW_BYTES + ((c ^ (row & 7)) << 4));
+        uint32_t p1[16], p2[16], p3[16];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          split3(x[c].x, x[c].y, p1[2 * c], p2[2 * c], p3[2 * c]);
+          split3(x[c].z, x[c].w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
+        }
+        if (b == P::SUBS - 1) {
+          __syncwarp();
+          if (lane == 0) sp_arrive(&raw_empty[r]);
+        }
+        if (b == 0) {      // the stage that had this place in tensor memory
+          ok = before < 0 || sp_wait(&empty[before % P::XSTAGES], (before / P::XSTAGES) & 1, abort_flag, 2);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st16(at + 48 * b, p1);       // (of a stage that is not full, the last block is not used)
+        tmem_st16(at + 48 * b + 16, p2);
+        tmem_st16(at + 48 * b + 32, p3);
       }
-      __syncwarp();
-      if (lane == 0) sp_arrive(&raw_empty[r]);
-      // the stage that had this place in tensor memory
-      ok = before < 0 || sp_wait(&empty[before % SP_XSTAGES], (before / SP_XSTAGES) & 1, abort_flag, 2);
-      if (!__all_sync(0xffffffffu, ok)) break;
-      tc_fence_after();
-      const uint32_t at = t_w + (i % SP_WSTAGES) * 48;
-      tmem_st16(at, p1);
-      tmem_st16(at + 16, p2);
-      tmem_st16(at + 32, p3);
+      if (!ok) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) sp_arrive(&full[i % SP_XSTAGES]);
+      if (lane == 0) sp_arrive(&full[i % P::XSTAGES]);
     }
     __syncwarp();
     reduce();
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    if (!FEW) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     if (warp == 12 && elect_one()) {
       // ---- TMA of W, which does not depend on earlier kernels
       for (int i = 0; i < n_k; ++i) {
-        const int r = i % SP_RAW, k = (k_first + i) * SP_K;
-        if (!sp_wait(&raw_empty[r], ((i / SP_RAW) & 1) ^ 1, abort_flag, 3)) break;
-        uint8_t* dst = raw + r * SP_RAW_BYTES;
-        mbar_expect_tx(&raw_full[r], SP_RAW_BYTES);
-        tma_load_2d(dst, &tm_w, &raw_full[r], k, n0);
-        if (SWIGLU) tma_load_2d(dst + SP_RAW_BYTES / 2, &tm_w, &raw_full[r], k, args.N + n0);
+        const int r = i % P::RAW;
+        if (!sp_wait(&raw_empty[r], ((i / P::RAW) & 1) ^ 1, abort_flag, 3)) break;
+        mbar_expect_tx(&raw_full[r], P::SUBS * SP_RAW_BYTES);     // (past K: zeros)
+#pragma unroll
+        for (int b = 0; b < P::SUBS; ++b) {
+          const int k = (k_first + i * P::SUBS + b) * SP_K;
+          uint8_t* dst = raw + (r * P::SUBS + b) * SP_RAW_BYTES;
+          tma_load_2d(dst, &tm_w, &raw_full[r], k, n0);
+          if (SWIGLU) tma_load_2d(dst + SP_RAW_BYTES / 2, &tm_w, &raw_full[r], k, args.N + n0);
+        }
       }
     } else if (warp == 14 && elect_one()) {
       // ---- TMA of X's pieces, all three of a stage at once
       pdl_wait();
       for (int i = 0; i < n_k; ++i) {
-        const int s = i % SP_XSTAGES;
-        if (!sp_wait(&empty[s], ((i / SP_XSTAGES) & 1) ^ 1, abort_flag, 2)) break;
-        mbar_expect_tx(&full[s], (uint32_t)bn * 192u);
-        tma_load_3d(smem + s * SP_XSTAGE, &tm_x, &full[s], (k_first + i) * SP_K, m0, 0);
+        const int s = i % P::XSTAGES;
+        if (!sp_wait(&empty[s], ((i / P::XSTAGES) & 1) ^ 1, abort_flag, 2)) break;
+        mbar_expect_tx(&full[s], (uint32_t)(bn * 192 * P::SUBS));
+#pragma unroll
+        for (int b = 0; b < P::SUBS; ++b)
+          tma_load_3d(smem + (s * P::SUBS + b) * P::XSUB, &tm_x, &full[s], (k_first + i * P::SUBS + b) * SP_K, m0, 0);
       }
-    } else if (warp == 13 && elect_one()) {
-      // ---- MMA issuer
+    } else if ((warp == 13 || (FEW && warp == 15)) && elect_one()) {
+      // ---- MMA issuer.  Of a tile of few tokens the leading products have a thread of their own: the waits for a stage and for
+      // a free accumulator cost some 250 cycles each even where nothing is left to wait for.
+      const bool smalls = !FEW || warp == 13, leading = !FEW || warp == 15;
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(SP_ROWS >> 4) << 24);
-      const uint32_t d_small = tmem + SP_COL_SMALL;
+      const uint32_t d_small = tmem + P::COL_SMALL;
       bool ok = true;
       uint32_t handed = 0;   // sums handed over so far
       bool fresh = true;     // the next leading product starts a sum
       for (int i = 0; i < n_k && ok; ++i) {
-        const int s = i % SP_XSTAGES, ws = i % SP_WSTAGES;
-        ok = sp_wait(&full[s], (i / SP_XSTAGES) & 1, abort_flag, 6);
+        const int s = i % P::XSTAGES, ws = i % P::WSTAGES;
+        ok = sp_wait(&full[s], (i / P::XSTAGES) & 1, abort_flag, 6);
         if (!ok) break;
         tc_fence_after();
-        const uint64_t x1 = smem_desc_k64(smem_u32(smem + s * SP_XSTAGE)), x2 = x1 + (uint64_t)bn * 4,
-                       x3 = x2 + (uint64_t)bn * 4;
-        const uint32_t w1 = tmem + SP_COL_W + ws * 48, w2 = w1 + 16, w3 = w2 + 16;
+        const int subs = min(P::SUBS, n_blocks - i * P::SUBS);
+        const uint64_t x0 = smem_desc_k64(smem_u32(smem + s * (P::SUBS * P::XSUB)));
+        const uint32_t w0 = tmem + P::COL_W + ws * (48 * P::SUBS);
+        if (smalls) {
 #pragma unroll
-        for (int k = 0; k < SP_K / 16; ++k) {
-          const uint64_t o = (uint64_t)k * 2;   // 32 bytes of shared memory, 8 columns of tensor memory
-          umma_bf16_ts(d_small, w3 + 8 * k, x1 + o, idesc, (i == 0 && k == 0) ? 0u : 1u);
-          umma_bf16_ts(d_small, w2 + 8 * k, x2 + o, idesc, 1u);
-          umma_bf16_ts(d_small, w1 + 8 * k, x3 + o, idesc, 1u);
-          umma_bf16_ts(d_small, w2 + 8 * k, x1 + o, idesc, 1u);
-          umma_bf16_ts(d_small, w1 + 8 * k, x2 + o, idesc, 1u);
-        }
-        const uint32_t buf = two ? handed & 1u : 0u, use = two ? handed >> 1 : handed;
-        if (fresh && use > 0) {
-          ok = sp_wait(&main_empty[buf], (use - 1) & 1, abort_flag, 8);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        const uint32_t d_main = tmem + buf * SP_TWO;
+          for (int b = 0; b < P::SUBS; ++b) {
+            if (b >= subs) break;
+            const uint64_t x1 = x0 + (uint64_t)(b * (P::XSUB >> 4)), x2 = x1 + (uint64_t)bn * 4, x3 = x2 + (uint64_t)bn * 4;
+            const uint32_t w1 = w0 + 48 * b, w2 = w1 + 16, w3 = w2 + 16;
 #pragma unroll
-        for (int k = 0; k < SP_K / 16; ++k)
-          umma_bf16_ts(d_main, w1 + 8 * k, x1 + (uint64_t)k * 2, idesc, (fresh && k == 0) ? 0u : 1u);
-        umma_commit(&empty[s]);
-        fresh = hands_over(i);
-        if (fresh) { umma_commit(&main_full[buf]); ++handed; }
+            for (int k = 0; k < SP_K / 16; ++k) {
+              const uint64_t o = (uint64_t)k * 2;   // 32 bytes of shared memory, 8 columns of tensor memory
+              umma_bf16_ts(d_small, w3 + 8 * k, x1 + o, idesc, (i == 0 && b == 0 && k == 0) ? 0u : 1u);
+              umma_bf16_ts(d_small, w2 + 8 * k, x2 + o, idesc, 1u);
+              umma_bf16_ts(d_small, w1 + 8 * k, x3 + o, idesc, 1u);
+              umma_bf16_ts(d_small, w2 + 8 * k, x1 + o, idesc, 1u);
+              umma_bf16_ts(d_small, w1 + 8 * k, x2 + o, idesc, 1u);
+            }
+          }
+        }
+        if (leading) {
+          const uint32_t buf = two ? handed & 1u : 0u, use = two ? handed >> 1 : handed;
+          if (fresh && use > 0) {
+            ok = sp_wait(&main_empty[buf], (use - 1) & 1, abort_flag, 8);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          const uint32_t d_main = tmem + buf * P::TWO;
+#pragma unroll
+          for (int b = 0; b < P::SUBS; ++b) {
+            if (b >= subs) break;
+#pragma unroll
+            for (int k = 0; k < SP_K / 16; ++k)
+              umma_bf16_ts(d_main, w0 + 48 * b + 8 * k, x0 + (uint64_t)(b * (P::XSUB >> 4) + k * 2), idesc,
+                           (fresh && b == 0 && k == 0) ? 0u : 1u);
+          }
+          umma_commit(&empty[s]);
+          fresh = hands_over(i);
+          if (fresh) { umma_commit(&main_full[buf]); ++handed; }
+        } else {
+          umma_commit(&empty[s]);
+        }
       }
-      if (ok) umma_commit(small_full);
+      if (ok && smalls) umma_commit(small_full);
     }
   }
   __syncwarp();
@@ -527,13 +580,11 @@ static SpEncodeFn sp_encode() {
   return fn;
 }
 
-#define SP_SMEM (1024 + SP_XSTAGES * SP_XSTAGE + SP_RAW * SP_RAW_BYTES + SP_TAIL)
-
-template <bool SWIGLU>
+template <bool SWIGLU, bool FEW>
 static cudaError_t sp_configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int splits) {
-  const cudaError_t set = tl_allow_smem<gemm_split_kernel<SWIGLU>>(SP_SMEM);
+  const cudaError_t set = tl_allow_smem<gemm_split_kernel<SWIGLU, FEW>>(Sp<FEW>::SMEM);
   cfg.blockDim = dim3(SP_THREADS);
-  cfg.dynamicSmemBytes = SP_SMEM;
+  cfg.dynamicSmemBytes = Sp<FEW>::SMEM;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = splits;
   attr[0].val.clusterDim.y = 1;
@@ -544,7 +595,8 @@ static cudaError_t sp_configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&a
   cfg.numAttrs = 2;
   return set;
 }
-// How many clusters of `splits` blocks run at once on this device (the GPCs differ in size: not the SMs divided by it).
+// How many clusters of `splits` blocks run at once on this device (the GPCs differ in size: not the SMs divided by it); a block
+// takes an SM either way.
 template <bool SWIGLU>
 static int sp_clusters(int splits, int num_sms) {
   static int known_on[TL_DEVICES][SP_MAX_SPLITS + 1];
@@ -558,25 +610,25 @@ static int sp_clusters(int splits, int num_sms) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     int n = 0;
-    cudaError_t e = sp_configure<SWIGLU>(cfg, attr, splits);
+    cudaError_t e = sp_configure<SWIGLU, false>(cfg, attr, splits);
     cfg.gridDim = dim3(splits);
     cfg.numAttrs = 1;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<SWIGLU>, &cfg);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<SWIGLU, false>, &cfg);
     if (e != cudaSuccess) { cudaGetLastError(); n = 0; }
     known[splits] = n > 0 ? n : -1;
   }
   return known[splits];
 }
 
-template <bool SWIGLU>
+template <bool SWIGLU, bool FEW>
 static int run_split(const CUtensorMap& tw, const CUtensorMap& tx, const SplitArgs& a, int tiles, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  cudaError_t e = sp_configure<SWIGLU>(cfg, attr, a.splits);
+  cudaError_t e = sp_configure<SWIGLU, FEW>(cfg, attr, a.splits);
   if (e != cudaSuccess) return (int)e;
   cfg.gridDim = dim3((unsigned)tiles * a.splits);
   cfg.stream = stream;
-  e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<SWIGLU>, tw, tx, a);
+  e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<SWIGLU, FEW>, tw, tx, a);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -652,7 +704,9 @@ extern "C" int tl_gemm_split(const float* X, int ldx, const float* W, int ldw, f
   const int rc = tl_launch(split_rows_kernel, dim3((unsigned)((n8 + 255) / 256 < 4096 ? (n8 + 255) / 256 : 4096)), dim3(256),
                            0, stream, X, ldx, M, K, Kp, (uint4*)scratch);
   if (rc != 0) return rc;
-  return swiglu ? run_split<true>(tw, tx, a, (int)tiles, stream) : run_split<false>(tw, tx, a, (int)tiles, stream);
+  if (a.bn <= SP_FEW)
+    return swiglu ? run_split<true, true>(tw, tx, a, (int)tiles, stream) : run_split<false, true>(tw, tx, a, (int)tiles, stream);
+  return swiglu ? run_split<true, false>(tw, tx, a, (int)tiles, stream) : run_split<false, false>(tw, tx, a, (int)tiles, stream);
 }
 
 // Reads and clears the error word that a kernel sets when one of its bounded waits ran out.  Synchronises the device.
