@@ -244,6 +244,28 @@ def test_a_cluster_of_blocks_samples_what_one_block_samples(rows, V):
                 assert a.tolist() == b.tolist(), (V, pad, t, k, p)
 
 
+@pytest.mark.parametrize("V", [300, 5000, 70000])
+def test_top_p_of_exponentials_at_the_ends_of_their_range(V):
+    """The nucleus found by digits of the exponential: thresholds where a digit carries over (1, powers of two, 32nds of them), just
+    above and below 2^-40, where weights begin, and where many small exponentials share a weight."""
+    from torchless_rs_b200.csrc import ops
+    s = ops.sampling_ops()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    ln2 = 0.6931471805599453
+    step = torch.randint(0, 41 * 32 + 40, (6, V), generator=g, device="cuda")
+    rows = [-step * (ln2 / 32), -(step // 32) * ln2, -40 * ln2 + (step % 7 - 3) * 1e-6, -30 * ln2 - (step % 64) * 1e-7,
+            torch.where(step == step.amin(), 0.0, -39.9 * ln2), -(step % 3) * 1e-7]
+    for x in rows:
+        x = x.float().contiguous()
+        x[:, V // 3] = 0.0
+        for p in (0.001, 0.5, 0.9, 0.999999, 0.9999999):
+            u = torch.rand((6,), generator=g, device="cuda")
+            a, b = (torch.full((6,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+            s.sample(x, 1.0, 0, p, u, a)
+            s.sample(x, 1.0, 0, p, u, b, walk=True)
+            assert a.tolist() == b.tolist(), p
+
+
 @pytest.mark.parametrize("rows,V,k,p,blocks", [
     (8, 131072, 0, 0.95, 8), (300, 200000, 0, 0.95, 8), (64, 131072, 50, 0.0, 4), (148, 131072, 50, 0.0, 0), (148, 131072, 50, 0.9, 4),
     (148, 200000, 0, 0.0, 0), (148, 200000, 50, 0.0, 0), (148, 200000, 50, 0.9, 0), (64, 200000, 0, 0.0, 8), (75, 200000, 50, 0.9, 8),

@@ -458,37 +458,26 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
 // fixed-point weight again in each.  Here an entry is read, divided and turned into its weight
 // once, a pass touches EPT registers, and what the blocks have to add up (histograms, sums,
 // counts of ties) goes through distributed shared memory.  Measured, temperature / top-k 50 / top-p 0.95 / both,
-// with the launch from Python: 8 rows of 131,072 entries 74 / 178 / 916 / 378 us by one block, 10 / 29 / 60 / 48 us
-// here; 8 x 32,000: 21 / 63 / 306 / 145 and 9 / 18 / 28 / 32 us; 64 x 131,072: 80 / 202 / 968 / 407 and 32 / 112 / 211 /
-// 169 us; 64 x 1000: 7 / 33 / 81 / 93 and 7 / 14 / 21 / 25 us.  What is left at top-p is the atomics of its four
-// passes on shared memory and eight cluster barriers.
+// with the launch from Python: 8 rows of 131,072 entries 74 / 178 / 916 / 378 us by one block, 10 / 29 / 35 / 48 us
+// here; 8 x 32,000: 21 / 63 / 306 / 145 and 9 / 18 / 28 / 32 us; 64 x 131,072: 80 / 202 / 968 / 407 and 32 / 110 / 86 /
+// 153 us; 64 x 1000: 7 / 33 / 81 / 93 and 7 / 14 / 21 / 25 us.  What is left at top-p is the atomics of its first
+// pass on shared memory and seven cluster barriers.
 // --------------------------------------------------------------------------
 // A block holds at most 32 x 1024 entries, so the sums of 16-bit pieces of its weights fit 32 bits, whose atomics
 // on shared memory are single instructions (64-bit ones are loops: with them a top-k pass took twice as long).
-// The first digit of a selection is little more than the exponent: a warp's lanes share a few bins, and one of them
-// adds for all that share its bin.  Later digits are spread, and every lane adds for itself (with the first form
-// there too, top-p over 8 x 131,072 took 82 us).
-template <bool SHARED_BINS>
-__device__ __forceinline__ void part_add(uint32_t (*part)[256], int bin, u64 w) {
-  if (SHARED_BINS) {
-    if (!__any_sync(0xffffffffu, bin >= 0)) return;
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    const uint32_t a = __reduce_add_sync(peers, (uint32_t)(w & 0xffffull));
-    const uint32_t b = __reduce_add_sync(peers, (uint32_t)((w >> 16) & 0xffffull));
-    const uint32_t c = __reduce_add_sync(peers, (uint32_t)(w >> 32));
-    if (bin >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) {
-      atomicAdd(&part[0][bin], a);
-      atomicAdd(&part[1][bin], b);
-      atomicAdd(&part[2][bin], c);
-    }
-  } else if (bin >= 0) {
-    atomicAdd(&part[0][bin], (uint32_t)(w & 0xffffull));
-    atomicAdd(&part[1][bin], (uint32_t)((w >> 16) & 0xffffull));
-    atomicAdd(&part[2][bin], (uint32_t)(w >> 32));
-  }
+// The first digit of top-k's selection is little more than the exponent: a warp's lanes share a few bins, and one of them
+// adds for all that share its bin.  Later digits are spread, and every lane adds for itself.  Top-p's first digit is spread
+// too: of the exponentials that have a weight, 2^-40 to 1, it is the exponent and five bits more, so that no lane has to
+// look for others of its bin (finding them and adding three sums for each group of lanes was half of the kernel), and two
+// digits of nine bits are left (8 x 131,072 64 -> 35 us, 64 x 131,072 217 -> 86, 64 x 32,000 63 -> 40).
+#define SAMPLE_BINS 1312      // of the first digit of top-p: 41 powers of two in 32 parts
+__device__ __forceinline__ void part_add(uint32_t (*part)[SAMPLE_BINS], int bin, u64 w) {
+  atomicAdd(&part[0][bin], (uint32_t)(w & 0xffffull));
+  atomicAdd(&part[1][bin], (uint32_t)((w >> 16) & 0xffffull));
+  atomicAdd(&part[2][bin], (uint32_t)(w >> 32));
 }
 template <bool SHARED_BINS>
-__device__ __forceinline__ void part_count(uint32_t (*part)[256], int bin) {
+__device__ __forceinline__ void part_count(uint32_t (*part)[SAMPLE_BINS], int bin) {
   if (SHARED_BINS) {
     if (!__any_sync(0xffffffffu, bin >= 0)) return;
     const unsigned peers = __match_any_sync(0xffffffffu, bin);
@@ -499,8 +488,8 @@ __device__ __forceinline__ void part_count(uint32_t (*part)[256], int bin) {
 }
 
 struct ClusterShared {
-  uint32_t part[3][256];// the block's histogram as it grows: counts, or weights in pieces of 16, 16 and 9 bits
-  u64 hist[2][256];     // of this block; two in turn, so that one cluster barrier per exchange is enough
+  uint32_t part[3][SAMPLE_BINS];// the block's histogram as it grows: counts, or weights in pieces of 16, 16 and 9 bits
+  u64 hist[2][SAMPLE_BINS];     // of this block; two in turn, so that one cluster barrier per exchange is enough
   u64 word[2][2];       // two numbers of this block, in turn likewise
   u64 pick[2];
   SampleShared blk;
@@ -549,36 +538,49 @@ struct RowCluster {
     for (uint32_t r = 0; r < size; ++r) m = fmaxf(m, __uint_as_float((uint32_t)ld_peer_u64(w, r)));
     return m;
   }
+  template <int BINS>
   __device__ void clear() {
-    if (threadIdx.x < 256) sm.part[0][threadIdx.x] = sm.part[1][threadIdx.x] = sm.part[2][threadIdx.x] = 0u;
+    for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS) sm.part[0][b] = sm.part[1][b] = sm.part[2][b] = 0u;
     __syncthreads();
   }
   // The highest bin at which the sum from the top bin down, on top of `above`, reaches `target` (bin 0 if none
   // does); `above` then holds what lies above that bin.  With `share` the target is that share of the whole.
+  template <int BINS>
   __device__ int choose(u64& above, u64& target, float share, bool share_given) {
+    constexpr int PER = (BINS + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
     u64* h = sm.hist[turn & 1];
     ++turn;
     __syncthreads();
-    if (threadIdx.x < 256)
-      h[threadIdx.x] = (u64)sm.part[0][threadIdx.x] + ((u64)sm.part[1][threadIdx.x] << 16) +
-                       ((u64)sm.part[2][threadIdx.x] << 32);
+    for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS)
+      h[b] = (u64)sm.part[0][b] + ((u64)sm.part[1][b] << 16) + ((u64)sm.part[2][b] << 32);
     cluster_barrier();
-    u64 v = 0;
-    if (threadIdx.x < 256)
-      for (uint32_t r = 0; r < size; ++r) v += ld_peer_u64(h + (255 - threadIdx.x), r);
+    u64 v[PER], mine = 0;      // bins from the top down
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int bin = BINS - 1 - ((int)threadIdx.x * PER + p);
+      v[p] = 0;
+      if (bin >= 0)
+        for (uint32_t r = 0; r < size; ++r) v[p] += ld_peer_u64(h + bin, r);
+      mine += v[p];
+    }
     u64 total;
-    const u64 inc = blk_scan(v, sm.blk, &total);
+    u64 run = blk_scan(mine, sm.blk, &total) - mine + above;
     if (share_given) {
       target = (u64)ceil((double)share * (double)total);
       if (target > total) target = total;
       if (target < 1ull) target = 1ull;
     }
-    if (threadIdx.x == 255) { sm.pick[0] = 0ull; sm.pick[1] = above + inc - v; }   // bin 0 unless another one takes it
-    __syncthreads();
-    if (threadIdx.x < 255 && above + inc - v < target && above + inc >= target) {
-      sm.pick[0] = (u64)(255 - threadIdx.x);
-      sm.pick[1] = above + inc - v;
+    int taken = -1;
+    u64 over = 0;
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int bin = BINS - 1 - ((int)threadIdx.x * PER + p);
+      if (bin == 0) { sm.pick[0] = 0ull; sm.pick[1] = run; }   // bin 0 unless another one takes it
+      if (bin > 0 && run < target && run + v[p] >= target) { taken = bin; over = run; }
+      run += v[p];
     }
+    __syncthreads();
+    if (taken > 0) { sm.pick[0] = (u64)taken; sm.pick[1] = over; }
     __syncthreads();
     above = sm.pick[1];
     const int bin = (int)sm.pick[0];
@@ -638,7 +640,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
     uint32_t prefix = 0u, mask = 0u;
     u64 above = 0, target = (u64)top_k;
     for (int shift = 24; shift >= 0; shift -= 8) {
-      rc.clear();
+      rc.clear<256>();
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const uint32_t k = float_key(z[e]);
@@ -646,7 +648,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
         if (shift == 24) part_count<true>(sm.part, bin);
         else part_count<false>(sm.part, bin);
       }
-      prefix |= (uint32_t)rc.choose(above, target, 0.0f, false) << shift;
+      prefix |= (uint32_t)rc.choose<256>(above, target, 0.0f, false) << shift;
       mask |= 255u << shift;
     }
     // target - above entries equal to the threshold are kept, lowest indices first
@@ -674,21 +676,27 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
   u64 S = 0;
   const bool use_p = top_p > 0.0f && top_p < 1.0f;
   if (use_p) {
-    uint32_t prefix = 0u, mask = 0u;
+    constexpr uint32_t least = 87u << 23;      // 2^-40: what lies below has no weight
     u64 above = 0, target = 0;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      rc.clear();
+    rc.clear<SAMPLE_BINS>();
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+      const uint32_t k = __float_as_uint(z[e]);
+      if (k >= least) part_add(sm.part, (int)((k - least) >> 18), weight(z[e]));
+    }
+    uint32_t prefix = (uint32_t)rc.choose<SAMPLE_BINS>(above, target, top_p, true);
+#pragma unroll
+    for (int shift = 9; shift >= 0; shift -= 9) {
+      rc.clear<512>();
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const uint32_t k = __float_as_uint(z[e]);
-        const u64 w = weight(z[e]);
-        const int bin = (w != 0ull && (k & mask) == prefix) ? (int)((k >> shift) & 255u) : -1;
-        if (shift == 24) part_add<true>(sm.part, bin, w);
-        else part_add<false>(sm.part, bin, w);
+        if (k >= least && (k - least) >> (shift + 9) == prefix)
+          part_add(sm.part, (int)((k - least) >> shift & 511u), weight(z[e]));
       }
-      prefix |= (uint32_t)rc.choose(above, target, top_p, shift == 24) << shift;
-      mask |= 255u << shift;
+      prefix = prefix << 9 | (uint32_t)rc.choose<512>(above, target, 0.0f, false);
     }
+    prefix += least;
     // small exponentials share a weight: ties are ties of the weight
     const u64 thr = weight(__uint_as_float(prefix));
     u64 over = 0, equal = 0, total, before, all, over_all;
