@@ -1008,3 +1008,10 @@ def test_gemm_scales_rows_by_their_partial_sums(M, N, K, mode, tiles):
     tol = 1e-5 if mode == 0 else 2.0 ** -8
     assert ((out.double() - want).abs() <= tol * (want.abs() + want.square().mean().sqrt())).all()
     assert GemmBf16.get().take_error() == 0
+
+
+@pytest.mark.parametrize("M", [129, 256, 300])
+@pytest.mark.parametrize("N,K,mode,tiles", [(4096, 4096, 2, 32), (2048, 1024, 2, 40), (4096, 4096, 0, 32), (1024, 14336, 0, 33), (4096, 512, 3, 3)])
+def test_gemm_scales_rows_of_more_than_128_tokens(M, N, K, mode, tiles):
+    """The same for tiles of 256 tokens, one and two of them, where the plain product has room for K splits and the SiLU-gate has not."""
+    test_gemm_scales_rows_by_their_partial_sums(M, N, K, mode, tiles)

@@ -1249,14 +1249,27 @@ static bool make_map(CUtensorMap* map, const void* ptr, long long rows, long lon
   return true;
 }
 
+// A block of the few-token kernel: bytes of a stage, of what follows the stages, and the stages that a budget of shared memory holds.
+static size_t few_stage(int bn, bool swiglu) {
+  return (swiglu ? 1 : 2) * ((size_t)TILE_N * TILE_K * 2 * (swiglu ? 2 : 1) + (size_t)bn * TILE_K * 2);
+}
+static size_t few_tail(int bn, bool swiglu) { return TAIL_BYTES + ((bn == 16 && !swiglu) ? TAIL_ROPE_BYTES : 0); }
+static int few_stages(int bn, bool swiglu, size_t budget) {
+  const int n = (int)((budget - 1024 - few_tail(bn, swiglu)) / few_stage(bn, swiglu));
+  return n > 8 ? 8 : n;
+}
+// With K split a block's partial tile, 32-bit, takes the place of its stages.  The SiLU-gate's of 256 tokens (256 KB beside 192 KB
+// of stages) does not fit: such a tile is never split.
+static bool partial_tile_fits(int bn, bool swiglu, size_t budget) {
+  return (size_t)(swiglu ? 2 : 1) * bn * TILE_N * sizeof(float) <= few_stages(bn, swiglu, budget) * few_stage(bn, swiglu);
+}
+
 template <int BN, bool SWIGLU>
 static int launch(const CUtensorMap& tw, const CUtensorMap& tx, GemmArgs a, int splits,
                   size_t smem_budget, cudaStream_t stream) {
-  const size_t stage = (SWIGLU ? 1 : 2) * ((size_t)TILE_N * TILE_K * 2 * (SWIGLU ? 2 : 1) + (size_t)BN * TILE_K * 2);
-  const size_t tail = TAIL_BYTES + ((BN == 16 && !SWIGLU) ? TAIL_ROPE_BYTES : 0);
-  int stages = (int)((smem_budget - 1024 - tail) / stage);
-  stages = stages > 8 ? 8 : stages;
-  if (stages < 2) return -2;
+  const size_t stage = few_stage(BN, SWIGLU), tail = few_tail(BN, SWIGLU);
+  const int stages = few_stages(BN, SWIGLU, smem_budget);
+  if (stages < 2 || (splits > 1 && !partial_tile_fits(BN, SWIGLU, smem_budget))) return -2;
   a.stages = stages;
   const size_t smem = 1024 + stages * stage + tail;
   static size_t configured = 0;   // per instantiation
@@ -1411,6 +1424,58 @@ static int clusters_at_once(int bn, bool swiglu, int s, size_t smem, int per_sm)
   return v < 0 ? v : v * per_sm;
 }
 
+// The few-token kernel's way with a product: tokens per tile, splits of K and the blocks of K (of a stage's elements) in each, and the
+// shared memory of a block.
+struct FewPlan { int bn, splits, kb_per_split; long long tiles; size_t budget; };
+static FewPlan few_plan(int M, int N, int K, bool swiglu, int num_sms) {
+  const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  const int n_tiles = (N + TILE_N - 1) / TILE_N, m_tiles = (M + bn - 1) / bn;
+  const long long tiles = (long long)n_tiles * m_tiles;
+  const int kb_total = (K + TILE_K - 1) / TILE_K;
+  // stages of the few-token kernel: 128 K-elements, 64 with the SiLU-gate's two matrices
+  const int kstep64 = swiglu ? 1 : 2;
+  const int kb_np = (K + TILE_K * kstep64 - 1) / (TILE_K * kstep64);
+  // two blocks per SM fit while the token tile is small
+  const bool two_per_sm = bn <= 64;
+  // small token tiles leave room for the blocks of the next kernel, which fetch their first
+  // weight tiles while this kernel drains
+  const size_t budget = !two_per_sm ? 224 * 1024 : (!swiglu && bn <= 32) ? 88 * 1024 : 112 * 1024;
+  const long long slots = (long long)num_sms * (two_per_sm ? 2 : 1);
+  int splits = 1;
+  if (tiles < slots && partial_tile_fits(bn, swiglu, budget)) {
+    // a power of two (clusters of 3, 5, 6 or 7 blocks do not tile the GPCs evenly, and a
+    // cluster that has to wait for a second wave doubles the kernel's time), as large as
+    // keeps every block resident at once
+    while (splits * 2 <= MAX_SPLITS && tiles * splits * 2 <= slots && splits * 2 <= kb_np / 2)
+      splits *= 2;
+    // 3, 5, 6 or 7 splits where that puts more blocks on the GPU and all their clusters are sure to run
+    // at once (measured at 8 tokens: 5120 x 14336 in 6 splits 26.0 us, in 4 splits 28.9 us, in 7, which
+    // do not all fit, 36.6 us; 6144 x 5120 in 5 splits 12.5 us, in 4 splits 13.5 us, in 6 19.5 us)
+    if (m_tiles == 1) {
+      for (int sp = MAX_SPLITS - 1; sp > splits; --sp) {
+        if ((sp & (sp - 1)) == 0 || tiles * sp > slots || sp > kb_np / 2) continue;
+        if (tiles <= clusters_at_once(bn, swiglu, sp, budget, two_per_sm ? 2 : 1)) { splits = sp; break; }
+      }
+    }
+    // token tiles of 128: the reduction of so wide a tile costs about as much as 16 K-blocks of 64
+    // elements (measured: q/k/v at 128 tokens 19.0 us unsplit, 17.0 us in two splits), so the split has
+    // to save more than that
+    if (!two_per_sm && ((kb_np + splits - 1) / splits) * kstep64 + 16 >= kb_total) splits = 1;
+  }
+  int kb_per_split = (kb_np + splits - 1) / splits;
+  splits = (kb_np + kb_per_split - 1) / kb_per_split;   // no empty split
+  return {bn, splits, kb_per_split, tiles, budget};
+}
+// Tokens per tile, splits of K, and the bytes of a block's partial tile (0 without splits) and of the stages where it lies, for the tests.
+extern "C" void tl_gemm_tc_plan(int M, int N, int K, int mode, int num_sms, int* bn, int* splits, int* partial, int* room) {
+  const bool swiglu = mode == MODE_SWIGLU;
+  const FewPlan p = few_plan(M, N, K, swiglu, num_sms);
+  *bn = p.bn;
+  *splits = p.splits;
+  *partial = p.splits > 1 ? (swiglu ? 2 : 1) * p.bn * TILE_N * (int)sizeof(float) : 0;
+  *room = (int)(few_stages(p.bn, swiglu, p.budget) * few_stage(p.bn, swiglu));
+}
+
 // What the caller passes to have rotation and cache write done by the q/k/v product.
 struct TlRopeArgs {
   void* q_out; void* k_pages; void* v_pages;
@@ -1450,42 +1515,11 @@ extern "C" int tl_gemm_tc_act(const void* X, int ldx, const void* W, int ldw, vo
       !(act == ACT_CLAMPED_GLU && mode == MODE_SWIGLU))
     return -1;
   const bool swiglu = mode == MODE_SWIGLU;
-  int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-  const int n_tiles = (N + TILE_N - 1) / TILE_N, m_tiles = (M + bn - 1) / bn;
-  const long long tiles = (long long)n_tiles * m_tiles;
-  const int kb_total = (K + TILE_K - 1) / TILE_K;
-  // stages of the few-token kernel: 128 K-elements, 64 with the SiLU-gate's two matrices
-  const int kstep64 = swiglu ? 1 : 2;
-  const int kb_np = (K + TILE_K * kstep64 - 1) / (TILE_K * kstep64);
-  // two blocks per SM fit while the token tile is small
-  const bool two_per_sm = bn <= 64;
-  // small token tiles leave room for the blocks of the next kernel, which fetch their first
-  // weight tiles while this kernel drains
-  const size_t budget = !two_per_sm ? 224 * 1024 : (!swiglu && bn <= 32) ? 88 * 1024 : 112 * 1024;
-  const long long slots = (long long)num_sms * (two_per_sm ? 2 : 1);
-  int splits = 1;
-  if (tiles < slots) {
-    // a power of two (clusters of 3, 5, 6 or 7 blocks do not tile the GPCs evenly, and a
-    // cluster that has to wait for a second wave doubles the kernel's time), as large as
-    // keeps every block resident at once
-    while (splits * 2 <= MAX_SPLITS && tiles * splits * 2 <= slots && splits * 2 <= kb_np / 2)
-      splits *= 2;
-    // 3, 5, 6 or 7 splits where that puts more blocks on the GPU and all their clusters are sure to run
-    // at once (measured at 8 tokens: 5120 x 14336 in 6 splits 26.0 us, in 4 splits 28.9 us, in 7, which
-    // do not all fit, 36.6 us; 6144 x 5120 in 5 splits 12.5 us, in 4 splits 13.5 us, in 6 19.5 us)
-    if (m_tiles == 1) {
-      for (int sp = MAX_SPLITS - 1; sp > splits; --sp) {
-        if ((sp & (sp - 1)) == 0 || tiles * sp > slots || sp > kb_np / 2) continue;
-        if (tiles <= clusters_at_once(bn, swiglu, sp, budget, two_per_sm ? 2 : 1)) { splits = sp; break; }
-      }
-    }
-    // token tiles of 128: the reduction of so wide a tile costs about as much as 16 K-blocks of 64
-    // elements (measured: q/k/v at 128 tokens 19.0 us unsplit, 17.0 us in two splits), so the split has
-    // to save more than that
-    if (!two_per_sm && ((kb_np + splits - 1) / splits) * kstep64 + 16 >= kb_total) splits = 1;
-  }
-  int kb_per_split = (kb_np + splits - 1) / splits;
-  splits = (kb_np + kb_per_split - 1) / kb_per_split;   // no empty split
+  const FewPlan few = few_plan(M, N, K, swiglu, num_sms);
+  const int kb_total = (K + TILE_K - 1) / TILE_K, kb_per_split = few.kb_per_split, splits = few.splits;
+  const long long tiles = few.tiles;
+  const size_t budget = few.budget;
+  int bn = few.bn;
   const int pairs = num_sms / 2;
   const int pair_n = swiglu ? 128 : 256;
   // token tiles of equal width, a multiple of 32 (300 tokens: two tiles of 160, not 256 + 44)
