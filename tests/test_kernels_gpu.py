@@ -1015,3 +1015,21 @@ def test_gemm_scales_rows_by_their_partial_sums(M, N, K, mode, tiles):
 def test_gemm_scales_rows_of_more_than_128_tokens(M, N, K, mode, tiles):
     """The same for tiles of 256 tokens, one and two of them, where the plain product has room for K splits and the SiLU-gate has not."""
     test_gemm_scales_rows_by_their_partial_sums(M, N, K, mode, tiles)
+
+
+@pytest.mark.parametrize("off", [1, 2, 3])
+@pytest.mark.parametrize("M", [9, 32, 64, 100])
+def test_gemm_takes_partial_sums_off_a_16_byte_boundary(M, off):
+    """A carry's sums may be a view that starts anywhere: read 16 or 4 bytes at a time, they are added in the same order."""
+    from types import SimpleNamespace
+    from torchless_rs_b200.csrc.gemm_bf16 import GemmBf16
+    N, K, tiles = 512, 1024, 36
+    a, w = _rand((M, K), torch.bfloat16, 1), _rand((N, K), torch.bfloat16, 2) * 0.05
+    room = torch.rand((M * tiles + 4,), device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)) * 9
+    outs = []
+    for ss in (room[off:off + M * tiles].view(M, tiles), room[off:off + M * tiles].clone().view(M, tiles)):
+        out = torch.empty((M, N), device=DEV)
+        carry = SimpleNamespace(xw=a, ss=ss, tiles=tiles, size=tiles * 128, eps=1e-5)
+        assert GemmBf16.get().run(a, w, out, 0, scaled=carry)
+        outs.append(out)
+    assert torch.equal(*outs) and outs[0].isfinite().all()

@@ -138,7 +138,8 @@ __device__ __forceinline__ float2* tail_cossin(uint8_t* tail) { return (float2*)
 // 32 sums' loads under way at once, since a round trip takes some 2 us beside the weights' stream.  For tiles of 64 tokens
 // and more.  (A warp per row is what smaller tiles take: its sum across lanes, root and quotient are a chain of 250 cycles, row
 // after row, and from 48 rows on that took longer than the product: q/k/v of 64 tokens 16.7 us, now 14.)  The sums are
-// added as a warp's exchange adds them, so the result does not depend on which of the two ran.
+// added as a warp's exchange adds them: the bits that smaller tiles have with K split (without a split they add a row's sums in
+// order, `row_rinv`).
 __device__ __forceinline__ void rows_rinv(const GemmArgs& a, int m0, int cols, float* rinv) {
   const int n = a.ss_in_tiles;
 #pragma unroll 1
@@ -148,7 +149,7 @@ __device__ __forceinline__ void rows_rinv(const GemmArgs& a, int m0, int cols, f
 #pragma unroll
     for (int l = 0; l < 32; ++l) v[l] = 0.0f;
     int t = 0;
-    if ((n & 3) == 0) {                 // (the sums' buffer starts on a 16-byte boundary)
+    if ((n & 3) == 0 && ((uintptr_t)a.ss_in & 15) == 0) {       // every row starts on a 16-byte boundary
 #pragma unroll 1
       for (; t + 32 <= n; t += 32) {
         float4 x[8];
