@@ -458,9 +458,9 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
 // fixed-point weight again in each.  Here an entry is read, divided and turned into its weight
 // once, a pass touches EPT registers, and what the blocks have to add up (histograms, sums,
 // counts of ties) goes through distributed shared memory.  Measured, temperature / top-k 50 / top-p 0.95 / both,
-// with the launch from Python: 8 rows of 131,072 entries 74 / 178 / 916 / 378 us by one block, 10 / 29 / 35 / 48 us
-// here; 8 x 32,000: 21 / 63 / 306 / 145 and 9 / 18 / 28 / 32 us; 64 x 131,072: 80 / 202 / 968 / 407 and 32 / 110 / 86 /
-// 153 us; 64 x 1000: 7 / 33 / 81 / 93 and 7 / 14 / 21 / 25 us.  What is left at top-p is the atomics of its first
+// with the launch from Python: 8 rows of 131,072 entries 74 / 178 / 916 / 378 us by one block, 10 / 29 / 30 / 47 us
+// here; 8 x 32,000: 21 / 63 / 306 / 145 and 9 / 18 / 22 / 32 us; 64 x 131,072: 80 / 202 / 968 / 407 and 31 / 100 / 78 /
+// 138 us; 64 x 1000: 7 / 33 / 81 / 93 and 7 / 13 / 13 / 20 us.  What is left at top-p is the atomics of its first
 // pass on shared memory and seven cluster barriers.
 // --------------------------------------------------------------------------
 // A block holds at most 32 x 1024 entries, so the sums of 16-bit pieces of its weights fit 32 bits, whose atomics
@@ -469,15 +469,18 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, float temperature
 // adds for all that share its bin.  Later digits are spread, and every lane adds for itself.  Top-p's first digit is spread
 // too: of the exponentials that have a weight, 2^-40 to 1, it is the exponent and five bits more, so that no lane has to
 // look for others of its bin (finding them and adding three sums for each group of lanes was half of the kernel), and two
-// digits of nine bits are left (8 x 131,072 64 -> 35 us, 64 x 131,072 217 -> 86, 64 x 32,000 63 -> 40).
+// digits of nine bits are left (8 x 131,072 69 -> 32 us, 64 x 131,072 250 -> 79, 64 x 32,000 67 -> 23, launched by a graph).  Its many
+// bins are what small vocabularies pay for after top-k, whose few entries never crowded a bin: the sums of the
+// blocks come over two bins to a load (8 x 32,000, both: 32 us with four digits of eight bits, 37 with a load per bin, 32).
 #define SAMPLE_BINS 1312      // of the first digit of top-p: 41 powers of two in 32 parts
-__device__ __forceinline__ void part_add(uint32_t (*part)[SAMPLE_BINS], int bin, u64 w) {
+template <int ROOM>
+__device__ __forceinline__ void part_add(uint32_t (*part)[ROOM], int bin, u64 w) {
   atomicAdd(&part[0][bin], (uint32_t)(w & 0xffffull));
   atomicAdd(&part[1][bin], (uint32_t)((w >> 16) & 0xffffull));
   atomicAdd(&part[2][bin], (uint32_t)(w >> 32));
 }
-template <bool SHARED_BINS>
-__device__ __forceinline__ void part_count(uint32_t (*part)[SAMPLE_BINS], int bin) {
+template <bool SHARED_BINS, int ROOM>
+__device__ __forceinline__ void part_count(uint32_t (*part)[ROOM], int bin) {
   if (SHARED_BINS) {
     if (!__any_sync(0xffffffffu, bin >= 0)) return;
     const unsigned peers = __match_any_sync(0xffffffffu, bin);
@@ -487,9 +490,10 @@ __device__ __forceinline__ void part_count(uint32_t (*part)[SAMPLE_BINS], int bi
   }
 }
 
+template <int ROOM>
 struct ClusterShared {
-  uint32_t part[3][SAMPLE_BINS];// the block's histogram as it grows: counts, or weights in pieces of 16, 16 and 9 bits
-  u64 hist[2][SAMPLE_BINS];     // of this block; two in turn, so that one cluster barrier per exchange is enough
+  uint32_t part[3][ROOM];// the block's histogram as it grows: counts, or weights in pieces of 16, 16 and 9 bits
+  alignas(16) u64 hist[2][ROOM];  // of this block; two in turn, so that one cluster barrier per exchange is enough
   u64 word[2][2];       // two numbers of this block, in turn likewise
   u64 pick[2];
   SampleShared blk;
@@ -506,11 +510,18 @@ __device__ __forceinline__ u64 ld_peer_u64(const u64* local, uint32_t rank) {
   asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(r) : "memory");
   return v;
 }
+__device__ __forceinline__ void ld_peer_2u64(const u64* local, uint32_t rank, u64& x, u64& y) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(r) : "memory");
+}
 
 // What the blocks of a row exchange.  `turn` counts the exchanges of either kind: a buffer is written
 // again two exchanges later, when the barrier between has seen every block past its reads.
+template <int ROOM>
 struct RowCluster {
-  ClusterShared& sm;
+  ClusterShared<ROOM>& sm;
   uint32_t rank, size;
   int turn;
 
@@ -540,47 +551,57 @@ struct RowCluster {
   }
   template <int BINS>
   __device__ void clear() {
-    for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS) sm.part[0][b] = sm.part[1][b] = sm.part[2][b] = 0u;
+    if constexpr (BINS <= SAMPLE_THREADS) {
+      if (threadIdx.x < BINS) sm.part[0][threadIdx.x] = sm.part[1][threadIdx.x] = sm.part[2][threadIdx.x] = 0u;
+    } else {
+      for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS) sm.part[0][b] = sm.part[1][b] = sm.part[2][b] = 0u;
+    }
     __syncthreads();
   }
   // The highest bin at which the sum from the top bin down, on top of `above`, reaches `target` (bin 0 if none
   // does); `above` then holds what lies above that bin.  With `share` the target is that share of the whole.
   template <int BINS>
   __device__ int choose(u64& above, u64& target, float share, bool share_given) {
-    constexpr int PER = (BINS + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
+    constexpr int PER = BINS <= SAMPLE_THREADS ? 1 : 2;       // bins per thread, from the top bin down
+    static_assert(BINS <= 2 * SAMPLE_THREADS && (PER == 1 || BINS % 2 == 0), "a thread has one bin or a pair of them");
     u64* h = sm.hist[turn & 1];
     ++turn;
     __syncthreads();
     for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS)
       h[b] = (u64)sm.part[0][b] + ((u64)sm.part[1][b] << 16) + ((u64)sm.part[2][b] << 32);
     cluster_barrier();
-    u64 v[PER], mine = 0;      // bins from the top down
-#pragma unroll
-    for (int p = 0; p < PER; ++p) {
-      const int bin = BINS - 1 - ((int)threadIdx.x * PER + p);
-      v[p] = 0;
-      if (bin >= 0)
-        for (uint32_t r = 0; r < size; ++r) v[p] += ld_peer_u64(h + bin, r);
-      mine += v[p];
-    }
+    const bool has = (int)threadIdx.x * PER < BINS;
+    const int low = BINS - PER - (int)threadIdx.x * PER;      // the lower one of a thread's bins
+    u64 v = 0, lower = 0;
+    if (has)
+      for (uint32_t r = 0; r < size; ++r) {
+        if constexpr (PER == 1) {
+          v += ld_peer_u64(h + low, r);
+        } else {
+          u64 x, y;
+          ld_peer_2u64(h + low, r, x, y);
+          lower += x;
+          v += y;
+        }
+      }
     u64 total;
-    u64 run = blk_scan(mine, sm.blk, &total) - mine + above;
+    const u64 over = above + blk_scan(v + lower, sm.blk, &total) - v - lower;
     if (share_given) {
       target = (u64)ceil((double)share * (double)total);
       if (target > total) target = total;
       if (target < 1ull) target = 1ull;
     }
-    int taken = -1;
-    u64 over = 0;
-#pragma unroll
-    for (int p = 0; p < PER; ++p) {
-      const int bin = BINS - 1 - ((int)threadIdx.x * PER + p);
-      if (bin == 0) { sm.pick[0] = 0ull; sm.pick[1] = run; }   // bin 0 unless another one takes it
-      if (bin > 0 && run < target && run + v[p] >= target) { taken = bin; over = run; }
-      run += v[p];
-    }
+    if (has && low == 0) { sm.pick[0] = 0ull; sm.pick[1] = over + (PER == 2 ? v : 0ull); }   // bin 0 unless another one takes it
     __syncthreads();
-    if (taken > 0) { sm.pick[0] = (u64)taken; sm.pick[1] = over; }
+    if (has && over < target) {
+      if (low + PER > 1 && over + v >= target) {
+        sm.pick[0] = (u64)(low + PER - 1);
+        sm.pick[1] = over;
+      } else if (PER == 2 && low > 0 && over + v < target && over + v + lower >= target) {
+        sm.pick[0] = (u64)low;
+        sm.pick[1] = over + v;
+      }
+    }
     __syncthreads();
     above = sm.pick[1];
     const int bin = (int)sm.pick[0];
@@ -589,15 +610,16 @@ struct RowCluster {
   }
 };
 
-template <int EPT>
+template <int EPT, bool TOP_K, bool TOP_P>
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float temperature, int top_k,
                       float top_p, const float* __restrict__ uniform, int* __restrict__ out) {
-  __shared__ ClusterShared sm;
+  constexpr int ROOM = TOP_P ? SAMPLE_BINS : 256;
+  __shared__ ClusterShared<ROOM> sm;
   uint32_t rank, size;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-  RowCluster rc{sm, rank, size, 0};
+  RowCluster<ROOM> rc{sm, rank, size, 0};
   const int tid = threadIdx.x;
   const int r = blockIdx.x / size;
   const float* row = logits + (size_t)r * ld;
@@ -634,13 +656,13 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
   }
 
   // ---- top-k: key of the k-th largest scaled logit by radix selection
-  const bool use_k = top_k > 0 && top_k < V;
+  const bool use_k = TOP_K && top_k > 0 && top_k < V;
   uint32_t dropped = 0;                           // bit e: not among the k largest
-  if (use_k) {
+  if constexpr (TOP_K) if (use_k) {
     uint32_t prefix = 0u, mask = 0u;
     u64 above = 0, target = (u64)top_k;
     for (int shift = 24; shift >= 0; shift -= 8) {
-      rc.clear<256>();
+      rc.template clear<256>();
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const uint32_t k = float_key(z[e]);
@@ -648,7 +670,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
         if (shift == 24) part_count<true>(sm.part, bin);
         else part_count<false>(sm.part, bin);
       }
-      prefix |= (uint32_t)rc.choose<256>(above, target, 0.0f, false) << shift;
+      prefix |= (uint32_t)rc.template choose<256>(above, target, 0.0f, false) << shift;
       mask |= 255u << shift;
     }
     // target - above entries equal to the threshold are kept, lowest indices first
@@ -674,27 +696,27 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
   // ---- top-p: the largest weight w such that the weights of w and above reach the share, by radix selection on
   // the bits of exp(z - max), which are in the order of the weights
   u64 S = 0;
-  const bool use_p = top_p > 0.0f && top_p < 1.0f;
-  if (use_p) {
+  const bool use_p = TOP_P && top_p > 0.0f && top_p < 1.0f;
+  if constexpr (TOP_P) if (use_p) {
     constexpr uint32_t least = 87u << 23;      // 2^-40: what lies below has no weight
     u64 above = 0, target = 0;
-    rc.clear<SAMPLE_BINS>();
+    rc.template clear<SAMPLE_BINS>();
 #pragma unroll
     for (int e = 0; e < EPT; ++e) {
       const uint32_t k = __float_as_uint(z[e]);
       if (k >= least) part_add(sm.part, (int)((k - least) >> 18), weight(z[e]));
     }
-    uint32_t prefix = (uint32_t)rc.choose<SAMPLE_BINS>(above, target, top_p, true);
-#pragma unroll
+    uint32_t prefix = (uint32_t)rc.template choose<SAMPLE_BINS>(above, target, top_p, true);
+#pragma unroll (EPT == 4 ? 1 : 2)      // (top-k at 8 x 32,000: 17.7 us with the loop, 18.9 without)
     for (int shift = 9; shift >= 0; shift -= 9) {
-      rc.clear<512>();
+      rc.template clear<512>();
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const uint32_t k = __float_as_uint(z[e]);
         if (k >= least && (k - least) >> (shift + 9) == prefix)
           part_add(sm.part, (int)((k - least) >> shift & 511u), weight(z[e]));
       }
-      prefix = prefix << 9 | (uint32_t)rc.choose<512>(above, target, 0.0f, false);
+      prefix = prefix << 9 | (uint32_t)rc.template choose<512>(above, target, 0.0f, false);
     }
     prefix += least;
     // small exponentials share a weight: ties are ties of the weight
@@ -747,7 +769,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, float tem
   cluster_barrier();   // no block leaves while another reads its shared memory
 }
 
-template <int EPT>
+template <int EPT, bool TOP_K, bool TOP_P>
 static int launch_sample_cluster(int blocks_per_row, const float* logits, int ld, int rows, int V, float temperature,
                                  int top_k, float top_p, const float* uniform, int* out, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
@@ -763,7 +785,7 @@ static int launch_sample_cluster(int blocks_per_row, const float* logits, int ld
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<EPT>, logits, ld, V, temperature, top_k, top_p,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<EPT, TOP_K, TOP_P>, logits, ld, V, temperature, top_k, top_p,
                                      uniform, out);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -821,12 +843,17 @@ extern "C" int tl_sample(const float* logits, int ld, int rows, int V, float tem
   int blocks, per;
   if (!sample_plan(rows, V, top_k, top_p, &blocks, &per))
     return tl_sample_walk(logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream);
-#define SAMPLE_CLUSTER(EPT_) \
-  return launch_sample_cluster<EPT_>(blocks, logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream)
-  if (per <= 4) SAMPLE_CLUSTER(4);
-  if (per <= 8) SAMPLE_CLUSTER(8);
-  if (per <= 16) SAMPLE_CLUSTER(16);
-  SAMPLE_CLUSTER(32);
+#define SAMPLE_CLUSTER(EPT_, K_, P_) \
+  return launch_sample_cluster<EPT_, K_, P_>(blocks, logits, ld, rows, V, temperature, top_k, top_p, uniform, out, stream)
+  // A kernel that can do everything, but for two: the registers that a digit's sums take from top-k and temperature cost top-k 4 % at
+  // 16 entries per thread (8 x 70,000: 30.8 us, 29.9 without top-p) and temperature 3 % at 32 (64 x 131,072: 31.6 and 30.8).
+  const bool use_k = top_k > 0 && top_k < V, use_p = top_p > 0.0f && top_p < 1.0f;
+  if (per <= 4) SAMPLE_CLUSTER(4, true, true);
+  if (per <= 8) SAMPLE_CLUSTER(8, true, true);
+  if (per <= 16 && use_p) SAMPLE_CLUSTER(16, true, true);
+  if (per <= 16) SAMPLE_CLUSTER(16, true, false);
+  if (use_k || use_p) SAMPLE_CLUSTER(32, true, true);
+  SAMPLE_CLUSTER(32, false, false);
 #undef SAMPLE_CLUSTER
 }
 
