@@ -186,3 +186,33 @@ def test_a_step_is_as_near_to_64_bits_as_on_the_cached_vectors(heads, lens, wind
     a, b = (float((x - want).norm() / want.norm()) for x in (formed, latent))
     print(f"error against 64 bits: formed {a:.3e}, latent {b:.3e}")
     assert a <= 1.2 * b and a < 2e-2, (a, b)
+
+
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("size", [0.3, 1.0, 3.0, 10.0])
+def test_weights_are_rounded_relative_to_the_running_maximum(size, sink):
+    """Flat and peaked softmaxes, from rounded queries, keys and values on.  The kernel rounds the weights relative to the maximum so
+    far, so that of the key that stands out not at all, and the result; a plain restatement of that in 64 bits has the same
+    error but for weights that 32-bit scores round the other way (some 2^-16 of the result: under a hundredth of 2^-10)."""
+    lens, heads, rot, scale = [1000], 3, 64, 192 ** -0.5
+    x, rank = _inputs(lens, heads, rot, 0, int(10 * size), size)
+    got, _ = _run(x, rank, lens, heads, rot, 0, None, None, sink, scale)
+    want, _ = _reference(x, rank, lens, heads, rot, 0, None, None, sink, scale)
+    T, f = lens[0], torch.tensor(scale * 1.4426950408889634, dtype=F32, device="cuda")
+    q = (x["q"][:, :heads * (DIM + rot)].view(T, heads, DIM + rot) * f).to(BF).to(F64)
+    kv, r = x["kv"].to(F64).view(T, 2, heads, DIM), x["latents"].to(F64)[:, rank:]
+    same = torch.empty_like(want)
+    for h in range(heads):
+        s = q[:, h, :DIM] @ kv[:, 0, h].T + q[:, h, DIM:] @ r.T
+        s.masked_fill_(torch.ones((T, T), dtype=torch.bool, device="cuda").triu(1), -float("inf"))
+        m = torch.full((T, 1), -float("inf"), dtype=F64, device="cuda")
+        l, o = torch.zeros_like(m), torch.zeros((T, DIM), dtype=F64, device="cuda")
+        for k in range(0, T, 64):
+            new = torch.maximum(m, s[:, k:k + 64].amax(1, keepdim=True))
+            p, a = torch.exp2(s[:, k:k + 64] - new).to(BF).to(F64), torch.exp2(m - new)
+            o, l, m = o * a + p @ kv[k:k + 64, 1, h], l * a + p.sum(1, keepdim=True), new
+        if sink:
+            l = l + torch.exp2(x["sink"][h].double() * 1.4426950408889634 - m)
+        same[:, h] = (o / l).to(BF).to(F64)
+    a, b = (float((y.double() - want).norm() / want.norm()) for y in (got, same))
+    assert a <= 1.01 * b, (a, b)

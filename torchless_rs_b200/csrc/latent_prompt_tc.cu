@@ -7,7 +7,7 @@
 // 192 + 128, and forming them costs two small products per token, which a prompt's queries share.  They are formed from
 // the step's own latents, which `latent_prep` leaves in token order, so a step that continues a sequence, and would have
 // to form the keys of all it has seen, runs on the kernels of [c | r].  Measured, 16 heads, one prompt, the whole mixer on
-// [c | r] / here: 300 tokens 107 / 72 us, 2048 393 / 154, 4096 963 / 283; of that this kernel 21, 49 and 116 us.
+// [c | r] / here: 300 tokens 107 / 72 us, 2048 393 / 154, 4096 963 / 283; of that this kernel 22, 55 and 129 us.
 //
 // A block owns 128 consecutive queries of one head and walks over the keys they see, 64 at a time:
 //   warps 0-3  softmax, a row per thread
@@ -20,8 +20,7 @@
 // that share their keys: 68 us against 52 then, because at 2048 tokens the longest blocks are left alone.)  The queries are turned,
 // scaled and rounded on their way into shared memory, and O / l leaves through it, gated, a warp per row.
 //
-// The reference of the exponentials moves only when a score exceeds it by 2^8, so that O is rarely rescaled; l sums the
-// weights as they were rounded, so that where few keys count their rounding cancels.
+// l sums the weights as they were rounded, so that where few keys count their rounding cancels.
 //
 // Every wait on an mbarrier is bounded; when a bound is hit the block records a code in tl_latent_prompt_error, stops,
 // frees its tensor memory and returns.
@@ -355,8 +354,7 @@ latent_prompt_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_
       const int pos = first + min(r, rows - 1);
       const int lo = a.window > 0 ? max(pos - a.window + 1, 0) : 0;
       const uint32_t lanes = (uint32_t)(warp * 32) << 16, t_o = tmem + LP_COL_O + lanes;
-      float m = a.sink != nullptr ? a.sink[h] * 1.4426950408889634f : -INFINITY;
-      float l = a.sink != nullptr ? 1.0f : 0.0f;     // a sink is in the denominator and has no value
+      float m = -INFINITY, l = 0.0f;
       bool ok = true;
       for (int i = 0; i < n_ch; ++i) {
         const uint32_t u = (uint32_t)i & 1u, t_s = tmem + u * LP_KEYS + lanes;
@@ -380,7 +378,11 @@ latent_prompt_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_
         float mx = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 32; ++j) mx = lp_max3(mx, __uint_as_float(sa[j]), __uint_as_float(sb[j]));
-        const float m_new = (mx > m + 8.0f || m == -INFINITY) ? fmaxf(m, mx) : m;
+        // The reference is the running maximum itself: the weight of the key that stands out is then 1, which bfloat16 holds
+        // exactly.  (One that moves only when a score exceeds it by 2^8 spares most of the rescaling of O, 49.6 us instead of
+        // 55.0 for 2048 tokens, but rounds that weight too: where few keys count the weights' part of the error is 1.8 times
+        // as large, and a result 7 % further from 64 bits.)
+        const float m_new = fmaxf(m, mx);
         const float ref = m_new == -INFINITY ? 0.0f : m_new;
         // (a row without a token, or that sees no key so far, must not ask for rescaling)
         const float alpha = valid && m_new != -INFINITY ? exp2f(m - ref) : 1.0f;
@@ -401,7 +403,7 @@ latent_prompt_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_
         float sum, sum_hi;
         lp_unpack2(lp_add2(sum_a, sum_b), sum, sum_hi);
         l = l * alpha + (sum + sum_hi);
-        // O is touched only when some row's reference moved; every warp waits for P(i - 1) . V(i - 1) on every chunk all
+        // O is touched only when some row's maximum moved; every warp waits for P(i - 1) . V(i - 1) on every chunk all
         // the same, so that no phase of its barrier is taken for another
         if (i > 0) {
           ok = lp_wait(o_done, (uint32_t)(i - 1) & 1u, abort_flag, 7);
@@ -436,7 +438,8 @@ latent_prompt_tc_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_
       asm volatile("bar.sync 2, 128;" ::: "memory");
       if (__all_sync(0xffffffffu, ok)) {
         tc_fence_after();
-        const float inv = 1.0f / l;
+        // a sink is in the denominator and has no value
+        const float inv = 1.0f / (a.sink != nullptr ? l + exp2f(a.sink[h] * 1.4426950408889634f - m) : l);
         float* row = o_s + r * LP_OLD;
 #pragma unroll 1
         for (int c = 0; c < LP_VDIM; c += 32) {
