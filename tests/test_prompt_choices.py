@@ -42,3 +42,13 @@ def test_latent_attention_forms_keys_for_long_steps_that_start_their_sequences(p
     from types import SimpleNamespace
     assert latent_bf16.LatentPrompt.takes(SimpleNamespace(is_decode=decode, past_lens=past, new_lens=new)) == formed
     assert not latent_bf16.LatentPrompt.takes(SimpleNamespace(is_decode=False))     # a step whose lengths nobody says
+
+
+@pytest.mark.parametrize("new,window,formed", [
+    ([512] + [1] * 127, None, False), ([600] + [1] * 99, None, True), ([600] + [1] * 99, 64, False), ([600] + [1] * 99, 600, True),
+    ([2048] + [1] * 200, 256, False), ([2048] + [1] * 200, 4096, True), ([600] + [14] * 60, 64, True), ([2048], 1, True)])
+def test_latent_attention_forms_keys_of_many_short_sequences_only_where_that_was_faster(new, window, formed):
+    """A sequence of a few tokens costs its block here what one of 128 costs, and with a window the other kernels have little to do."""
+    from types import SimpleNamespace
+    step = SimpleNamespace(is_decode=False, past_lens=[0] * len(new), new_lens=new)
+    assert latent_bf16.LatentPrompt.takes(step, window) == formed

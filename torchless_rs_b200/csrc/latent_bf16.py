@@ -129,14 +129,22 @@ class LatentPrompt:
     # rounds at other places, which moves logits by 5e-3 of their size either way and a greedy choice in forty: short
     # prompts, where that buys some 30 us a layer, keep the numbers that they and the steps after them always had.
     FROM_TOKENS = 512
+    # Tokens per sequence up to which a step does not run here, without a window and with one of fewer tokens than the longest
+    # sequence: every sequence costs a block of 128 rows per head, however few it fills, and a window leaves the other kernels little
+    # to do.  600 tokens and 99 single ones (7 a sequence), the mixer on the cached vectors / here, us: 16 heads 201 / 150, with a
+    # window of 64 130 / 150; 32 heads 275 / 246, with a window of 256 232 / 239; 512 and 127 (5): 174 / 157, 32 heads 230 / 261, 64 heads
+    # 404 / 477; 2048 and 200 (11): 897 / 411, window 64 276 / 396, 256 358 / 400; 600 and 60 of 10 (20): 208 / 137, window 64 160 / 136.
+    SCATTERED, SCATTERED_WINDOW = 6, 16
 
     @classmethod
-    def takes(cls, batch) -> bool:
+    def takes(cls, batch, window: Optional[int] = None) -> bool:
         """Whether a step's keys are the ones it brings (every sequence starts with it), and enough of them."""
         past = getattr(batch, "past_lens", None)
         if batch.is_decode or past is None or any(past):
             return False
-        return max(batch.new_lens) >= cls.FROM_TOKENS and sum(batch.new_lens) > 4 * len(past)
+        longest = max(batch.new_lens)
+        scattered = cls.SCATTERED_WINDOW if window is not None and window < longest else cls.SCATTERED
+        return longest >= cls.FROM_TOKENS and sum(batch.new_lens) > scattered * len(past)
 
     def run(self, q: torch.Tensor, turn: Optional[torch.Tensor], kv: torch.Tensor, latents: torch.Tensor, out: torch.Tensor,
             gate: Optional[torch.Tensor], sink: Optional[torch.Tensor], batch, heads: int, rank: int, rot: int, dims: int,

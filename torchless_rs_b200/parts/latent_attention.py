@@ -184,7 +184,7 @@ class LatentAttention:
         dkv = s[:, n_q:g_off]
         cq = ws.get("latent_cq", (T, q_rank), rt.act_dtype) if q_rank else None
         gate = s[:, g_off:g_off + self.gate_rows] if self.gate_rows else None
-        forms = self.prompt is not None and self.prompt.takes(batch)
+        forms = self.prompt is not None and self.prompt.takes(batch, self.window)
         flat = ws.get("latent_flat", (T, rank + rot), rt.act_dtype) if forms else None
         turn = ws.get("latent_turn", (T, self.rot_dims), torch.float32) if forms and self.rot_dims else None
         o.latent_prep(s[:, :q_rank] if q_rank else None, dkv, self.norm_q, self.norm_c, self.eps, cq, c.pages,
