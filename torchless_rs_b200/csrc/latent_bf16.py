@@ -122,12 +122,14 @@ class LatentPrompt:
     def fits(cls, dim: int, vdim: int, rank: int, rot: int) -> bool:
         return dim == cls.DIM and vdim == cls.VDIM and rank % 8 == 0 and rot % 8 == 0 and rot <= cls.MOST_ROT
 
-    # Tokens of the longest sequence from which a step runs here.  The whole mixer with the keys formed / on the cached vectors, 16
-    # heads, query latent of 768, us: one prompt of 100 tokens 61 / 84, 300 72 / 107, 512 94 / 134, 1000 107 / 181, 2048 154 / 393,
-    # 4096 283 / 963; 16 prompts of 100 120 / 199, 64 of 3 95 / 92 (a block per head and 128 tokens of a sequence costs some
-    # 8 us however few of its rows are filled); 32 heads, 2048 tokens 298 / 773.  It would be faster from some 20 tokens on, but
-    # rounds at other places, which moves logits by 5e-3 of their size either way and a greedy choice in forty: short
-    # prompts, where that buys some 30 us a layer, keep the numbers that they and the steps after them always had.
+    # Tokens of the longest sequence from which a step runs here.  The whole mixer on the cached vectors / with the keys formed, 16
+    # heads, query latent of 768, us: one prompt of 100 tokens 85 / 62, 300 107 / 73, 512 134 / 94, 1000 180 / 109, 2048 390 / 157,
+    # 4096 960 / 289; 16 prompts of 100 198 / 120, 64 of 3 91 / 96; 32 heads, 2048 tokens 695 / 232.  So the line is not one of time
+    # (that would be near 20 tokens).  The two ways round at other places, which moves logits by 5e-3 of their size either
+    # way and a greedy choice in forty, and where it buys some 30 us a layer a step keeps the numbers that it has always had.  That
+    # is said of steps, not of prompts: a short prompt fed beside a long one is computed here, and one that is fed in pieces on
+    # the cached vectors from the second piece on, so its roundings depend on how it is fed (as they do, more finely,
+    # through the products, whose tiles and K splits go by a step's tokens).
     FROM_TOKENS = 512
     # Tokens per sequence up to which a step does not run here, without a window and with one of fewer tokens than the longest
     # sequence: every sequence costs a block of 128 rows per head, however few it fills, and a window leaves the other kernels little

@@ -7,7 +7,7 @@
 // 192 + 128, and forming them costs two small products per token, which a prompt's queries share.  They are formed from
 // the step's own latents, which `latent_prep` leaves in token order, so a step that continues a sequence, and would have
 // to form the keys of all it has seen, runs on the kernels of [c | r].  Measured, 16 heads, one prompt, the whole mixer on
-// [c | r] / here: 300 tokens 107 / 72 us, 2048 393 / 154, 4096 963 / 283; of that this kernel 22, 55 and 129 us.
+// [c | r] / here: 300 tokens 107 / 73 us, 2048 390 / 157, 4096 960 / 289; of that this kernel 22, 55 and 128 us.
 //
 // A block owns 128 consecutive queries of one head and walks over the keys they see, 64 at a time:
 //   warps 0-3  softmax, a row per thread
