@@ -216,3 +216,22 @@ def test_weights_are_rounded_relative_to_the_running_maximum(size, sink):
         same[:, h] = (o / l).to(BF).to(F64)
     a, b = (float((y.double() - want).norm() / want.norm()) for y in (got, same))
     assert a <= 1.01 * b, (a, b)
+
+
+def test_the_values_matrix_is_held_once():
+    """The matrix that forms keys and values ends with W_uv, which the other steps multiply by: no second copy of it."""
+    from torchless_rs_b200.config.spec import PartSpec
+    from torchless_rs_b200.parts import latent_attention
+    from torchless_rs_b200.parts.runtime import Runtime
+    rt, heads, rank = Runtime("cuda:0", BF), 3, 72
+    for vdim, shared in ((DIM, True), (64, False)):        # heads with values of 64 are not formed
+        spec = PartSpec("latent_attention", {"hidden_size": 256, "heads": heads, "dim": DIM, "rot_dim": 64, "vdim": vdim, "q_rank": 96,
+                                             "kv_rank": rank, "window": None, "eps": 1e-5})
+        part = latent_attention.LatentAttention(spec, "m", rt, None)
+        w = {n: torch.randn(tuple(t.shape), device="cuda").to(BF) for n, t in part.expected_tensors(spec, "m").items()}
+        part.load(w)
+        assert torch.equal(part.w_uv, w["m.uv"].view(heads, vdim, rank)) and part.w_uv.is_contiguous()
+        assert (part.prompt is not None) == shared
+        if shared:
+            assert part.w_uv.untyped_storage().data_ptr() == part.w_kv.untyped_storage().data_ptr()
+            assert torch.equal(part.w_kv, torch.cat([w["m.uk"], w["m.uv"]]))

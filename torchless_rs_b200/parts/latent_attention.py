@@ -142,12 +142,14 @@ class LatentAttention:
         # per head, transposed: the query's plain part is multiplied by W_uk,h^T
         uk = weights[f"{p}.uk"].reshape(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uk_t = rt.matrix(uk)                                          # [heads, rank, dim]
-        self.w_uv = rt.matrix(weights[f"{p}.uv"].reshape(self.heads, self.vdim, self.rank))
         self.w_o = rt.matrix(weights[f"{p}.o"])
         self.prompt = None
         if not rt.is_f32 and latent_bf16.LatentPrompt.fits(self.dim, self.vdim, self.rank, self.rot):
             self.prompt = latent_bf16.LatentPrompt.get()
             self.w_kv = rt.stack([weights[f"{p}.uk"], weights[f"{p}.uv"]])
+            self.w_uv = self.w_kv[self.heads * self.dim:].view(self.heads, self.vdim, self.rank)    # (held once)
+        else:
+            self.w_uv = rt.matrix(weights[f"{p}.uv"].reshape(self.heads, self.vdim, self.rank))
         f32 = lambda t: t.to(device=rt.device, dtype=torch.float32).contiguous()
         self.norm_q = f32(weights[f"{p}.dq.norm"]) if self.q_rank else None
         self.norm_c = f32(weights[f"{p}.dkv.norm"])
