@@ -22,3 +22,18 @@ def test_a_partial_tile_fits_where_the_stages_lay(mode, sms):
                 split |= {bn.value} if splits.value > 1 else set()
     if sms >= 132:      # the sweep reaches splits of every tile that has room for them
         assert split == {16, 32, 64, 128} | ({256} if mode == 0 else set())
+
+
+def test_32_bit_products_on_tensor_cores_go_by_rows_and_sizes_in_order():
+    """More rows, columns or longer sums never send a 32-bit product back to the CUDA cores, and both sides of the line at K = 3072."""
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    takes, sizes = GemmF32.takes, (64, 255, 341, 342, 512, 1024, 2048, 3071, 3072, 4095, 4096, 4736, 6144, 14336)
+    for M in (1, 3, 4, 5, 8, 9, 100):
+        for N in sizes:
+            for K in sizes:
+                if takes(M, N, K):
+                    assert takes(M + 1, N, K) and takes(M, N + 1, K) and takes(M, N, K + 1), (M, N, K)
+    for M in (4, 5, 8):
+        assert takes(M, 1024, 4096) and takes(M, 512, 3072) and takes(M, 4096, 4032) and takes(M, 342, 3072)
+        assert not takes(M, 341, 3072) and not takes(M, 1024, 3071) and not takes(M, 255, 4096)
+    assert not takes(4, 4736, 2560) and takes(5, 4736, 2560) and not takes(3, 4096, 4096)

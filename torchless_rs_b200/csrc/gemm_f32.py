@@ -44,12 +44,15 @@ class GemmF32:
 
     @staticmethod
     def takes(M: int, N: int, K: int) -> bool:
-        """Up to three rows the CUDA-core kernel reads the weights at the copy rate or near it.  Four rows (there / here, us):
-        4096 x 1024 7.0 / 9.8, 4096 x 2048 11.5 / 12.8, and where K is long, so that its blocks are few, 1024 x 4096 18.5 / 12.1,
-        4096 x 4096 21.7 / 17.8, 6144 x 4096 40.6 / 25.0, 4096 x 14336 87 / 44.  Eight rows: 4096 x 1024 15.1 / 9.9, of 4096 x
-        2048 28 / 13.  From nine rows on it is several times slower, until the launch more that is made here costs what the
-        product does.  Below 1024 elements its sums are so short that they are nearer to the exact result."""
-        least = GemmF32.LEAST if M > 8 else (6 << 20 if M > 4 else (4 << 20 if K >= 4096 else 20 << 20))
+        """Up to three rows the CUDA-core kernel reads the weights at the copy rate or near it.  With four and more its time goes by
+        K once its blocks are few, so from K = 3072 on all but the smallest products run here.  Four rows (there / here, us): 1024 x
+        3072 14.7 / 10.8, 4096 x 3072 16.3 / 14.9, 512 x 4096 19.0 / 11.7, 6144 x 4096 40 / 25, 4096 x 14336 87 / 44; at K = 2560 1024
+        columns 12.5 / 10.3 and 4736 14.3 / 15.8, at 2048 10.2 / 9.7 and 4096 11.4 / 13.2, at 1024 6.2 / 8.6 and 4096 7.1 / 9.9.  Below,
+        four rows run here from 20 M weights on.  Five to eight are faster here at nearly every size that was measured (8 rows of 4096 x
+        1024 15.0 / 9.9, 512 x 2048 25 / 9.4); below K = 3072 their line stays at 6 M weights, where smaller products have always
+        had the other kernel's bits.  From nine rows on that one is several times slower, until the launch more that is made here
+        costs what the product does.  Below 1024 elements its sums are so short that they are nearer to the exact result."""
+        least = GemmF32.LEAST if M > 8 or K >= 3072 else (6 << 20 if M > 4 else 20 << 20)
         return M >= 4 and K >= 1024 and N * K >= least
 
     def run(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, workspace) -> bool:
