@@ -237,7 +237,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // first stages are requested before the wait for those kernels; the activations after it.
     const int pre = n_kb < stages ? n_kb : stages;
     uint64_t once = 0;
-    if (MANY) once = l2_evict_first();   // every weight goes to one block
+    if (MANY) once = l2_evict_first();   // (a weight goes to one block, but with a folded norm beyond 256 tokens)
     auto load_tile = [&](uint8_t* dst, uint64_t* bar, int k, int row) {
       if (MANY) tma_load_2d_once(dst, &tm_w, bar, k, row, once);
       else tma_load_2d(dst, &tm_w, bar, k, row);

@@ -35,10 +35,14 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// A load of bytes that nobody reads again soon (weights of a step of few tokens): they leave the L2 cache before anything
-// else does.  Loaded without the hint, the weights of one layer of 7B sizes sweep the cache of what is small and used at once,
-// the activations between two products and the kernels' own instructions.  A chain of the four products of six such
-// layers (437 MB each), without / with the hint: 64 tokens 97 / 94 us a layer, 100 tokens 119 / 110 us.
+// A load of bytes that nobody reads again soon (weights of a step of 33 to 256 tokens, each for one block): they leave the L2
+// cache before anything else does.  Loaded without the hint, the weights of a layer sweep the cache of what is small and used at once,
+// the activations between two products and the kernels' own instructions.  A chain of a layer's four products, us a layer
+// without / with the hint: 4096 wide (437 MB) at 48 tokens 92 / 87, at 64 97 / 90, at 100 117 / 105, at 128 121 / 109; 4096 x 14336
+// alone at 129 and 256 tokens 34.9 / 33.9 and 38.6 / 37.3; six layers 2048 wide (554 MB) 40.7 / 40.6 at 64 tokens and 62.2 / 59.5 at
+// 100.  What pays for it is a model that stays in the cache whole: one such layer over and over (92 MB) 38.1 / 40.4 and 58.1 /
+// 59.5.  The hint for matrices from 40 MB on alone would spare that one (38.8, 56.8), but three layers 3072 wide, whose
+// smaller matrices then sweep the cache, take 59.2 and 72.3 instead of 55.4 and 67.9.
 __device__ __forceinline__ uint64_t l2_evict_first() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
