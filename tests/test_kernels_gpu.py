@@ -1033,3 +1033,19 @@ def test_gemm_takes_partial_sums_off_a_16_byte_boundary(M, off):
         assert GemmBf16.get().run(a, w, out, 0, scaled=carry)
         outs.append(out)
     assert torch.equal(*outs) and outs[0].isfinite().all()
+
+
+@pytest.mark.parametrize("M,N,K,few", [(33, 2048, 2048, True), (64, 2048, 5632, True), (96, 1024, 4096, True), (33, 6144, 4096, False),
+                                       (64, 4096, 4096, False), (48, 14336, 4096, False), (32, 2048, 2048, True), (64, 8192, 1056, False)])
+def test_gemm_split_takes_narrow_tiles_where_they_were_faster(M, N, K, few):
+    """33 to 96 rows: several tiles of up to 32 for small matrices, whose blocks idle otherwise, one wide tile for the others."""
+    import ctypes
+    from torchless_rs_b200.csrc.gemm_f32 import GemmF32
+    g = GemmF32.get()
+    if g.lib is None:
+        g._load()
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("drawn for 148 SMs")
+    v = [ctypes.c_int() for _ in range(3)]
+    g.lib.tl_gemm_split_plan(M, N, K, 0, 148, *(ctypes.byref(x) for x in v))
+    assert (v[0].value <= 32) == few, [x.value for x in v]

@@ -61,7 +61,7 @@
 #define SP_THREADS 512
 #define SP_ROWS 128             // rows of W per tile
 #define SP_BN 192               // most tokens per tile
-#define SP_K 32                 // K elements per stage
+#define SP_K 32                 // K elements per block of a stage
 #define SP_RAW_BYTES (SP_ROWS * SP_K * 4)
 #define SP_TAIL 512
 #define SP_FEW 32               // most tokens of a tile that leaves its room to W
@@ -91,9 +91,13 @@ struct Sp {
 };
 #define SP_MAX_SPLITS 8         // portable cluster size
 
-// What a stage, a round of blocks and a reduction take, in cycles, for the choice of tiles (tl_gemm_split)
+// What a block of SP_K elements, a round of blocks and a reduction take, in cycles, for the choice of tiles (sp_plan).  All ways of
+// cutting twelve products of 4 to 96 tokens were timed: up to 32 tokens the choice was the fastest each time; with 750 cycles for the narrow
+// tiles too, which were the tiles of many tokens' when this was drawn, 33 to 96 tokens of small matrices took wide tiles that
+// are slower (us, then / now): 2048 x 2048 at 64 tokens 13.7 / 12.3, 2048 x 5632 22.2 / 20.8, 1024 x 4096 15.6 / 14.2.
 #define SP_COST_TOKEN 6.5
 #define SP_COST_STAGE 750.0
+#define SP_COST_FEW 500.0
 #define SP_COST_ROUND 8000.0
 #define SP_COST_REDUCE 40.0
 
@@ -175,7 +179,7 @@ struct SplitArgs {
   const float* W;
   float* C;
   int ldx, ldw, ldc, M, N, K, mode, bn, m_tiles;
-  int splits, k_per_split;   // K in stages
+  int splits, k_per_split;   // K in blocks of SP_K
 };
 
 __device__ __forceinline__ float sp_silu(float g) { return g / (1.0f + expf(-g)); }
@@ -632,9 +636,10 @@ static int run_split(const CUtensorMap& tw, const CUtensorMap& tx, const SplitAr
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// Tokens per tile and splits of K into `a`: the choice that takes the fewest cycles.  A stage takes SP_COST_TOKEN per token
-// for its instructions and SP_COST_STAGE for splitting W at the least; a round of blocks SP_COST_ROUND besides, and
-// the reduction over a cluster SP_COST_REDUCE per token of the tile.  Returns the tiles along N.
+// Tokens per tile and splits of K into `a`: the choice that takes the fewest cycles.  A block of SP_K elements takes SP_COST_TOKEN
+// per token for its instructions and SP_COST_STAGE for splitting W at the least, SP_COST_FEW in tiles of few tokens, whose stages are
+// paid for whole; a round of blocks SP_COST_ROUND besides, and the reduction over a cluster SP_COST_REDUCE per token of the
+// tile.  Returns the tiles along N.
 static int sp_plan(SplitArgs& a, int num_sms) {
   const bool swiglu = a.mode == MODE_SWIGLU;
   const int n_tiles = (a.N + (swiglu ? 64 : 128) - 1) / (swiglu ? 64 : 128), k_all = (a.K + SP_K - 1) / SP_K, M = a.M;
@@ -647,8 +652,10 @@ static int sp_plan(SplitArgs& a, int num_sms) {
       if (at_once <= 0 || (sp > 1 && tiles > at_once)) continue;    // K is split only over blocks that would idle
       const int per = (k_all + sp - 1) / sp;
       if (per * (sp - 1) >= k_all) continue;                        // no empty split
-      const double stage = SP_COST_TOKEN * bn > SP_COST_STAGE ? SP_COST_TOKEN * bn : SP_COST_STAGE;
-      const double cost = (double)((tiles + at_once - 1) / at_once) * (per * stage + SP_COST_ROUND) +
+      const bool few = bn <= SP_FEW;
+      const double least = few ? SP_COST_FEW : SP_COST_STAGE, block = SP_COST_TOKEN * bn > least ? SP_COST_TOKEN * bn : least;
+      const int paid = few ? (per + Sp<true>::SUBS - 1) / Sp<true>::SUBS * Sp<true>::SUBS : per;
+      const double cost = (double)((tiles + at_once - 1) / at_once) * (paid * block + SP_COST_ROUND) +
                           (sp > 1 ? SP_COST_REDUCE * bn : 0.0);
       if (best < 0.0 || cost < best) { best = cost; a.bn = bn; a.splits = sp; a.k_per_split = per; }
     }
