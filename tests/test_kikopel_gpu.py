@@ -591,3 +591,37 @@ def test_latent_attention_of_prompts_keeps_unseen_values_out(heads, n, new, wind
         assert LatentBf16.get().take_error() == 0
     finally:
         LatentBf16.FROM_ROWS = keep
+
+
+def test_prompts_fed_whole_in_pieces_and_beside_others_at_sizes_whose_keys_are_formed():
+    """Heads of 128 + 64 with values of 128: a prompt of 512 tokens and more forms its keys in one step, in pieces only the first one
+    of such a length does, and a short prompt does beside a long one; then decoding.  Each way rounds at other places, and
+    each is within the type's bound of the plain implementation."""
+    from kikopel_tiny import config, latent, recur, with_ff
+    from torchless_rs_b200.csrc import ops
+    km = KModel(config(128, 211, [with_ff(latent(3, 128, 64, 128, 96, 136, window=None, dims=48), 160), with_ff(recur(2, 32, 32), None),
+                                  with_ff(latent(2, 128, 32, 128, 64, 128, window=300), 96)]), "bfloat16", seed=17, max_tokens=4096)
+    rng = np.random.default_rng(23)
+    long, short = tokens_of(rng, 650, 211), tokens_of(rng, 45, 211)
+    formed = lambda: ops.launch_counts().get("latent_prompt_tc", 0)
+    for cuts, n in (([640], 2), ([320, 320], 0), ([560, 80], 2), ([511, 129], 0), ([512, 128], 2)):
+        s, before = km.engine.start_sequences(1), formed()
+        got = _feed(km, s[0], long, cuts)
+        assert formed() - before == n, cuts
+        km.engine.end_sequences(s)
+        assert_close(got, km.reference(long), "bfloat16", f"cut {cuts}")
+    s, before = km.engine.start_sequences(2), formed()
+    out = km.step_np(s, [long[:600], short[:40]], "all")
+    assert formed() - before == 2
+    rows = [[out[:600]], [out[600:]]]
+    for t in range(5):
+        out = km.step_np(s, [[long[600 + t]], [short[40 + t]]], "last")
+        rows[0].append(out[:1])
+        rows[1].append(out[1:])
+    km.engine.end_sequences(s)
+    for toks, r in ((long[:605], rows[0]), (short, rows[1])):
+        assert_close(np.concatenate(r), km.reference(toks), "bfloat16", f"{len(toks)} tokens beside another prompt")
+    s, before = km.engine.start_sequences(1), formed()
+    assert_close(_feed(km, s[0], short, [40]), km.reference(short), "bfloat16", "alone")
+    assert formed() == before
+    km.engine.check_kernels()

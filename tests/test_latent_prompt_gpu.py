@@ -235,3 +235,129 @@ def test_the_values_matrix_is_held_once():
         if shared:
             assert part.w_uv.untyped_storage().data_ptr() == part.w_kv.untyped_storage().data_ptr()
             assert torch.equal(part.w_kv, torch.cat([w["m.uk"], w["m.uv"]]))
+
+
+def _mixer(heads, rot, dims, pairing, ramp, q_rank, window, gate, lens, seed):
+    """A mixer with rotation, bound to pages that hold each sequence and one token more; its weights in 64 bits."""
+    from torchless_rs_b200.config.spec import PartSpec
+    from torchless_rs_b200.parts import latent_attention
+    from torchless_rs_b200.parts.position import RotaryHalfSplit, RotaryInterleaved
+    from torchless_rs_b200.parts.runtime import Runtime
+    rt, W, rank = Runtime("cuda:0", BF), 256, 136
+    scaling = {"kind": "ramp", "factor": 4.0, "original": 256, "fast": 32, "slow": 1} if ramp else None
+    position = {"half_split": RotaryHalfSplit, "interleaved": RotaryInterleaved}[pairing](
+        PartSpec("rope", {"head_dim": dims, "theta": 10000.0, "scaling": scaling}), rt)
+    spec = PartSpec("latent_attention", {"hidden_size": W, "heads": heads, "dim": DIM, "rot_dim": rot, "vdim": DIM, "q_rank": q_rank,
+                                         "kv_rank": rank, "window": window, "eps": 1e-5, "rot_dims": dims, "gate": gate})
+    part = latent_attention.LatentAttention(spec, "m", rt, position)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = {n: (torch.randn(tuple(t.shape), device="cuda", generator=g) * (t.shape[1] ** -0.5 if len(t.shape) == 2 else 1.0)).to(BF)
+         for n, t in part.expected_tensors(spec, "m").items()}
+    part.load(w)
+    need = [-(-(n + 1) // 64) for n in lens]
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    for b in range(len(lens)):
+        table[b, :need[b]] = torch.arange(sum(need[:b]), sum(need[:b + 1]))
+    part.bind_cache(SimpleNamespace(pages=torch.zeros((sum(need), 64, rank + rot), device="cuda", dtype=BF), page_table=table.cuda()))
+    xs = [torch.randn((n + 1, W), device="cuda", generator=g).to(BF) for n in lens]
+    return part, {k[2:]: v.double() for k, v in w.items()}, xs
+
+
+def _mixer_in_64_bits(part, d, x, pairing):
+    n, H, rot, dims, rank = x.shape[0], part.heads, part.rot, part.rot_dims, part.rank
+    rms = lambda t: t / torch.sqrt((t * t).mean(-1, keepdim=True) + 1e-5)
+    ang = torch.arange(n, device="cuda").double()[:, None] * part.position.inv_freq.double()
+    c, s = ang.cos() * part.amplitude, ang.sin() * part.amplitude
+
+    def turned(t):                                     # [n, ..., rot]
+        cs, sn = (a.view((n,) + (1,) * (t.dim() - 2) + (-1,)) for a in (c, s))
+        t = t.clone()
+        i = torch.arange(dims // 2, device="cuda")
+        a, b = (i, i + dims // 2) if pairing == "half_split" else (2 * i, 2 * i + 1)
+        u, v = t[..., a].clone(), t[..., b].clone()
+        t[..., a], t[..., b] = u * cs - v * sn, v * cs + u * sn
+        return t
+    h = x.double()
+    q = ((rms(h @ d["dq"].T) * d["dq.norm"]) @ d["uq"].T if "dq" in d else h @ d["q"].T).view(n, H, DIM + rot)
+    q = torch.cat([q[..., :DIM], turned(q[..., DIM:])], -1)
+    down = h @ d["dkv"].T
+    lat = rms(down[:, :rank]) * d["dkv.norm"]
+    k = torch.cat([(lat @ d["uk"].T).view(n, H, DIM), turned(down[:, rank:])[:, None].expand(n, H, rot)], -1)
+    sc = torch.einsum("thd,shd->hts", q, k) * part.scale
+    i = torch.arange(n, device="cuda")
+    sc.masked_fill_((i[:, None] < i) | ((i[:, None] - i >= part.window) if part.window else (i[:, None] < i)), -float("inf"))
+    y = torch.einsum("hts,shd->thd", torch.softmax(sc, -1), (lat @ d["uv"].T).view(n, H, DIM))
+    if "g" in d:
+        gate = torch.sigmoid(h @ d["g"].T)
+        y = y * (gate[:, :, None] if gate.shape[1] == H else gate.view(n, H, DIM))
+    return y.reshape(n, -1) @ d["o"].T
+
+
+@pytest.mark.parametrize("heads,rot,dims,pairing,ramp,q_rank,window,gate,lens", [
+    (3, 64, 64, "half_split", False, 96, None, "entry", [600, 33]), (2, 64, 64, "interleaved", True, None, 130, "head", [1, 513]),
+    (4, 64, 24, "interleaved", False, 96, None, False, [520]), (2, 32, 12, "half_split", True, 72, 65, "entry", [513, 64, 90]),
+    (2, 32, 32, "interleaved", False, None, None, "head", [700])])
+def test_a_turned_step_and_the_step_after_it(heads, rot, dims, pairing, ramp, q_rank, window, gate, lens):
+    """The mixer with rotation (whole and partial, both pairings, an amplitude): the prompt with its keys formed is as near to 64 bits
+    as on the cached vectors (a fifth for the draw of roundings), leaves the same cache to the bit, and so the next
+    step, on the cached vectors, gives the same bits after either."""
+    from torchless_rs_b200.csrc import ops
+    part, d, xs = _mixer(heads, rot, dims, pairing, ramp, q_rank, window, gate, lens, sum(lens))
+    keep, (B, T) = part.prompt, (len(lens), sum(lens))
+    assert part.amplitude != 1.0 if ramp else part.amplitude == 1.0
+
+    def step(x, pos, seq, batch):
+        batch.token_pos, batch.token_seq, batch.seq_slot, batch.plans = _i32(pos), _i32(seq), _i32(list(range(B))), {}
+        batch.len_bucket = max(lens) + 64
+        out = torch.zeros((x.shape[0], x.shape[1]), device="cuda")
+        part.forward(x.contiguous(), out, batch, overwrite=True)
+        return out.double()
+
+    got = {}
+    for name, prompt in (("formed", keep), ("latent", None)):
+        part.prompt = prompt
+        part.cache.pages.zero_()
+        before = ops.launch_counts().get("latent_prompt_tc", 0)
+        first = step(torch.cat([x[:-1] for x in xs]), sum([list(range(n)) for n in lens], []),
+                     sum([[b] * n for b, n in enumerate(lens)], []), _step(lens))
+        pages = part.cache.pages.clone()
+        one = SimpleNamespace(is_decode=True, n_seqs=B, max_new=1, past_lens=list(lens), new_lens=[n + 1 for n in lens],
+                              seq_start=_i32(list(range(B + 1))))
+        second = step(torch.cat([x[-1:] for x in xs]), lens, list(range(B)), one)
+        assert ops.launch_counts().get("latent_prompt_tc", 0) == before + (prompt is not None)
+        got[name] = (first, second, pages)
+    assert torch.equal(got["formed"][2], got["latent"][2]) and torch.equal(got["formed"][1], got["latent"][1])
+    want = [_mixer_in_64_bits(part, d, x, pairing) for x in xs]
+    rel = lambda a, b: float((a - b).norm() / b.norm())
+    whole, last = torch.cat([y[:-1] for y in want]), torch.cat([y[-1:] for y in want])
+    formed, latent, after = rel(got["formed"][0], whole), rel(got["latent"][0], whole), rel(got["formed"][1], last)
+    assert formed <= 1.2 * latent and formed < 1.5e-2 and after < 1.5e-2, (formed, latent, after)
+
+
+@pytest.mark.parametrize("dims,amplitude", [(64, 1.0), (24, 1.3), (0, 1.0)])
+def test_latent_prep_also_leaves_rows_in_token_order_and_the_turns(dims, amplitude):
+    """`flat`: the page rows to the bit; `turn`: cosine and sine of position x frequency times the amplitude, of 32-bit angles."""
+    from torchless_rs_b200.csrc import ops
+    o, rank, rot, lens = ops.core_ops(BF), 72, 64, [130, 7, 64]
+    T, g = sum(lens), torch.Generator(device="cuda").manual_seed(dims)
+    dkv = torch.randn((T, rank + rot), device="cuda", generator=g)
+    wc = torch.randn(rank, device="cuda", generator=g)
+    inv = (1e4 ** (-torch.arange(max(dims // 2, 1), dtype=F64) * 2 / max(dims, 1))).float().cuda()
+    pos = sum([list(range(5, 5 + n)) for n in lens], [])
+    table = torch.tensor([[4, 1, 0], [3, -1, -1], [2, 5, -1]], dtype=torch.int32, device="cuda")
+    pages = torch.zeros((6, 64, rank + rot), device="cuda", dtype=BF)
+    flat = torch.full((T, rank + rot), float("nan"), device="cuda", dtype=BF)
+    turn = torch.full((T, dims), float("nan"), device="cuda") if dims else None
+    seq = sum([[b] * n for b, n in enumerate(lens)], [])
+    o.latent_prep(None, dkv, None, wc, 1e-5, None, pages, _i32(pos), _i32(seq), _i32([0, 1, 2]), table, inv if dims else None, rank, rot,
+                  dims, amplitude=amplitude, flat=flat, turn=turn)
+    p, s = torch.tensor(pos, device="cuda"), torch.tensor(seq, device="cuda")
+    assert torch.equal(flat, pages[table[s, p // 64].long(), p % 64])
+    if dims:
+        ang = p.double()[:, None] * inv.double()
+        want = torch.stack([ang.cos(), ang.sin()], -1).view(T, dims) * amplitude
+        assert ((turn.double() - want).abs() <= 1.4 * (2.0 ** -24 * ang.repeat_interleave(2, -1) + 2.0 ** -22)).all()
+        u, v = dkv[:, rank:rank + dims // 2].double(), dkv[:, rank + dims // 2:rank + dims].double()
+        c, sn = want.view(T, -1, 2).unbind(-1)
+        r = torch.cat([u * c - v * sn, v * c + u * sn, dkv[:, rank + dims:].double()], -1)
+        assert ((flat[:, rank:].double() - r).abs() <= 2.0 ** -8 * r.abs() + 1e-4).all()
