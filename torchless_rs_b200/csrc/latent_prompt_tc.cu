@@ -14,8 +14,10 @@
 //   warp 4     TMA: a chunk's k_h and r beside it (one slot, free again after Q . K^T), v_h (two slots)
 //   warp 5     issues Q . K^T, up to two chunks ahead (two S buffers)
 //   warp 6     issues P . V: P from tensor memory, V's rows read across (the positions are the contracted dimension)
-// and the blocks of an SM, two of them, fill each other's waits.  What bounds it then is shared memory: a step of Q . K^T reads 6
-// KB for 32 cycles of the tensor core, 830 cycles for a chunk of either block where 940 are measured.  (Two slots of keys and
+// and the blocks of an SM, two of them, fill each other's waits.  What bounds it is the chain of a chunk: at 2048 tokens and 16 heads
+// all 256 blocks run at once, and the longest takes some 1.5 us for each of its 32 chunks (scores out of tensor memory, the
+// exponentials, O times what the maximum moved by, the weights back) while the tensor pipe is busy for 20 % of the cycles, the issue
+// slots for 35 and the loads from shared memory for 3.  (Two slots of keys and
 // one of values: 74 us instead of 66 for 2048 tokens and 16 heads, both as first written.  One block an SM of two tiles
 // that share their keys: 68 us against 52 then, because at 2048 tokens the longest blocks are left alone.)  The queries are turned,
 // scaled and rounded on their way into shared memory, and O / l leaves through it, gated, a warp per row.
