@@ -55,6 +55,30 @@ def _time(fn, iters: int) -> float:
     return e0.elapsed_time(e1) * 1e3 / (3 * iters)   # microseconds
 
 
+def _formed_rows(report, case: str, batch, heads: int, rank: int, rot: int, window, iters: int, gate=None, sink=None) -> None:
+    """Latent attention with the step's keys and values formed (heads of 128 plain entries), where a step of these lengths runs so:
+    the product that forms them, and the attention.  `gate`: None, "entry" or "head"."""
+    from .csrc.gemm_bf16 import GemmBf16
+    from .csrc.latent_bf16 import LatentPrompt
+    if not LatentPrompt.takes(batch, window):
+        return
+    T, dim, bf = sum(batch.new_lens), LatentPrompt.DIM, torch.bfloat16
+    seen = sum(sum(min(p + 1, window or n) for p in range(n)) for n in batch.new_lens)
+    latents = torch.randn((T, rank + rot), device="cuda", dtype=bf)
+    w = torch.randn((2 * heads * dim, rank), device="cuda", dtype=bf) * rank ** -0.5
+    kv, out = torch.empty((T, 2 * heads * dim), device="cuda", dtype=bf), torch.empty((T, heads * dim), device="cuda", dtype=bf)
+    us = _time(lambda: GemmBf16.get().run(latents[:, :rank], w, kv, 3), iters)
+    report("keys and values (product)", case, us, 2.0 * (T * rank + w.numel() + kv.numel()), 2.0 * T * w.numel())
+    q = torch.randn((T, heads * (dim + rot)), device="cuda")
+    angle = torch.randn((T, rot // 2), device="cuda")
+    turn = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
+    g = None if gate is None else torch.randn((T, heads * (dim if gate == "entry" else 1)), device="cuda")
+    us = _time(lambda: LatentPrompt.get().run(q, turn, kv, latents, out, g, sink, batch, heads, rank, rot, rot, window,
+                                              (dim + rot) ** -0.5), iters)
+    byts = q.numel() * 4.0 + kv.numel() * 2.0 + T * rot * 6.0 + out.numel() * 2.0 + (g.numel() * 4.0 if g is not None else 0.0)
+    report("latent_prompt (keys formed)", case, us, byts, 2.0 * heads * seen * (2 * dim + rot))
+
+
 def gemm(M: int, N: int, K: int, mode: int, iters: int) -> None:
     from .csrc.gemm_bf16 import GemmBf16
     g = GemmBf16.get()
@@ -257,7 +281,9 @@ def kikopel_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None) 
         us = _time(lambda: o.latent_attn(q, width, q, width, rank, pages, mix, pos, seq, slot, table, inv, H, rank,
                                          rot, rot, z["window"], 0.04, batch=_step_of(seqs, per, past, start)), max(2, iters // 8) if n_tok > 64 else iters)
         cache_b = 2.0 * seqs * min(past + per, z["window"]) * width
+        # (on the cached vectors: what steps that continue a sequence and short prompts run; a long prompt's own kernels after it)
         report("latent_attn", case, us, cache_b + n_tok * H * (width + rank) * 4.0, 2.0 * H * seen * (width + rank))
+        _formed_rows(report, case, _step_of(seqs, per, past, start), H, rank, rot, z["window"], iters, gate="entry")
         nkv = max(1, H // 4)
         att = AttentionBf16.get(128)
         kp, vp, tab2, slot2 = _paged(seqs, past + per, nkv, 128)
@@ -901,6 +927,7 @@ def fezolorn_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None)
                                          rot, rot, None, 0.04, max_keys=past + per, workspace=ws, sink=lsink,
                                          batch=_step_of(seqs, per, past, start)), few)
         report("latent_attn (sink, no window)", case, us, lat_b, 2.0 * mh * all_seen * (width + rank))
+        _formed_rows(report, case, _step_of(seqs, per, past, start), mh, rank, rot, None, iters, sink=lsink)
         us = _time(lambda: o.latent_attn(ql, width, ql, width, rank, pages, mix, pos, seq, slot, ltab, inv2, mh, rank,
                                          rot, rot, None, 0.04, max_keys=past + per, workspace=ws,
                                          batch=_step_of(seqs, per, past, start)), few)
@@ -1283,6 +1310,7 @@ def beralix_kernels(size: str, T: int, B: int, ctx: int, iters: int, file=None) 
                                          batch=_step_of(seqs, per, past, start)), few)
         byts = 2.0 * seqs * (past + per) * width + n_tok * mh * (width + rank) * 4.0
         report("latent_attn", case, us, byts, 2.0 * mh * seen * (width + rank))
+        _formed_rows(report, case, _step_of(seqs, per, past, start), mh, rank, rot, None, iters, gate="head")
         ql = torch.randn((n_tok, mh * width), device=dev)
         us = _time(lambda: o.latent_attn(ql, width, ql, width, rank, pages, mix, pos, seq, slot, ltab, inv2, mh, rank, rot,
                                          rot, None, 0.04, max_keys=past + per, workspace=ws,
