@@ -300,11 +300,13 @@ __global__ void rope_cache_write_kernel(const float* __restrict__ qkv, int ld,
 //    thread with 16-byte loads, PASSES of them, whose loads are all issued before the angles are worked out;
 //  - blockIdx.y == rot_groups, `turned`: 32 consecutive tokens of one value head; the tile is turned in shared memory, so
 //    that the transposed value pages are written in runs of positions;
-//  - blockIdx.y == rot_groups otherwise: one token's value heads, written as they are read.
+//  - blockIdx.y >= rot_groups otherwise: 512 entries of one token's value heads, written as they are read.
 // What bounds it is the chain of a block (position, angle, sine; sequence, slot, page) beside few bytes, hence the loads
 // first.  Bfloat16, 32 + 8 heads of 128, a warp per head below 256 tokens and loads after the angles from there on / now: in
 // decode steps of 64 sequences 7.0 / 4.2 us, in prompts of 100 tokens 7.1 / 4.2 us, of 2048 20.6 / 19.3 us; alone 200 tokens
-// 10.4 / 4.2 us, 2048 14.3 / 12.5 us, 8192 63 / 54 us (302 MB).
+// 10.4 / 4.2 us, 2048 14.3 / 12.5 us, 8192 63 / 54 us (302 MB).  (Those of the steps with all of a token's value heads in one block,
+// whose scattered stores ended last: one token 2.5 us, now 2.0, 64 of their own pages 3.9 / 2.4; 8 value heads of 256, one token 3.9 /
+// 2.0, by a warp per head 3.1.)
 #define ROPE_PASSES 4
 template <int PASSES>
 __global__ void __launch_bounds__(128)
@@ -347,17 +349,15 @@ rope_cache_write_vec_kernel(const float* __restrict__ qkv, int ld, act_t* __rest
   const int t = blockIdx.x;
   const int pos = token_pos[t];
   const int page = page_table[(size_t)seq_slot[token_seq[t]] * table_stride + pos / TL_PAGE];
-  if ((int)blockIdx.y == rot_groups) {
+  if ((int)blockIdx.y >= rot_groups) {
     const float* row = qkv + (size_t)t * ld + (size_t)(nh + nkv) * hd;
     act_t* dst = v_pages + (size_t)page * nkv * (size_t)(TL_PAGE * hd) + (pos % TL_PAGE);
-    if (page < 0) return;
-#pragma unroll 2
-    for (int d = threadIdx.x * 4; d < nkv * hd; d += 512) {     // (the heads of a page follow one another)
-      float v[4];
-      load4(row + d, v);
+    const int d = ((int)blockIdx.y - rot_groups) * 512 + threadIdx.x * 4;
+    if (page < 0 || d >= nkv * hd) return;
+    float v[4];
+    load4(row + d, v);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dst[(size_t)(d + j) * TL_PAGE] = from_f32<act_t>(v[j]);
-    }
+    for (int j = 0; j < 4; ++j) dst[(size_t)(d + j) * TL_PAGE] = from_f32<act_t>(v[j]);     // (the heads of a page follow one another)
     return;
   }
   const int half = hd >> 1;
@@ -419,11 +419,11 @@ extern "C" int TL_NAME(tl_rope_cache_write)(const float* qkv, int ld, void* q_ou
     // while the GPU has few blocks a pass to a block, then as many as a thread's registers take
     const int rot_groups = (long long)T * passes < 640 ? passes : (passes + ROPE_PASSES - 1) / ROPE_PASSES;
     const int per_group = (passes + rot_groups - 1) / rot_groups;
-    if (rot_groups > 65534) return TL_ERR_UNSUPPORTED;
-    const int turned = T >= 128;
+    const int turned = T >= 128, value_groups = turned ? 1 : (int)(((long long)nkv * hd + 511) / 512);
+    if ((long long)rot_groups + value_groups > 65535) return TL_ERR_UNSUPPORTED;
     const size_t smem = (turned ? (size_t)32 * (hd + 1) : (size_t)hd) * sizeof(float);
 #define ROPE(P)                                                                                                          \
-  return tl_launch(rope_cache_write_vec_kernel<P>, dim3(T, rot_groups + 1), dim3(128), smem, stream, qkv, ld,            \
+  return tl_launch(rope_cache_write_vec_kernel<P>, dim3(T, rot_groups + value_groups), dim3(128), smem, stream, qkv, ld, \
                    (act_t*)q_out, (act_t*)k_pages, (act_t*)v_pages, token_pos, token_seq, seq_slot, page_table,          \
                    table_stride, inv_freq, T, nh, nkv, hd, rot_groups, turned)
     switch (per_group) {
